@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/tf_b200.h"
+#include "tf_factor.cuh"
 #include "tf_internal.cuh"
 
 using namespace tfb;
@@ -36,6 +37,8 @@ constexpr int kMlTopMax = 160;       // sets of the multilevel space's densely i
 constexpr int kMlAutoNodes = 100000; // single tissues from this size take the multilevel space
 constexpr int kMlTopMaxAge = 8;      // solves between refreshes of the multilevel top inverse
 constexpr int kWarmSlots = 8;        // Newton iterations whose solutions are kept for warm starts
+constexpr int kFcMaxIters = 8;       // iterations after which a factorised solve counts as failed
+constexpr double kFcMaxFlops = 4e11; // largest factorisation (operations of one tissue, or mean of a batch)
 
 struct DevBuf {
     void* p = nullptr;
@@ -164,6 +167,16 @@ struct tf_ctx {
     int32_t ilu_colours = 0;
     DevBuf ilu_cnodes, ilu_lo_ptr, ilu_lo_idx, ilu_up_ptr, ilu_up_idx, ilu_lu, ilu_uinv, ilu_y;
     cudaGraphExec_t ilu_graph = nullptr;
+
+    // sparse factorisation (tf_factor.cuh): the plan of the current pattern and its buffers
+    FcPlan fc;
+    bool fc_dirty = true;      // the pattern changed since the plan was built
+    bool fc_ready = false;     // plan and buffers exist
+    bool fc_used = false;      // the last solve was a factorised one
+    bool fc_same = false;      // the factor on the device is of the current J (further right-hand sides)
+    std::vector<int32_t> fc_chunk0;
+    DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_tp, fc_vec, fc_z,
+        fc_sign, fc_flags, fc_chunks, fc_chunk0_d, fc_running, fc_part;
 
     // adjoint: forward checkpoints every adj_k steps, segment recompute buffers, adjoint state
     int32_t adj_steps = 0, adj_k = 0;
@@ -458,6 +471,7 @@ int upload_structure(tf_ctx* ctx) {
         if (irc != TF_OK) return irc;
     }
     ctx->coarse_dirty = true;
+    ctx->fc_dirty = true;
     const size_t np2 = std::max((size_t)std::max(spmv_grid(N), vec_grid(N)) * 2,
                                 (size_t)ctx->persistent_grid_max * 8) + 64;
     TF_CK(dalloc(ctx->partials, sizeof(double) * np2));
@@ -1659,10 +1673,175 @@ bool use_persistent(tf_ctx* ctx) {
            ctx->persistent_grid_max > 0 && (ctx->params.persistent || ctx->T > 1);
 }
 
+// ---- factorised solves ------------------------------------------------------------------
+//
+// With the default preconditioner and a symmetric J, conjugate gradients are preconditioned by a
+// sparse factorisation of J where the tissue is small enough for one: the separators' Schur
+// complement is the coarse operator then, eliminated exactly.
+
+// Whether this solve may take the factorisation. Packing pairs add blocks outside the pattern and make
+// J indefinite (MINRES); krylov_warm_start = 0 asks for solves that keep nothing from earlier ones.
+bool factor_wanted(const tf_ctx* c) {
+    return c->params.precond == TF_PRECOND_TWO_LEVEL && c->params.krylov_method == TF_KRYLOV_AUTO && !c->has_visc &&
+           c->params.krylov_warm_start && !(c->pk_on && c->pk_pairs_n > 0);
+}
+
+int build_factor(tf_ctx* ctx) {
+    ctx->fc_dirty = false;
+    ctx->fc_ready = false;
+    const int N = ctx->N, T = ctx->T;
+    int G = std::max(ctx->col_G, 1);
+    for (int t = 0; t < T; ++t)
+        if ((ctx->tissue_node0[t + 1] - ctx->tissue_node0[t]) % G != 0) G = 1;
+    std::vector<double> X((size_t)(N / G) * 3, 0.0);
+    for (int e = 0; e < ctx->E; ++e)
+        for (int a = 0; a < 6; ++a) {
+            const int32_t n = ctx->conn[(size_t)e * 6 + a];
+            if (n % G == 0)
+                for (int d = 0; d < 3; ++d) X[(size_t)(n / G) * 3 + d] = ctx->xref[(size_t)e * 18 + a * 3 + d];
+        }
+    FcPlan& P = ctx->fc;
+    build_factor_plan(N, G, ctx->rowptr.data(), ctx->colidx.data(), X.data(), T, ctx->tissue_node0.data(), kFcMaxFlops * T, P);
+    if (!P.ok) return TF_OK;
+    std::vector<FcChunk> chunks;
+    ctx->fc_chunk0.assign(1, 0);
+    for (int t = 0; t < T; ++t) {
+        for (int r = ctx->tissue_node0[t]; r < ctx->tissue_node0[t + 1]; r += kFcChunkRows)
+            chunks.push_back({t, r, std::min(r + kFcChunkRows, ctx->tissue_node0[t + 1])});
+        ctx->fc_chunk0.push_back((int32_t)chunks.size());
+    }
+    auto room = [&](DevBuf& b, int64_t doubles) { return dalloc(b, sizeof(double) * (size_t)std::max<int64_t>(doubles, 2)); };
+    auto up = [&](DevBuf& b, const void* h, size_t bytes) -> cudaError_t {
+        cudaError_t e = dalloc(b, std::max<size_t>(bytes, 16));
+        if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(b.p, h, bytes, cudaMemcpyHostToDevice, ctx->stream);
+        return e;
+    };
+    cudaError_t e = room(ctx->fc_factor, P.n_factor);
+    if (e == cudaSuccess) e = room(ctx->fc_scratch, P.n_scratch);
+    for (int q = 0; q < 2; ++q)
+        if (e == cudaSuccess) e = room(ctx->fc_contrib[q], P.n_contrib[q]);
+    if (e == cudaSuccess) e = room(ctx->fc_tp, P.n_tp);
+    if (e == cudaSuccess) e = room(ctx->fc_vec, P.n_vec);
+    if (e == cudaSuccess) e = room(ctx->fc_z, P.n_piv);
+    if (e == cudaSuccess) e = room(ctx->fc_sign, P.n_piv);
+    if (e == cudaSuccess) e = room(ctx->fc_part, 3 * (int64_t)chunks.size());
+    if (e == cudaErrorMemoryAllocation) {  // no room for the factor: the iterative solve needs far less
+        (void)cudaGetLastError();
+        for (DevBuf* b : {&ctx->fc_factor, &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1]}) dfree(*b);
+        return TF_OK;
+    }
+    TF_CK(e);
+    TF_CK(dalloc(ctx->fc_flags, sizeof(int32_t) * T));
+    TF_CK(dalloc(ctx->fc_running, sizeof(int32_t) * T));
+    TF_CK(up(ctx->fc_fronts, P.fronts.data(), sizeof(FcFront) * P.fronts.size()));
+    TF_CK(up(ctx->fc_maps, P.maps.data(), sizeof(int32_t) * P.maps.size()));
+    TF_CK(up(ctx->fc_verts, P.verts.data(), sizeof(int32_t) * P.verts.size()));
+    TF_CK(up(ctx->fc_jblk, P.jblk.data(), sizeof(int2) * P.jblk.size()));
+    TF_CK(up(ctx->fc_tasks, P.tasks.data(), sizeof(FcTask) * P.tasks.size()));
+    TF_CK(up(ctx->fc_chunks, chunks.data(), sizeof(FcChunk) * chunks.size()));
+    TF_CK(up(ctx->fc_chunk0_d, ctx->fc_chunk0.data(), sizeof(int32_t) * ctx->fc_chunk0.size()));
+    TF_CK(cudaStreamSynchronize(ctx->stream));
+    // the launches need the task ranges and the fronts' sizes only
+    P.maps = {};
+    P.verts = {};
+    P.jblk = {};
+    ctx->fc_ready = true;
+    return TF_OK;
+}
+
+FcWork make_factor(tf_ctx* c) {
+    FcWork f{};
+    f.gd = c->fc.gd;
+    f.fronts = dptr<FcFront>(c->fc_fronts);
+    f.maps = dptr<int32_t>(c->fc_maps);
+    f.verts = dptr<int32_t>(c->fc_verts);
+    f.jblk = dptr<int2>(c->fc_jblk);
+    f.tasks = dptr<FcTask>(c->fc_tasks);
+    f.active = dptr<int32_t>(c->active_d);
+    f.factor = dptr<double>(c->fc_factor);
+    f.scratch = dptr<double>(c->fc_scratch);
+    f.contrib[0] = dptr<double>(c->fc_contrib[0]);
+    f.contrib[1] = dptr<double>(c->fc_contrib[1]);
+    f.tp = dptr<double>(c->fc_tp);
+    f.vec = dptr<double>(c->fc_vec);
+    f.z = dptr<double>(c->fc_z);
+    f.sign = dptr<double>(c->fc_sign);
+    f.flags = dptr<int32_t>(c->fc_flags);
+    return f;
+}
+
+// One factorised solve of every active tissue: conjugate gradients from zero whose preconditioner is
+// the factor of J, so that one or two iterations meet the tolerance (the residual's recurrence is
+// the refinement). *done = false when a tissue did not get there (a zero pivot, a non-finite
+// value, an ill-conditioned J): the caller solves them all again by the iterative path.
+int factor_solve(tf_ctx* ctx, bool* done) {
+    *done = false;
+    const KrylovWork w = make_work(ctx);
+    FcWork f = make_factor(ctx);
+    FcCg c;
+    c.n_chunks = ctx->fc_chunk0.back();
+    c.T = ctx->T;
+    c.chunks = dptr<FcChunk>(ctx->fc_chunks);
+    c.chunk0 = dptr<int32_t>(ctx->fc_chunk0_d);
+    c.sc = dptr<KrylovScalars>(ctx->tscalars);
+    c.active = dptr<int32_t>(ctx->active_d);
+    c.running = dptr<int32_t>(ctx->fc_running);
+    c.part = dptr<double>(ctx->fc_part);
+    if (!ctx->fc_same) {
+        TF_CK(cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream));
+        TF_CK(launch_factor(ctx->fc, f, w.vals, &ctx->launches, ctx->stream));
+        ++ctx->coarse_refreshes;
+    }
+    const int cap = std::min(kFcMaxIters, ctx->params.krylov_max_iters);
+    TF_CK(launch_fc_start(w, c, ctx->params.krylov_rtol, cap, ctx->stream));
+    ctx->launches += 2;
+    f.active = c.running;
+    double* z = w.phat;
+    bool running = true;
+    for (int it = 0; it < cap && running; ++it) {
+        TF_CK(launch_factor_solve(ctx->fc, f, w.r, z, &ctx->launches, ctx->stream));
+        TF_CK(launch_fc_iteration(w, c, z, w.v, ctx->stream));
+        ctx->launches += 5;
+        TF_CK(cudaMemcpyAsync(ctx->h_tsc, ctx->tscalars.p, sizeof(KrylovScalars) * ctx->T, cudaMemcpyDeviceToHost, ctx->stream));
+        TF_CK(cudaStreamSynchronize(ctx->stream));
+        running = false;
+        for (int t = 0; t < ctx->T; ++t)
+            if (ctx->T == 1 || ctx->h_active[t]) {
+                const int st = ctx->h_tsc[t].status;
+                if (st == KS_RUNNING)
+                    running = true;
+                else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters))
+                    return TF_OK;
+            }
+    }
+    *ctx->h_sc = ctx->h_tsc[0];
+    ctx->last_solve_iters = 0;
+    for (int t = 0; t < ctx->T; ++t)
+        if (ctx->T == 1 || ctx->h_active[t]) {
+            ctx->last_method = std::max<int32_t>(ctx->last_method, KM_CG);
+            ctx->cg_iters += ctx->h_tsc[t].iter;
+            ctx->last_solve_iters = std::max(ctx->last_solve_iters, ctx->h_tsc[t].iter);
+        }
+    ctx->last_solve_method = KM_CG;
+    *done = true;
+    return TF_OK;
+}
+
 // Solve J du = g (buffers in the context) for every active tissue. Leaves the scalars in
 // ctx->h_tsc[T] (persistent) or ctx->h_sc (chunked, single tissue).
 int krylov_solve(tf_ctx* ctx) {
     KrylovWork w = make_work(ctx);
+    if (use_persistent(ctx) && factor_wanted(ctx)) {
+        if (ctx->fc_dirty) {
+            const int frc = build_factor(ctx);
+            if (frc != TF_OK) return frc;
+        }
+        ctx->fc_used = false;
+        if (ctx->fc_ready) {
+            const int frc = factor_solve(ctx, &ctx->fc_used);
+            if (frc != TF_OK || ctx->fc_used) return frc;
+        }
+    }
     if (use_persistent(ctx)) {
         if (ctx->params.precond == TF_PRECOND_TWO_LEVEL || ctx->params.precond == TF_PRECOND_MULTILEVEL) {
             if (ctx->ml_active && (ctx->plan_ncta.empty() || ctx->plan_ncta[0] != ctx->ml_nct))
@@ -1926,7 +2105,12 @@ int newton_core(tf_ctx* ctx, double dt, tf_step_stats* st) {
         for (int t = 0; t < T; ++t)
             weight[t] = (ctx->tissue_node0[t + 1] - ctx->tissue_node0[t]) * std::max(8.0, (double)ctx->last_krylov[t]);
     ctx->last_krylov.assign(T, 0);
-    if (T > 1 && persistent && ctx->params.precond == TF_PRECOND_TWO_LEVEL && ctx->coarse_dirty) {
+    if (persistent && factor_wanted(ctx) && ctx->fc_dirty) {
+        const int frc = build_factor(ctx);
+        if (frc != TF_OK) return frc;
+    }
+    if (T > 1 && persistent && ctx->params.precond == TF_PRECOND_TWO_LEVEL && ctx->coarse_dirty &&
+        !(factor_wanted(ctx) && ctx->fc_ready)) {
         const int crc = build_coarse(ctx);  // the batch plan gives every CTA whole aggregates
         if (crc != TF_OK) return crc;
     }
@@ -2060,7 +2244,9 @@ int newton_solve(tf_ctx* ctx) {
     TF_CK(cudaMemcpyAsync(ctx->lm_gsave_d.p, ctx->g.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     TF_CK(cudaMemcpyAsync(ctx->g.p, ctx->lm_G_d.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     ctx->reuse_precond = true;
+    ctx->fc_same = ctx->fc_used;  // the factor is of this J
     rc = krylov_solve(ctx);
+    ctx->fc_same = false;
     ctx->reuse_precond = false;
     if (rc != TF_OK) return rc;
     TF_CK(cudaMemcpyAsync(ctx->lm_z_d.p, ctx->du.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -2451,6 +2637,10 @@ void tf_destroy(tf_ctx* ctx) {
                      &ctx->ml_first_cta_d, &ctx->ml_slot_a_d, &ctx->ml_out_ptr_d, &ctx->ml_out_slots_d,
                      &ctx->ml_out_set_d, &ctx->ml_out_col_d, &ctx->ml_out_dst_d, &ctx->ml_pairs_d, &ctx->ml_pos_leaf_d};
     for (DevBuf* b : mlb) dfree(*b);
+    DevBuf* fcb[] = {&ctx->fc_fronts, &ctx->fc_maps, &ctx->fc_verts, &ctx->fc_jblk, &ctx->fc_tasks, &ctx->fc_factor,
+                     &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1], &ctx->fc_tp, &ctx->fc_vec, &ctx->fc_z,
+                     &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
+    for (DevBuf* b : fcb) dfree(*b);
     if (ctx->h_coarse_info) cudaFreeHost(ctx->h_coarse_info);
     if (ctx->h_active) cudaFreeHost(ctx->h_active);
     if (ctx->h_du2) cudaFreeHost(ctx->h_du2);
@@ -2851,7 +3041,9 @@ int tf_solve(tf_ctx* ctx, const double* bsr_vals, const double* g, double* du, i
             const double r2 = ctx->h_sc->du2;
             rel = std::sqrt(r2 / bb);
             if (!(r2 > 0.0)) break;  // exact (or non-finite: reported by the next solve's status)
+            ctx->fc_same = ctx->fc_used;
             rc = krylov_solve(ctx);
+            ctx->fc_same = false;
             if (rc != TF_OK) break;
             const KrylovScalars sk = *ctx->h_sc;
             total_iters += sk.iter;
@@ -3080,7 +3272,10 @@ int tf_time_step(tf_ctx* ctx, const double* x_n, double dt, double* x_out, tf_st
 int tf_get_preconditioner(tf_ctx* ctx, int32_t* precond, int32_t* n_coarse, int32_t* coarse_refreshes) {
     if (!ctx) return TF_ERR_ARGUMENT;
     if (precond) *precond = ctx->ml_active ? TF_PRECOND_MULTILEVEL : ctx->params.precond;
-    if (n_coarse) *n_coarse = (ctx->coarse_m > 0 || ctx->bc_active || ctx->ml_active) ? ctx->n_coarse : 0;
+    if (n_coarse) {
+        *n_coarse = (ctx->coarse_m > 0 || ctx->bc_active || ctx->ml_active) ? ctx->n_coarse : 0;
+        if (ctx->fc_used) *n_coarse = (int32_t)ctx->fc.n_root;
+    }
     if (coarse_refreshes) *coarse_refreshes = ctx->coarse_refreshes;
     return TF_OK;
 }

@@ -1,0 +1,133 @@
+// tf_factor.cuh -- plan and kernel entry points of the sparse factorisation of a symmetric J.
+//
+// A tissue's unknowns are ordered by nested dissection: a small set of prism columns (a separator)
+// splits the mesh in two halves that share no Jacobian block, each half is split again, and so on.
+// Every separator (and every undivided piece at the bottom) is a front: its own unknowns, the
+// pivots, and the boundary, the unknowns of enclosing separators its subtree touches. A front's
+// dense matrix is its share of J plus what its (at most two) children left on their boundaries;
+// eliminating its pivots leaves a matrix on the boundary for its parent. All fronts of one depth
+// of the tree are processed together, the deepest first.
+//
+// With the front's matrix [A11 A21^T; A21 A22], A11 = G S G^T (G lower triangular, S = diag(+-1)):
+//   x11 = G^-1 (p x p, lower), l21 = A21 G^-T S (b x p), contribution C = A22 - l21 S l21^T.
+// A solve is then one pass up the tree, z = x11 v_P, v_B -= l21 z, and one down,
+// x_P = x11^T (S z - l21^T x_B): matrix-vector products only, no triangular solves.
+#pragma once
+
+#include <vector>
+
+#include "tf_internal.cuh"
+
+namespace tfb {
+
+constexpr int kFcTile = 64;        // pivot panel width and GEMM tile
+constexpr int kFcGatherRows = 32;  // rows of a front per assembly task
+constexpr int kFcScatter = 256;    // Jacobian blocks per assembly task
+constexpr int kFcRows = 32;        // front rows per solve task
+constexpr int kFcBackRows = 128;   // boundary rows per backward task
+constexpr int kFcMaxPivots = 5000; // pivots of one front (the solve stages them in shared memory)
+
+struct FcFront {
+    int32_t p, b;          // pivot and boundary unknowns
+    int32_t ldp, ldb;      // leading dimensions (even): rows of x11 / l21 / a21, rows of c
+    int32_t tissue;
+    int32_t child[2];      // fronts one depth below, or -1
+    int32_t map[2];        // offsets into maps: per column of this front, its index on the child's boundary
+    int32_t verts;         // offset into verts: the pivots' columns, then the boundary's
+    int32_t j0, j1;        // its Jacobian blocks in jblk
+    int32_t vec, piv;      // offsets of the boundary vector (b) and of z / the signs (p)
+    int64_t x11, l21;      // kept factors
+    int64_t a21, lp;       // scratch of the front's depth: A21, and the current panel of L11 (p x 64)
+    int64_t c;             // contribution (b x b, lower), in the scratch of the depth's parity
+    int64_t tp;            // scratch of the backward pass: partial sums per boundary chunk (chunks x p)
+};
+
+struct FcTask {
+    int32_t front;
+    int16_t i, j;
+};
+
+struct FcRange {
+    int32_t begin = 0, count = 0;
+};
+
+struct FcPanel {
+    FcRange col, upd;
+};
+
+struct FcDepth {
+    FcRange gather, scatter, diag, l21, schur, fwd1, fwd2, bwd1, bwd2;
+    int32_t panel0 = 0, n_panel = 0;
+};
+
+// Host side of a factorisation: the symbolic result, laid out for the device.
+struct FcPlan {
+    int gd = 3;  // unknowns per column (three per node)
+    std::vector<FcFront> fronts;
+    std::vector<int32_t> maps, verts;
+    std::vector<int2> jblk;  // {block, row << 16 | column} in the front's [x11; a21] rows
+    std::vector<FcTask> tasks;
+    std::vector<FcDepth> depths;  // 0: the roots
+    std::vector<FcPanel> panels;
+    int64_t n_factor = 0, n_scratch = 0, n_contrib[2] = {0, 0}, n_tp = 0;  // doubles
+    int64_t n_vec = 0, n_piv = 0;
+    int64_t n_root = 0;   // pivots of the root fronts
+    double flops = 0.0;   // multiplications and additions of one factorisation
+    int chain = 0;        // dependent 64-pivot panels over the depths
+    bool ok = false;
+};
+
+// Symbolic factorisation of the block pattern (G consecutive nodes form one column with in-plane
+// position X[3 column]); tissue t owns nodes [node0[t], node0[t+1]). plan.ok = false when a front
+// is too large for the kernels or the operation count exceeds max_flops.
+void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colidx, const double* X, int T,
+                       const int32_t* node0, double max_flops, FcPlan& plan);
+
+// Device side.
+struct FcWork {
+    int gd;
+    const FcFront* fronts;
+    const int32_t* maps;
+    const int32_t* verts;
+    const int2* jblk;
+    const FcTask* tasks;
+    const int32_t* active;  // [T]
+    double* factor;
+    double* scratch;
+    double* contrib[2];
+    double* tp;
+    double* vec;
+    double* z;
+    double* sign;    // [n_piv] +1 / -1
+    int32_t* flags;  // [T] 1: a zero or non-finite pivot
+};
+
+// Numeric factorisation of J (vals: the full BSR3 values; block (row, column) is read from the row of
+// the earlier pivot, transposed). Returns the kernels launched in *launches.
+cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, cudaStream_t s);
+// x = (factor)^-1 in on the active tissues' unknowns (every unknown is a pivot of one front).
+cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
+                                cudaStream_t s);
+
+// Preconditioned conjugate gradients with the factor as preconditioner, one kernel per phase, every
+// tissue with its own scalars. A chunk is a run of rows of one tissue; the dot products are summed
+// per chunk and then per tissue in chunk order.
+struct FcChunk {
+    int32_t tissue, row0, row1;
+};
+constexpr int kFcChunkRows = 256;
+struct FcCg {
+    int n_chunks, T;
+    const FcChunk* chunks;
+    const int32_t* chunk0;  // [T+1]
+    KrylovScalars* sc;      // [T]
+    const int32_t* active;  // [T] tissues of this solve
+    int32_t* running;       // [T] still iterating (the preconditioner's active flags)
+    double* part;           // [3][n_chunks]: (r, z), (p, J p), (r, r) / (b, b)
+};
+// x = 0, r = b, p = 0; every active tissue running (unless b = 0)
+cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int max_iter, cudaStream_t s);
+// one iteration after z = M^-1 r: p = z + beta p, q = J p, x += alpha p, r -= alpha q, and the test
+cudaError_t launch_fc_iteration(const KrylovWork& w, const FcCg& c, const double* z, double* q, cudaStream_t s);
+
+}  // namespace tfb

@@ -1,0 +1,440 @@
+// tf_factor_plan.cu -- nested dissection and symbolic factorisation of the Jacobian's block pattern
+// (host code; the numeric kernels are in tf_factor.cu). No counterpart in the reference, which
+// hands every system to Pardiso (NewtonRaphsonSolver.cpp:498-763).
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <numeric>
+#include <thread>
+
+#include "tf_factor.cuh"
+
+namespace tfb {
+namespace {
+
+struct Node {
+    std::vector<int32_t> piv, bnd;  // columns
+    int depth = 0;
+    int child[2] = {-1, -1};
+};
+
+// Columns of one tissue: their graph (ptr / adj over local ids), positions, and the dissection.
+struct Dissection {
+    const int32_t* ptr;
+    const int32_t* adj;
+    const double* X;  // [n][3]
+    int leaf;
+    std::vector<Node> nodes;
+    std::vector<int32_t> perm, label, match, seen, pos;
+    int32_t next_label = 0, stamp = 0;
+
+    // Augmenting path of the bipartite cut graph from a on side A (labels la) to side B (lb).
+    bool augment(int32_t a, int32_t lb) {
+        for (int32_t k = ptr[a]; k < ptr[a + 1]; ++k) {
+            const int32_t b = adj[k];
+            if (label[b] != lb || seen[b] == stamp) continue;
+            seen[b] = stamp;
+            if (match[b] < 0 || augment(match[b], lb)) {
+                match[b] = a;
+                match[a] = b;
+                return true;
+            }
+        }
+        return false;
+    }
+    // Columns reached from unmatched a by alternating paths (Koenig's construction).
+    void reach(int32_t a, int32_t lb) {
+        seen[a] = stamp;
+        for (int32_t k = ptr[a]; k < ptr[a + 1]; ++k) {
+            const int32_t b = adj[k];
+            if (label[b] != lb || seen[b] == stamp) continue;
+            seen[b] = stamp;
+            if (match[b] >= 0 && seen[match[b]] != stamp) reach(match[b], lb);
+        }
+    }
+
+    // Splits perm[lo, hi) in two halves across the longest side of its bounding box; the separator is
+    // a smallest set of columns that covers every block between the halves (a minimum vertex cover
+    // of the cut edges, from a maximum matching).
+    int split(int32_t lo, int32_t hi, int depth) {
+        const int id = (int)nodes.size();
+        nodes.emplace_back();
+        nodes[id].depth = depth;
+        if (hi - lo <= leaf) {
+            nodes[id].piv.assign(perm.begin() + lo, perm.begin() + hi);
+            return id;
+        }
+        double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
+        for (int32_t k = lo; k < hi; ++k)
+            for (int d = 0; d < 3; ++d) {
+                mn[d] = std::min(mn[d], X[(size_t)perm[k] * 3 + d]);
+                mx[d] = std::max(mx[d], X[(size_t)perm[k] * 3 + d]);
+            }
+        int ax = 0;
+        for (int d = 1; d < 3; ++d)
+            if (mx[d] - mn[d] > mx[ax] - mn[ax]) ax = d;
+        const int32_t mid = lo + (hi - lo) / 2;
+        const int a2 = ax == 0 ? 1 : 0;  // columns at the split coordinate are ordered along the cut
+        std::nth_element(perm.begin() + lo, perm.begin() + mid, perm.begin() + hi, [&](int32_t u, int32_t v) {
+            const double xu = X[(size_t)u * 3 + ax], xv = X[(size_t)v * 3 + ax];
+            if (xu != xv) return xu < xv;
+            const double yu = X[(size_t)u * 3 + a2], yv = X[(size_t)v * 3 + a2];
+            return yu != yv ? yu < yv : u < v;
+        });
+        const int32_t la = next_label++, lb = next_label++;
+        for (int32_t k = lo; k < hi; ++k) {
+            label[perm[k]] = k < mid ? la : lb;
+            match[perm[k]] = -1;
+        }
+        std::vector<int32_t> front_a;  // columns of A next to B
+        for (int32_t k = lo; k < mid; ++k) {
+            const int32_t a = perm[k];
+            for (int32_t q = ptr[a]; q < ptr[a + 1]; ++q)
+                if (label[adj[q]] == lb) {
+                    front_a.push_back(a);
+                    break;
+                }
+        }
+        for (int32_t a : front_a)  // greedy matching first, then augmenting paths
+            for (int32_t q = ptr[a]; q < ptr[a + 1]; ++q) {
+                const int32_t b = adj[q];
+                if (label[b] == lb && match[b] < 0) {
+                    match[a] = b;
+                    match[b] = a;
+                    break;
+                }
+            }
+        for (int32_t a : front_a)
+            if (match[a] < 0) {
+                ++stamp;
+                augment(a, lb);
+            }
+        ++stamp;
+        for (int32_t a : front_a)
+            if (match[a] < 0 && seen[a] != stamp) reach(a, lb);
+        // cover: unreached columns of A, reached columns of B
+        const int32_t ls = next_label++;
+        std::vector<int32_t> sep;
+        for (int32_t a : front_a) {
+            if (seen[a] != stamp) sep.push_back(a);
+            for (int32_t q = ptr[a]; q < ptr[a + 1]; ++q) {
+                const int32_t b = adj[q];
+                if (label[b] == lb && seen[b] == stamp) {
+                    label[b] = ls;
+                    sep.push_back(b);
+                }
+            }
+        }
+        for (int32_t v : sep) label[v] = ls;
+        const auto ea = std::stable_partition(perm.begin() + lo, perm.begin() + hi, [&](int32_t v) { return label[v] == la; });
+        const auto eb = std::stable_partition(ea, perm.begin() + hi, [&](int32_t v) { return label[v] == lb; });
+        const int32_t ma = (int32_t)(ea - perm.begin()), mb = (int32_t)(eb - perm.begin());
+        nodes[id].piv.assign(eb, perm.begin() + hi);
+        // pivots in order along the separator
+        std::sort(nodes[id].piv.begin(), nodes[id].piv.end(), [&](int32_t u, int32_t v) {
+            const double yu = X[(size_t)u * 3 + a2], yv = X[(size_t)v * 3 + a2];
+            return yu != yv ? yu < yv : u < v;
+        });
+        int n = 0;
+        if (ma > lo) {
+            const int c = split(lo, ma, depth + 1);
+            nodes[id].child[n++] = c;
+        }
+        if (mb > ma) {
+            const int c = split(ma, mb, depth + 1);
+            nodes[id].child[n++] = c;
+        }
+        return id;
+    }
+
+    // Elimination positions (children before their parent) and every front's boundary.
+    int32_t order(int id, int32_t at) {
+        for (int c : nodes[id].child)
+            if (c >= 0) at = order(c, at);
+        for (int32_t v : nodes[id].piv) pos[v] = at++;
+        return at;
+    }
+    void boundary(int id) {
+        for (int k = 0; k < 2; ++k)
+            if (nodes[id].child[k] >= 0) boundary(nodes[id].child[k]);
+        Node& f = nodes[id];
+        ++stamp;
+        for (int32_t v : f.piv) seen[v] = stamp;
+        auto add = [&](int32_t v, int32_t after) {
+            if (pos[v] > after && seen[v] != stamp) {
+                seen[v] = stamp;
+                f.bnd.push_back(v);
+            }
+        };
+        int32_t last = -1;  // position of the subtree's last eliminated column
+        for (int32_t v : f.piv) last = std::max(last, pos[v]);
+        for (int32_t v : f.piv)
+            for (int32_t k = ptr[v]; k < ptr[v + 1]; ++k) add(adj[k], last);
+        for (int c : f.child)
+            if (c >= 0)
+                for (int32_t v : nodes[c].bnd) add(v, last);
+        std::sort(f.bnd.begin(), f.bnd.end(), [&](int32_t u, int32_t v) { return pos[u] < pos[v]; });
+    }
+
+    void run(int32_t n) {
+        perm.resize(n);
+        std::iota(perm.begin(), perm.end(), 0);
+        label.assign(n, -1);
+        match.assign(n, -1);
+        seen.assign(n, -1);
+        pos.assign(n, 0);
+        split(0, n, 0);
+        order(0, 0);
+        stamp = next_label + 1 + stamp;
+        boundary(0);
+    }
+};
+
+template <class F>
+void parallel_items(int n, F f) {
+    const int nt = std::min<int>(n, (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
+    std::atomic<int> next{0};
+    auto work = [&] {
+        for (int i; (i = next.fetch_add(1)) < n;) f(i);
+    };
+    std::vector<std::thread> th;
+    for (int t = 1; t < nt; ++t) th.emplace_back(work);
+    work();
+    for (auto& x : th) x.join();
+}
+
+}  // namespace
+
+void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colidx, const double* X, int T,
+                       const int32_t* node0, double max_flops, FcPlan& plan) {
+    plan = FcPlan();
+    const int nc = N / G, gd = 3 * G;
+    plan.gd = gd;
+    // column graph (no self edges), global ids; a tissue's columns are consecutive
+    std::vector<int32_t> ptr(nc + 1, 0), adj;
+    {
+        std::vector<std::vector<int32_t>> part(T);
+        parallel_items(T, [&](int t) {
+            const int c0 = node0[t] / G, c1 = node0[t + 1] / G;
+            std::vector<int32_t> mark(c1 - c0, -1);
+            for (int c = c0; c < c1; ++c) {
+                const size_t before = part[t].size();
+                for (int i = c * G; i < (c + 1) * G; ++i)
+                    for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
+                        const int32_t d = colidx[k] / G;
+                        if (d != c && mark[d - c0] != c) {
+                            mark[d - c0] = c;
+                            part[t].push_back(d - c0);
+                        }
+                    }
+                ptr[c + 1] = (int32_t)(part[t].size() - before);
+            }
+        });
+        for (int c = 0; c < nc; ++c) ptr[c + 1] += ptr[c];
+        adj.reserve(ptr[nc]);
+        for (int t = 0; t < T; ++t) adj.insert(adj.end(), part[t].begin(), part[t].end());
+    }
+    std::vector<Dissection> ds(T);
+    parallel_items(T, [&](int t) {
+        const int c0 = node0[t] / G, c1 = node0[t + 1] / G;
+        Dissection& d = ds[t];
+        std::vector<int32_t> lp(c1 - c0 + 1);
+        for (int c = c0; c <= c1; ++c) lp[c - c0] = ptr[c] - ptr[c0];
+        d.ptr = lp.data();
+        d.adj = adj.data() + ptr[c0];
+        d.X = X + (size_t)c0 * 3;
+        d.leaf = std::max(1, kFcTile / gd);
+        d.run(c1 - c0);
+    });
+    // fronts of all tissues by depth
+    int depths = 0;
+    double flops = 0.0;
+    std::vector<std::vector<std::pair<int, int>>> at;  // per depth: (tissue, node)
+    for (int t = 0; t < T; ++t)
+        for (int k = 0; k < (int)ds[t].nodes.size(); ++k) {
+            const Node& f = ds[t].nodes[k];
+            if (f.depth >= depths) at.resize(depths = f.depth + 1);
+            at[f.depth].push_back({t, k});
+            const double p = (double)f.piv.size() * gd, b = (double)f.bnd.size() * gd;
+            flops += p * p * p * (2.0 / 3.0) + p * p * b + b * b * p;
+            if (p > kFcMaxPivots || p + b >= 65536) return;
+        }
+    plan.flops = flops;
+    if (flops > max_flops) return;
+    std::vector<std::vector<int32_t>> id(T);
+    for (int t = 0; t < T; ++t) id[t].resize(ds[t].nodes.size());
+    int nf = 0;
+    for (auto& level : at)
+        for (auto& q : level) id[q.first][q.second] = nf++;
+    plan.fronts.resize(nf);
+    plan.depths.resize(depths);
+    std::vector<std::pair<int, int>> of(nf);
+    int64_t n_map = 0, n_vert = 0;
+    for (int d = 0; d < depths; ++d) {
+        int64_t scratch = 0, contrib = 0, tp = 0;
+        for (auto& q : at[d]) {
+            const int fi = id[q.first][q.second];
+            of[fi] = q;
+            const Node& f = ds[q.first].nodes[q.second];
+            FcFront& F = plan.fronts[fi];
+            const int np = (int)f.piv.size(), nb = (int)f.bnd.size();
+            F.p = np * gd;
+            F.b = nb * gd;
+            F.ldp = (F.p + 1) & ~1;
+            F.ldb = (F.b + 1) & ~1;
+            F.tissue = q.first;
+            F.verts = (int32_t)n_vert;
+            n_vert += np + nb;
+            for (int k = 0; k < 2; ++k) {
+                F.child[k] = f.child[k] >= 0 ? id[q.first][f.child[k]] : -1;
+                F.map[k] = (int32_t)n_map;
+                if (f.child[k] >= 0) n_map += np + nb;
+            }
+            F.vec = (int32_t)plan.n_vec;
+            F.piv = (int32_t)plan.n_piv;
+            plan.n_vec += F.b;
+            plan.n_piv += F.ldp;
+            F.x11 = plan.n_factor;
+            F.l21 = F.x11 + (int64_t)F.p * F.ldp;
+            plan.n_factor = F.l21 + (int64_t)F.b * F.ldp;
+            F.a21 = scratch;
+            F.lp = F.a21 + (int64_t)F.b * F.ldp;
+            scratch = F.lp + (F.p > kFcTile ? (int64_t)F.p * kFcTile : 0);
+            F.c = contrib;
+            contrib += (int64_t)F.b * F.ldb;
+            F.tp = tp;
+            tp += (int64_t)((F.b + kFcBackRows - 1) / kFcBackRows) * F.ldp;
+            if (d == 0) plan.n_root += F.p;
+        }
+        plan.n_scratch = std::max(plan.n_scratch, scratch);
+        plan.n_contrib[d & 1] = std::max(plan.n_contrib[d & 1], contrib);
+        plan.n_tp = std::max(plan.n_tp, tp);
+    }
+    if (n_map > INT32_MAX || n_vert > INT32_MAX || plan.n_vec > INT32_MAX || plan.n_piv > INT32_MAX) return;
+    plan.maps.resize(n_map);
+    plan.verts.resize(n_vert);
+    // columns, child maps and Jacobian blocks of every front
+    std::vector<std::vector<int2>> jb(nf);
+    const int step = 64;
+    parallel_items((nf + step - 1) / step, [&](int chunk) {
+        std::vector<int32_t> where;  // position in the front's column list, by local column
+        for (int fi = chunk * step; fi < std::min(nf, (chunk + 1) * step); ++fi) {
+            const int t = of[fi].first;
+            const Dissection& D = ds[t];
+            const Node& f = D.nodes[of[fi].second];
+            FcFront& F = plan.fronts[fi];
+            const int c0 = node0[t] / G, np = (int)f.piv.size(), nb = (int)f.bnd.size();
+            if ((int)where.size() < (int)D.perm.size()) where.resize(D.perm.size());
+            for (int k = 0; k < np + nb; ++k) {
+                const int32_t v = k < np ? f.piv[k] : f.bnd[k - np];
+                plan.verts[F.verts + k] = v + c0;
+                where[v] = k;
+            }
+            for (int q = 0; q < 2; ++q) {
+                if (f.child[q] < 0) continue;
+                const Node& c = D.nodes[f.child[q]];
+                int32_t* m = plan.maps.data() + F.map[q];
+                std::fill(m, m + np + nb, -1);
+                for (int k = 0; k < (int)c.bnd.size(); ++k) m[where[c.bnd[k]]] = k;
+            }
+            const int32_t first = np ? D.pos[f.piv[0]] : 0;
+            for (int k = 0; k < np; ++k)
+                for (int a = 0; a < G; ++a) {
+                    const int node = (f.piv[k] + c0) * G + a;
+                    for (int32_t e = rowptr[node]; e < rowptr[node + 1]; ++e) {
+                        const int32_t other = colidx[e], v = other / G - c0;
+                        const int32_t pv = D.pos[v], pk = D.pos[f.piv[k]];
+                        if (pv < first || pv < pk || (pv == pk && other < node)) continue;
+                        const int row = where[v] * gd + (other % G) * 3, col = k * gd + a * 3;
+                        jb[fi].push_back(make_int2(e, (int)((uint32_t)row << 16 | (uint32_t)col)));
+                    }
+                }
+        }
+    });
+    int64_t nj = 0;
+    for (int fi = 0; fi < nf; ++fi) {
+        plan.fronts[fi].j0 = (int32_t)nj;
+        nj += (int64_t)jb[fi].size();
+        plan.fronts[fi].j1 = (int32_t)nj;
+    }
+    if (nj > INT32_MAX) return;
+    plan.jblk.resize(nj);
+    parallel_items((nf + step - 1) / step, [&](int chunk) {
+        for (int fi = chunk * step; fi < std::min(nf, (chunk + 1) * step); ++fi)
+            std::copy(jb[fi].begin(), jb[fi].end(), plan.jblk.begin() + plan.fronts[fi].j0);
+    });
+    // task lists, the tasks of a launch by falling front size (the long ones start first)
+    auto cdiv = [](int a, int b) { return (a + b - 1) / b; };
+    for (int d = 0; d < depths; ++d) {
+        FcDepth& L = plan.depths[d];
+        std::vector<int32_t> fs;
+        for (auto& q : at[d]) fs.push_back(id[q.first][q.second]);
+        std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) { return plan.fronts[a].p > plan.fronts[b].p; });
+        auto list = [&](FcRange& r, auto emit) {
+            r.begin = (int32_t)plan.tasks.size();
+            for (int32_t fi : fs) emit(fi, plan.fronts[fi]);
+            r.count = (int32_t)plan.tasks.size() - r.begin;
+        };
+        auto push = [&](int32_t f, int i, int j) { plan.tasks.push_back(FcTask{f, (int16_t)i, (int16_t)j}); };
+        list(L.gather, [&](int32_t fi, const FcFront& F) {
+            if (F.p > 0)
+                for (int i = 0; i < cdiv(F.p + F.b, kFcGatherRows); ++i) push(fi, i, 0);
+        });
+        list(L.scatter, [&](int32_t fi, const FcFront& F) {
+            for (int i = 0; i < cdiv(F.j1 - F.j0, kFcScatter); ++i) push(fi, i, 0);
+        });
+        list(L.diag, [&](int32_t fi, const FcFront& F) {
+            if (F.p > 0) push(fi, 0, 0);
+        });
+        int np = 0;
+        for (int32_t fi : fs) np = std::max(np, cdiv(plan.fronts[fi].p, kFcTile));
+        plan.chain += np;
+        L.panel0 = (int32_t)plan.panels.size();
+        L.n_panel = std::max(0, np);
+        for (int k = 0; k < np; ++k) {
+            FcPanel P;
+            // panel k of a front with nt panels: the column below the diagonal block (rows i > k), the
+            // inverse's row k (columns j < k); then every tile below row k
+            list(P.col, [&](int32_t fi, const FcFront& F) {
+                const int nt = cdiv(F.p, kFcTile);
+                if (nt <= k) return;
+                for (int i = 0; i < nt; ++i)
+                    if (i != k) push(fi, i, 0);
+            });
+            list(P.upd, [&](int32_t fi, const FcFront& F) {
+                const int nt = cdiv(F.p, kFcTile);
+                // the next diagonal block first: its factorisation is the long one
+                if (k + 1 < nt) push(fi, k + 1, k + 1);
+                for (int i = k + 1; i < nt; ++i)
+                    for (int j = 0; j <= i; ++j)
+                        if (!(i == k + 1 && j == k + 1)) push(fi, i, j);
+            });
+            plan.panels.push_back(P);
+        }
+        list(L.l21, [&](int32_t fi, const FcFront& F) {
+            for (int i = 0; i < cdiv(F.b, kFcTile); ++i)
+                for (int j = cdiv(F.p, kFcTile) - 1; j >= 0; --j) push(fi, i, j);
+        });
+        list(L.schur, [&](int32_t fi, const FcFront& F) {
+            for (int i = 0; i < cdiv(F.b, kFcTile); ++i)
+                for (int j = 0; j <= i; ++j) push(fi, i, j);
+        });
+        list(L.fwd1, [&](int32_t fi, const FcFront& F) {
+            for (int i = cdiv(F.p, kFcRows) - 1; i >= 0; --i) push(fi, i, 0);
+        });
+        list(L.fwd2, [&](int32_t fi, const FcFront& F) {
+            for (int i = 0; i < cdiv(F.b, kFcRows); ++i) push(fi, i, 0);
+        });
+        list(L.bwd1, [&](int32_t fi, const FcFront& F) {
+            for (int i = 0; i < cdiv(F.b, kFcBackRows); ++i)
+                for (int j = 0; j < cdiv(F.p, kFcTile); ++j) push(fi, i, j);
+        });
+        list(L.bwd2, [&](int32_t fi, const FcFront& F) {
+            for (int i = 0; i < cdiv(F.p, kFcRows); ++i) push(fi, i, 0);
+        });
+    }
+    if (plan.tasks.size() > (size_t)INT32_MAX) return;
+    plan.ok = true;
+}
+
+}  // namespace tfb
