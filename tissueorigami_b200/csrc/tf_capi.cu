@@ -38,6 +38,9 @@ constexpr int kMlAutoNodes = 100000; // single tissues from this size take the m
 constexpr int kMlTopMaxAge = 8;      // solves between refreshes of the multilevel top inverse
 constexpr int kWarmSlots = 8;        // Newton iterations whose solutions are kept for warm starts
 constexpr int kFcMaxIters = 8;       // iterations after which a factorised solve counts as failed
+constexpr double kFcKeepFlops = 5e7; // factorisations from this size on are kept from the second Newton iteration
+                                     // (342 prisms, 1e7: 1.18 ms a step anew, 1.54 kept; 2,713 prisms,
+                                     // 2e8: 4.6 and 3.9; 79,650 prisms, 4.3e10: 26.5 and 19.6)
 constexpr double kFcMaxFlops = 4e11; // largest factorisation (operations of one tissue, or mean of a batch)
 
 struct DevBuf {
@@ -174,9 +177,14 @@ struct tf_ctx {
     bool fc_ready = false;     // plan and buffers exist
     bool fc_used = false;      // the last solve was a factorised one
     bool fc_same = false;      // the factor on the device is of the current J (further right-hand sides)
+    bool fc_near = false;      // ... or of the J of an earlier iteration of this Newton loop, close to it
     std::vector<int32_t> fc_chunk0;
+    // the launches of a factorisation and of a solve are the same every time (50 to 300 short kernels
+    // whose launch alone, 3.4 us each, took longer than many of them): replayed as graphs (0.75 us each)
+    cudaGraphExec_t fc_graph[2] = {nullptr, nullptr};
+    int64_t fc_graph_launches[2] = {0, 0};
     DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_tp, fc_vec, fc_z,
-        fc_sign, fc_flags, fc_chunks, fc_chunk0_d, fc_running, fc_part;
+        fc_sign, fc_flags, fc_neg, fc_chunks, fc_chunk0_d, fc_running, fc_part;
 
     // adjoint: forward checkpoints every adj_k steps, segment recompute buffers, adjoint state
     int32_t adj_steps = 0, adj_k = 0;
@@ -1686,9 +1694,41 @@ bool factor_wanted(const tf_ctx* c) {
            c->params.krylov_warm_start && !(c->pk_on && c->pk_pairs_n > 0);
 }
 
+void drop_factor_graphs(tf_ctx* c) {
+    for (auto& g : c->fc_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
+// Runs `launch` (which adds its kernels to the counter it is given) on the context's stream, as a
+// graph captured the first time.
+template <class F>
+int replay_factor(tf_ctx* ctx, int which, F launch) {
+    if (!ctx->params.use_graphs) {
+        TF_CK(launch(&ctx->launches));
+        return TF_OK;
+    }
+    if (!ctx->fc_graph[which]) {
+        cudaGraph_t graph = nullptr;
+        ctx->fc_graph_launches[which] = 0;
+        TF_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+        const cudaError_t lerr = launch(&ctx->fc_graph_launches[which]);
+        cudaError_t cerr = cudaStreamEndCapture(ctx->stream, &graph);
+        if (lerr == cudaSuccess && cerr == cudaSuccess) cerr = cudaGraphInstantiate(&ctx->fc_graph[which], graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        TF_CK(lerr);
+        TF_CK(cerr);
+    }
+    TF_CK(cudaGraphLaunch(ctx->fc_graph[which], ctx->stream));
+    ctx->launches += ctx->fc_graph_launches[which];
+    return TF_OK;
+}
+
 int build_factor(tf_ctx* ctx) {
     ctx->fc_dirty = false;
     ctx->fc_ready = false;
+    drop_factor_graphs(ctx);
     const int N = ctx->N, T = ctx->T;
     int G = std::max(ctx->col_G, 1);
     for (int t = 0; t < T; ++t)
@@ -1732,6 +1772,7 @@ int build_factor(tf_ctx* ctx) {
     }
     TF_CK(e);
     TF_CK(dalloc(ctx->fc_flags, sizeof(int32_t) * T));
+    TF_CK(dalloc(ctx->fc_neg, sizeof(int32_t) * P.fronts.size()));
     TF_CK(dalloc(ctx->fc_running, sizeof(int32_t) * T));
     TF_CK(up(ctx->fc_fronts, P.fronts.data(), sizeof(FcFront) * P.fronts.size()));
     TF_CK(up(ctx->fc_maps, P.maps.data(), sizeof(int32_t) * P.maps.size()));
@@ -1767,6 +1808,7 @@ FcWork make_factor(tf_ctx* c) {
     f.z = dptr<double>(c->fc_z);
     f.sign = dptr<double>(c->fc_sign);
     f.flags = dptr<int32_t>(c->fc_flags);
+    f.neg = dptr<int32_t>(c->fc_neg);
     return f;
 }
 
@@ -1787,21 +1829,25 @@ int factor_solve(tf_ctx* ctx, bool* done) {
     c.active = dptr<int32_t>(ctx->active_d);
     c.running = dptr<int32_t>(ctx->fc_running);
     c.part = dptr<double>(ctx->fc_part);
-    if (!ctx->fc_same) {
+    const bool kept = ctx->fc_same || ctx->fc_near;
+    if (!kept) {
         TF_CK(cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream));
-        TF_CK(launch_factor(ctx->fc, f, w.vals, &ctx->launches, ctx->stream));
+        TF_CK(cudaMemsetAsync(ctx->fc_neg.p, 0, sizeof(int32_t) * ctx->fc.fronts.size(), ctx->stream));
+        const int rc = replay_factor(ctx, 0, [&](int64_t* n) { return launch_factor(ctx->fc, f, w.vals, n, ctx->stream); });
+        if (rc != TF_OK) return rc;
         ++ctx->coarse_refreshes;
     }
     const int cap = std::min(kFcMaxIters, ctx->params.krylov_max_iters);
     TF_CK(launch_fc_start(w, c, ctx->params.krylov_rtol, cap, ctx->stream));
-    ctx->launches += 2;
+    ctx->launches += 1;
     f.active = c.running;
     double* z = w.phat;
     bool running = true;
     for (int it = 0; it < cap && running; ++it) {
-        TF_CK(launch_factor_solve(ctx->fc, f, w.r, z, &ctx->launches, ctx->stream));
-        TF_CK(launch_fc_iteration(w, c, z, w.v, ctx->stream));
-        ctx->launches += 5;
+        const int rc = replay_factor(ctx, 1, [&](int64_t* n) { return launch_factor_solve(ctx->fc, f, w.r, z, n, ctx->stream); });
+        if (rc != TF_OK) return rc;
+        ctx->launches += launch_fc_iteration(w, c, it == 0, z, w.v, ctx->stream);
+        TF_CK(cudaGetLastError());
         TF_CK(cudaMemcpyAsync(ctx->h_tsc, ctx->tscalars.p, sizeof(KrylovScalars) * ctx->T, cudaMemcpyDeviceToHost, ctx->stream));
         TF_CK(cudaStreamSynchronize(ctx->stream));
         running = false;
@@ -1810,8 +1856,11 @@ int factor_solve(tf_ctx* ctx, bool* done) {
                 const int st = ctx->h_tsc[t].status;
                 if (st == KS_RUNNING)
                     running = true;
-                else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters))
-                    return TF_OK;
+                else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters)) {
+                    if (!ctx->fc_near) return TF_OK;
+                    ctx->fc_near = false;  // the kept factor does not fit: with one of this J
+                    return factor_solve(ctx, done);
+                }
             }
     }
     *ctx->h_sc = ctx->h_tsc[0];
@@ -2125,7 +2174,12 @@ int newton_core(tf_ctx* ctx, double dt, tf_step_stats* st) {
         if (rc != TF_OK) return rc;
         TF_CK(cudaEventRecord(ctx->ev[2], ctx->stream));
         ctx->warm_k = ctx->warm_call && T == 1 ? ctx->t_iters[0] : -1;
+        // From the third iteration on the iterate moves by under 1e-3 of the second update, and the
+        // factor of the second iteration's J still preconditions: four iterations there, three in the
+        // fourth Newton iteration, instead of a factorisation each.
+        ctx->fc_near = round >= 2 && ctx->fc_used && ctx->fc.flops >= kFcKeepFlops;
         rc = newton_solve(ctx);
+        ctx->fc_near = false;
         ctx->warm_k = -1;
         if (rc != TF_OK) return rc;
         KrylovWork w = make_work(ctx);
@@ -2639,8 +2693,9 @@ void tf_destroy(tf_ctx* ctx) {
     for (DevBuf* b : mlb) dfree(*b);
     DevBuf* fcb[] = {&ctx->fc_fronts, &ctx->fc_maps, &ctx->fc_verts, &ctx->fc_jblk, &ctx->fc_tasks, &ctx->fc_factor,
                      &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1], &ctx->fc_tp, &ctx->fc_vec, &ctx->fc_z,
-                     &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
+                     &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_neg, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
     for (DevBuf* b : fcb) dfree(*b);
+    drop_factor_graphs(ctx);
     if (ctx->h_coarse_info) cudaFreeHost(ctx->h_coarse_info);
     if (ctx->h_active) cudaFreeHost(ctx->h_active);
     if (ctx->h_du2) cudaFreeHost(ctx->h_du2);

@@ -20,7 +20,7 @@ constexpr int kT = kFcTile;
 constexpr int kLd = kT + 4;  // shared leading dimension: 8-byte reads of a fragment hit distinct banks
 constexpr int kKc = 16;      // K extent of one stage of the long GEMMs
 constexpr int kKld = kKc + 4;
-constexpr int kStages = 3;
+constexpr int kStages = 2;
 
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -52,9 +52,8 @@ __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int pari
 #pragma unroll
     for (int q = 0; q < 2; ++q)
         if (F.child[q] >= 0) {
-            const FcFront& ch = w.fronts[F.child[q]];
-            C[q] = w.contrib[parity ^ 1] + ch.c;
-            ldc[q] = ch.ldb;
+            C[q] = w.contrib[parity ^ 1] + F.child_c[q];
+            ldc[q] = F.child_ldb[q];
         }
     for (int c = threadIdx.x; c < F.p; c += blockDim.x) {
         const int v = c / w.gd, r = c - v * w.gd;
@@ -81,12 +80,12 @@ __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int pari
             }
         const int n = row < F.p ? row + 1 : F.p;
         double* out = row < F.p ? w.factor + F.x11 + (size_t)row * F.ldp : w.scratch + F.a21 + (size_t)(row - F.p) * F.ldp;
+#pragma unroll 4
         for (int c = lane; c < n; c += 32) {
             const int2 m = s_col[c];
-            double s = 0.0;
-            if (R[0] && m.x >= 0) s = R[0][m.x];
-            if (R[1] && m.y >= 0) s += R[1][m.y];
-            out[c] = s;
+            const double s0 = R[0] && m.x >= 0 ? R[0][m.x] : 0.0;
+            const double s1 = R[1] && m.y >= 0 ? R[1][m.y] : 0.0;
+            out[c] = s0 + s1;
         }
     }
 }
@@ -110,81 +109,145 @@ __global__ void __launch_bounds__(256) k_fc_scatter(FcWork w, const double* __re
 
 // ---- pivot block -----------------------------------------------------------------------------
 
-// LDL^T of the 64 x 64 block whose lower triangle is in s (rows / columns from n on: the identity), by
-// the row operations that also turn the identity into L^-1, in place: 256 threads, thread 4 r + q holds
-// row r, columns q, q + 4, ... A chain of 64 steps (one shared row exchange each) bounds it.
-// Writes G^-1 = |D|^-1/2 L^-1 (upper triangle zero) to out and sign(D) to sign.
-__device__ void factor_block(double (*s)[kLd], int n, double* out, int ld, double* sign, int32_t* flag) {
-    __shared__ double s_row[2][kT];
-    __shared__ double s_d[kT];
-    const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
-    double v[16];
+// LDL^T of an n x n block (n <= 64, its lower triangle in s, rows of ld), by the row operations that also
+// turn the identity into L^-1, in place: 8 warps, warp w holds rows 8 w .. 8 w + 7 as the accumulator
+// fragments of eight 8 x 8 tiles. Per block of 8 pivots every warp below it eliminates the pivot tile
+// and its own tile of those columns by shuffles (the pivot tile redundantly, so that the 8 steps need no
+// barrier), and its other tiles by two tensor instructions each. Returns the rows of
+// G^-1 = |D|^-1/2 L^-1 (zero right of the diagonal and outside the block) and writes sign(D).
+// Bound by the chain of 8 steps (a shuffle, a reciprocal and two FP64 operations, ~125 cycles each). A row
+// per four threads with the pivot row read from shared memory took 571 cycles a step (64 pivots:
+// 36.6 k): 256 threads x 16 entries a step is 256 cycles of shared-memory reads alone.
+struct __align__(16) FactorShared {
+    double rows[2][8][kLd];
+    double d[kT];
+};
+__device__ __forceinline__ void factor_block(const double* s, int ld, int n, FactorShared& sh, double (&v)[8][2], double* sign,
+                                             int32_t* flag, int32_t* neg) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, lr = lane >> 2, lk = lane & 3, r = 8 * w + lr;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        const int c = 4 * k + q;
-        v[k] = r < n && c < n ? (c <= r ? s[r][c] : s[c][r]) : (r == c ? 1.0 : 0.0);
-    }
-    bool bad = false;
+    for (int t = 0; t < 8; ++t)
 #pragma unroll
-    for (int jk = 0; jk < 16; ++jk) {
-        for (int jq = 0; jq < 4; ++jq) {
-            const int j = 4 * jk + jq, buf = j & 1;
-            if (r == j) {
+        for (int h = 0; h < 2; ++h) {
+            const int c = 8 * t + 2 * lk + h;
+            v[t][h] = r < n && c < n ? (c <= r ? s[r * ld + c] : s[c * ld + r]) : (r == c ? 1.0 : 0.0);
+        }
 #pragma unroll
-                for (int k = 0; k < 16; ++k) s_row[buf][4 * k + q] = v[k];
+    for (int kb = 0; kb < 8; ++kb) {
+        if (8 * kb >= n) break;
+        double(*rows)[kLd] = sh.rows[kb & 1];
+        if (w == kb) {
+#pragma unroll
+            for (int t = 0; t < 8; ++t) *reinterpret_cast<double2*>(&rows[lr][8 * t + 2 * lk]) = make_double2(v[t][0], v[t][1]);
+        }
+        __syncthreads();
+        if (w < kb) continue;
+        double D[2] = {rows[lr][8 * kb + 2 * lk], rows[lr][8 * kb + 2 * lk + 1]};
+        double O[2] = {v[kb][0], v[kb][1]};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double d = __shfl_sync(0xffffffffu, D[j & 1], 4 * j + (j >> 1));
+            const double p0 = __shfl_sync(0xffffffffu, D[0], 4 * j + lk), p1 = __shfl_sync(0xffffffffu, D[1], 4 * j + lk);
+            const double aD = __shfl_sync(0xffffffffu, D[j & 1], (lane & 28) + (j >> 1));
+            const double aO = __shfl_sync(0xffffffffu, O[j & 1], (lane & 28) + (j >> 1));
+            const double inv = __drcp_rn(d);
+            const double mD = aD * inv, mO = aO * inv;
+            O[0] -= mO * p0;
+            O[1] -= mO * p1;
+            if (lr > j) {
+                D[0] -= mD * p0;
+                D[1] -= mD * p1;
             }
-            __syncthreads();
-            const double d = s_row[buf][j];
-            if (threadIdx.x == 0) s_d[j] = d;
-            if (!(fabs(d) > 0.0) || !isfinite(d)) bad = true;
-            const double a = __shfl_sync(0xffffffffu, v[jk], (threadIdx.x & 28) | jq);
-            if (r > j) {
-                const double m = a / d;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const int c = 4 * k + q;
-                    v[k] = c == j ? -m : v[k] - m * s_row[buf][c];
-                }
+            if (lk == (j >> 1)) {
+                O[j & 1] = -mO;
+                if (lr > j) D[j & 1] = -mD;
             }
+            if (w == kb && lane == 0) sh.d[8 * kb + j] = d;
+        }
+        if (w == kb) {
+            O[0] = D[0];
+            O[1] = D[1];
+        }
+        v[kb][0] = O[0];
+        v[kb][1] = O[1];
+        // the tile as an A fragment: below the pivots minus the multipliers of the published rows; for the pivot
+        // rows L^-1 itself (unit diagonal)
+        double a[2];
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            const int src = (lane & 28) + 2 * f + (lk >> 1), k = 4 * f + lk;
+            const double x0 = __shfl_sync(0xffffffffu, O[0], src), x1 = __shfl_sync(0xffffffffu, O[1], src);
+            a[f] = lk & 1 ? x1 : x0;
+            if (w == kb) a[f] = k < lr ? a[f] : (k == lr ? 1.0 : 0.0);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            if (t == kb) continue;
+            if (w == kb) v[t][0] = v[t][1] = 0.0;
+            mma_f64(v[t], a[0], rows[lk][8 * t + lr]);
+            mma_f64(v[t], a[1], rows[4 + lk][8 * t + lr]);
         }
     }
     __syncthreads();
-    // row r now holds L^-1 left of the diagonal
-    const double d = s_d[r];
-    const double g = 1.0 / sqrt(fabs(d));
-    if (r < n) {
+    const double d = r < n ? sh.d[r] : 1.0;
+    const double g = r < n ? 1.0 / sqrt(fabs(d)) : 0.0;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const int c = 4 * k + q;
-            if (c < n) out[(size_t)r * ld + c] = c < r ? v[k] * g : (c == r ? g : 0.0);
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = 8 * t + 2 * lk + h;
+            v[t][h] = c < r ? v[t][h] * g : (c == r ? g : 0.0);
         }
-        if (q == 0) sign[r] = d < 0.0 ? -1.0 : 1.0;
+    if (r < n && lk == 0) {
+        sign[r] = d < 0.0 ? -1.0 : 1.0;
+        if (d < 0.0) *neg = 1;
+        if (!(fabs(d) > 0.0) || !isfinite(d)) *flag = 1;
     }
-    if (bad && threadIdx.x == 0) *flag = 1;
+}
+
+// factor_block's rows to memory (rows and columns below n).
+__device__ __forceinline__ void store_rows(const double (&v)[8][2], int n, double* out, int ld) {
+    const int lane = threadIdx.x & 31, r = 8 * (threadIdx.x >> 5) + (lane >> 2);
+    if (r >= n) return;
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = 8 * t + 2 * (lane & 3) + h;
+            if (c < n) out[(size_t)r * ld + c] = v[t][h];
+        }
+}
+
+// A 64 x 64 tile of a matrix with `rows` x `cols` valid entries at src (its rows 16-byte aligned) into
+// shared memory, zero outside, by asynchronous copies of two entries: both tiles of a product are
+// in flight together. Follow with tile_wait.
+__device__ __forceinline__ void load_tile(double (*s)[kLd], const double* src, int ld, int rows, int cols) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int id = threadIdx.x + e * 256, r = id >> 5, c = (id & 31) * 2, left = r < rows ? cols - c : 0;
+        const int bytes = left >= 2 ? 16 : (left > 0 ? 8 : 0);
+        cp_async16(&s[r][c], bytes ? src + (size_t)r * ld + c : src, bytes);
+    }
+}
+__device__ __forceinline__ void tile_wait() {
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
 }
 
 __global__ void __launch_bounds__(256) k_fc_diag(FcWork w, int begin) {
-    __shared__ double s[kT][kLd];
+    __shared__ __align__(16) double s[kT][kLd];
+    __shared__ FactorShared sh;
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
     double* A = w.factor + F.x11;
     const int n = min(kT, F.p);
-    for (int e = threadIdx.x; e < n * kT; e += blockDim.x) {
-        const int r = e / kT, c = e - r * kT;
-        if (c <= r) s[r][c] = A[(size_t)r * F.ldp + c];
-    }
-    __syncthreads();
-    factor_block(s, n, A, F.ldp, w.sign + F.piv, w.flags + F.tissue);
-}
-
-// A 64 x 64 tile of a matrix with `rows` x `cols` valid entries at src into shared memory (zero
-// outside), optionally its columns times sign.
-__device__ __forceinline__ void load_tile(double (*s)[kLd], const double* src, int ld, int rows, int cols) {
-    for (int e = threadIdx.x; e < kT * kT; e += 256) {
-        const int r = e >> 6, c = e & 63;
-        s[r][c] = r < rows && c < cols ? src[(size_t)r * ld + c] : 0.0;
-    }
+    load_tile(s, A, F.ldp, n, n);  // above the diagonal: not initialised, and not read
+    tile_wait();
+    double v[8][2];
+    factor_block(&s[0][0], kLd, n, sh, v, w.sign + F.piv, w.flags + F.tissue, w.neg + tk.front);
+    store_rows(v, n, A, F.ldp);
 }
 
 // 64 x 64 x 64 product of two shared tiles by 8 warps (16 x 32 each): acc = A B^T (BT: B as [col][k]) or
@@ -224,40 +287,84 @@ __device__ __forceinline__ void tile_each(double (&acc)[2][4][2], F f) {
             for (int h = 0; h < 2; ++h) f(r0 + 8 * i, c0 + 8 * j + h, acc[i][j][h]);
 }
 
+__device__ __forceinline__ void tile_sub(double (&a)[2][4][2], const double (&b)[2][4][2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) a[i][j][h] -= b[i][j][h];
+}
+
 constexpr int kPanelSmem = 2 * kT * kLd * (int)sizeof(double);
 
-// Panel k, G_k^-1 known: task i > k: L_ik = A_ik G_k^-T S_k into the panel scratch; i < k: the inverse's
-// row panel, X_ki = G_k^-1 X_ki in place.
+// Panel k, G_k^-1 known. Task (i > k, part): 16 rows of L_ik = A_ik G_k^-T S_k into the panel scratch; (i < k, part): 16
+// columns of the inverse's row panel, X_ki = G_k^-1 X_ki in place. Quarter tiles: these launches are on the
+// critical path with few tiles (22 tiles of the wing disc's second depth: 9.4 us whole).
 __global__ void __launch_bounds__(256) k_fc_col(FcWork w, int begin, int k) {
     extern __shared__ double s_dyn[];
     double(*sA)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn);
     double(*sB)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn + kT * kLd);
-    const FcTask tk = w.tasks[begin + blockIdx.x];
+    const FcTask tk = w.tasks[begin + (blockIdx.x >> 2)];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
     double* X = w.factor + F.x11;
-    const int i = tk.i, nk = min(kT, F.p - k * kT), ni = min(kT, F.p - i * kT);
+    const int i = tk.i, part = (blockIdx.x & 3) * 16, nk = min(kT, F.p - k * kT), ni = min(kT, F.p - i * kT);
     const double* Gk = X + (size_t)k * kT * F.ldp + k * kT;
-    double acc[2][4][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lk = lane & 3;
     if (i > k) {
-        load_tile(sA, X + (size_t)i * kT * F.ldp + k * kT, F.ldp, ni, nk);
+        if (part >= ni) return;
+        const double* A = X + ((size_t)i * kT + part) * F.ldp + k * kT;
+        {
+            const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;  // 16 rows x 64 columns
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int left = part + r < ni ? nk - (c + 2 * h) : 0, bytes = left >= 2 ? 16 : (left > 0 ? 8 : 0);
+                cp_async16(&sA[r][c + 2 * h], bytes ? A + (size_t)r * F.ldp + c + 2 * h : A, bytes);
+            }
+        }
         load_tile(sB, Gk, F.ldp, nk, nk);
-        __syncthreads();
-        tile_mma<true>(sA, sB, acc);
-        double* lp = w.scratch + F.lp + (size_t)i * kT * kT;
+        tile_wait();
+        double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};  // warp: columns 8 warp .. 8 warp + 7, 16 rows
+        const int kend = min(kT, 8 * warp + 8);       // G_k^-1 is lower triangular
+        for (int q = lk; q < kend; q += 4) {
+            const double b = sB[8 * warp + lr][q];
+            mma_f64(acc[0], sA[lr][q], b);
+            mma_f64(acc[1], sA[8 + lr][q], b);
+        }
+        double* lp = w.scratch + F.lp + ((size_t)i * kT + part) * kT;
         const double* sg = w.sign + F.piv + k * kT;
-        tile_each(acc, [&](int r, int c, double v) {
-            if (r < ni) lp[r * kT + c] = c < nk ? v * sg[c] : 0.0;
-        });
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = 8 * x + lr, c = 8 * warp + 2 * lk + h;
+                if (part + r < ni) lp[r * kT + c] = c < nk ? acc[x][h] * sg[c] : 0.0;
+            }
     } else {
-        double* Xk = X + (size_t)k * kT * F.ldp + i * kT;
+        double* Xk = X + (size_t)k * kT * F.ldp + i * kT + part;
+        {
+            const int r = threadIdx.x >> 2, c = (threadIdx.x & 3) * 4;  // 64 rows x 16 columns
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                cp_async16(&sB[r][c + 2 * h], r < nk ? Xk + (size_t)r * F.ldp + c + 2 * h : Xk, r < nk ? 16 : 0);
+        }
         load_tile(sA, Gk, F.ldp, nk, nk);
-        load_tile(sB, Xk, F.ldp, nk, kT);
-        __syncthreads();
-        tile_mma<false>(sA, sB, acc);
-        tile_each(acc, [&](int r, int c, double v) {
-            if (r < nk) Xk[(size_t)r * F.ldp + c] = v;
-        });
+        tile_wait();
+        double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};  // warp: rows 8 warp .. 8 warp + 7, 16 columns
+        const int kend = min(kT, 8 * warp + 8);
+        for (int q = lk; q < kend; q += 4) {
+            const double a = sA[8 * warp + lr][q];
+            mma_f64(acc[0], a, sB[q][lr]);
+            mma_f64(acc[1], a, sB[q][8 + lr]);
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = 8 * warp + lr, c = 8 * x + 2 * lk + h;
+                if (r < nk) Xk[(size_t)r * F.ldp + c] = acc[x][h];
+            }
     }
 }
 
@@ -265,6 +372,7 @@ __global__ void __launch_bounds__(256) k_fc_col(FcWork w, int begin, int k) {
 // The tile that is the next diagonal block is factorised at once.
 __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
     extern __shared__ double s_dyn[];
+    __shared__ FactorShared sh;
     double(*sA)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn);
     double(*sB)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn + kT * kLd);
     const FcTask tk = w.tasks[begin + blockIdx.x];
@@ -275,50 +383,231 @@ __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
     const int ni = min(kT, F.p - i * kT), nj = min(kT, F.p - j * kT), nk = min(kT, F.p - k * kT);
     const double* lp = w.scratch + F.lp;
     double* out = X + (size_t)i * kT * F.ldp + j * kT;
-    double acc[2][4][2];
+    double acc[2][4][2], old[2][4][2];
+    tile_each(old, [&](int r, int c, double& v) {  // in flight during the product
+        v = j != k && r < ni && c < nj && (i != j || c <= r) ? out[(size_t)r * F.ldp + c] : 0.0;
+    });
     load_tile(sA, lp + (size_t)i * kT * kT, kT, ni, nk);
     if (j > k) {
         const double* sg = w.sign + F.piv + k * kT;
-        const double* lj = lp + (size_t)j * kT * kT;
-        for (int e = threadIdx.x; e < kT * kT; e += 256) {
-            const int r = e >> 6, c = e & 63;
-            sB[r][c] = r < nj && c < nk ? lj[r * kT + c] * sg[c] : 0.0;
+        load_tile(sB, lp + (size_t)j * kT * kT, kT, nj, nk);
+        tile_wait();
+        if (w.neg[tk.front]) {
+            for (int e = threadIdx.x; e < kT * kT; e += 256) sB[e >> 6][e & 63] *= (e & 63) < nk ? sg[e & 63] : 0.0;
+            __syncthreads();
         }
-        __syncthreads();
         tile_mma<true>(sA, sB, acc);
         if (i == k + 1 && j == k + 1) {
             __syncthreads();
-            tile_each(acc, [&](int r, int c, double v) {
-                if (r < ni && c <= r) sA[r][c] = out[(size_t)r * F.ldp + c] - v;
-            });
+            tile_sub(old, acc);
+            tile_each(old, [&](int r, int c, double v) { sA[r][c] = v; });
             __syncthreads();
-            factor_block(sA, ni, out, F.ldp, w.sign + F.piv + i * kT, w.flags + F.tissue);
+            double v[8][2];
+            factor_block(&sA[0][0], kLd, ni, sh, v, w.sign + F.piv + i * kT, w.flags + F.tissue, w.neg + tk.front);
+            store_rows(v, ni, out, F.ldp);
         } else {
-            tile_each(acc, [&](int r, int c, double v) {
-                if (r < ni && c < nj && (i != j || c <= r)) out[(size_t)r * F.ldp + c] -= v;
+            tile_sub(old, acc);
+            tile_each(old, [&](int r, int c, double v) {
+                if (r < ni && c < nj && (i != j || c <= r)) out[(size_t)r * F.ldp + c] = v;
             });
         }
         return;
     }
     load_tile(sB, X + (size_t)k * kT * F.ldp + j * kT, F.ldp, nk, j == k ? nk : kT);
-    __syncthreads();
+    tile_wait();
     tile_mma<false>(sA, sB, acc);
     if (j == k)
         tile_each(acc, [&](int r, int c, double v) {
             if (r < ni && c < nk) out[(size_t)r * F.ldp + c] = -v;
         });
-    else
-        tile_each(acc, [&](int r, int c, double v) {
-            if (r < ni) out[(size_t)r * F.ldp + c] -= v;
+    else {
+        tile_sub(old, acc);
+        tile_each(old, [&](int r, int c, double v) {
+            if (r < ni) out[(size_t)r * F.ldp + c] = v;
         });
+    }
+}
+
+// ---- small fronts --------------------------------------------------------------------------------
+
+// A front of at most 64 pivots and kFcSmallB boundary unknowns, all of it in one CTA: its [A11; A21] is
+// gathered, completed with the Jacobian's blocks, factorised and turned into l21 in shared memory, and the
+// contribution is formed from there. One launch per depth instead of five, and A21 never leaves the
+// SM; the bottom half of a tree is made of such fronts.
+// Dynamic shared memory: A11 / G^-1 and A21 / l21 (rows of ld doubles), the map of both children (ints).
+__device__ __host__ __forceinline__ int small_ld(int p) { return ((p + 15) & ~15) + 4; }
+__device__ __host__ __forceinline__ int small_smem(int p, int b) {
+    return (((p + 7) & ~7) + ((b + 31) & ~31)) * small_ld(p) * 8 + 2 * (p + b) * 4;
+}
+
+__global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __restrict__ vals, int begin, int parity) {
+    extern __shared__ __align__(16) double s_dyn[];
+    __shared__ FactorShared sh;
+    __shared__ double s_sign[kT];
+    const FcTask tk = w.tasks[begin + blockIdx.x];
+    const FcFront F = w.fronts[tk.front];
+    if (!w.active[F.tissue]) return;
+    const int p = F.p, b = F.b, n = p + b, ld = small_ld(p), p8r = (p + 7) & ~7, b32 = (b + 31) & ~31;
+    double* sX = s_dyn;
+    double* sL = sX + p8r * ld;
+    int* s_map = reinterpret_cast<int*>(sL + b32 * ld);  // [2][n]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double* C[2] = {nullptr, nullptr};
+    int ldc[2] = {0, 0};
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+        if (F.child[q] >= 0) {
+            C[q] = w.contrib[parity ^ 1] + F.child_c[q];
+            ldc[q] = F.child_ldb[q];
+        }
+    for (int e = tid; e < 2 * n; e += 256) {
+        const int q = e >= n, c = e - q * n;
+        int m = -1;
+        if (C[q]) {
+            const int v = c / w.gd, k = w.maps[F.map[q] + v];
+            if (k >= 0) m = k * w.gd + (c - v * w.gd);
+        }
+        s_map[e] = m;
+    }
+    for (int e = tid; e < (p8r + b32) * ld; e += 256) s_dyn[e] = 0.0;
+    __syncthreads();
+    {
+        const int n9 = (F.j1 - F.j0) * 9;
+#pragma unroll 4
+        for (int e = tid; e < n9; e += 256) {
+            const int k = e / 9, en = e - k * 9, cc = en / 3, rr = en - cc * 3;
+            const int2 jb = w.jblk[F.j0 + k];
+            const int row = (int)((uint32_t)jb.y >> 16) + rr, col = (jb.y & 0xffff) + cc;
+            (row < p ? sX + row * ld : sL + (row - p) * ld)[col] = vals[(size_t)jb.x * 9 + en];
+        }
+    }
+    __syncthreads();
+    if (C[0] || C[1]) {  // eight rows a warp pass, the loads of all of them in flight
+        for (int r0 = warp; r0 < n; r0 += 64)
+            for (int c = lane; c < p; c += 32) {
+                const int c0 = s_map[c], c1 = s_map[n + c];
+                double x[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int row = r0 + 8 * u;
+                    double s = 0.0;
+                    if (row < n && (row >= p || c <= row)) {
+                        const int m0 = s_map[row], m1 = s_map[n + row];
+                        if (m0 >= 0 && c0 >= 0) s = C[0][(size_t)m0 * ldc[0] + c0];
+                        if (m1 >= 0 && c1 >= 0) s += C[1][(size_t)m1 * ldc[1] + c1];
+                    }
+                    x[u] = s;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int row = r0 + 8 * u;
+                    if (row < n && (row >= p || c <= row)) (row < p ? sX + row * ld : sL + (row - p) * ld)[c] += x[u];
+                }
+            }
+        __syncthreads();
+    }
+    {
+        double v[8][2];
+        factor_block(sX, ld, p, sh, v, s_sign, w.flags + F.tissue, w.neg + tk.front);
+        store_rows(v, p, w.factor + F.x11, F.ldp);
+        const int r = 8 * warp + (lane >> 2);  // every row of s was read before factor_block's last barrier
+        if (r < p8r)
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (8 * t < p) *reinterpret_cast<double2*>(sX + r * ld + 8 * t + 2 * (lane & 3)) = make_double2(v[t][0], v[t][1]);
+        __syncthreads();
+        if (tid < p) w.sign[F.piv + tid] = s_sign[tid];
+    }
+    // l21 = A21 G^-T S, a strip of eight rows per warp: its A21 entries stay in registers, so it is
+    // overwritten in place
+    const int lr = lane >> 2, lk = lane & 3, p8 = (p + 7) >> 3;
+    for (int r0 = warp * 8; r0 < b; r0 += 64) {
+        double* strip = sL + (size_t)r0 * ld;
+        double a[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) a[k] = 4 * k < p ? strip[lr * ld + 4 * k + lk] : 0.0;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j >= p8) break;
+            double d[2] = {0.0, 0.0}, d2[2] = {0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < 2 * j + 2; k += 2) {
+                mma_f64(d, a[k], sX[(8 * j + lr) * ld + 4 * k + lk]);
+                mma_f64(d2, a[k + 1], sX[(8 * j + lr) * ld + 4 * k + 4 + lk]);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = 8 * j + 2 * lk + h;
+                if (c < p) {
+                    const double x = (d[h] + d2[h]) * s_sign[c];
+                    strip[lr * ld + c] = x;
+                    if (r0 + lr < b) w.factor[F.l21 + (size_t)(r0 + lr) * F.ldp + c] = x;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // contribution, 16 x 32 tiles of the lower triangle
+    const bool neg = w.neg[tk.front] != 0;
+    double* Cf = w.contrib[parity] + F.c;
+    int task = 0;
+    for (int i = 0; i * 16 < b; ++i)
+        for (int j = 0; j * 32 <= i * 16 + 15 && j * 32 < b; ++j, ++task) {
+            if ((task & 7) != warp) continue;
+            // the children's entries are fetched ahead of the product
+            double acc[2][4][2], kid[2][4][2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int r = i * 16 + 8 * x + lr, c = j * 32 + 8 * y + 2 * lk + h;
+                        double s = 0.0;
+                        if (r < b && c <= r) {
+                            const int r0 = s_map[p + r], c0 = s_map[p + c], r1 = s_map[n + p + r], c1 = s_map[n + p + c];
+                            if (r0 >= 0 && c0 >= 0) s = C[0][(size_t)r0 * ldc[0] + c0];
+                            if (r1 >= 0 && c1 >= 0) s += C[1][(size_t)r1 * ldc[1] + c1];
+                        }
+                        kid[x][y][h] = s;
+                        acc[x][y][h] = 0.0;
+                    }
+            const double* A = sL + (i * 16 + lr) * ld + lk;
+            const double* B = sL + (j * 32 + lr) * ld + lk;
+            for (int k = 0; k < p; k += 4) {
+                double av[2], bv[4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) av[x] = A[8 * x * ld + k];
+#pragma unroll
+                for (int y = 0; y < 4; ++y) bv[y] = B[8 * y * ld + k];
+                if (neg) {
+                    const double sg = k + lk < p ? s_sign[k + lk] : 0.0;
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) bv[y] *= sg;
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) mma_f64(acc[x][y], av[x], bv[y]);
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int r = i * 16 + 8 * x + lr, c = j * 32 + 8 * y + 2 * lk + h;
+                        if (r < b && c <= r) Cf[(size_t)r * F.ldb + c] = kid[x][y][h] - acc[x][y][h];
+                    }
+        }
 }
 
 // ---- boundary GEMMs ---------------------------------------------------------------------------
 
 // 64 x 64 tile of A B^T, both row-major with K contiguous, by 4 warps (32 x 32 each: 16 accumulator
 // tiles hide the tensor instruction's latency), K in stages of 16 through a 3-stage cp.async ring.
-// a_rows / b_rows: valid rows (0 outside); K: valid columns. SIGN: B's columns times sign.
-template <bool SIGN>
+// a_rows / b_rows: valid rows (0 outside); K: valid columns; B's columns times sign unless it is null.
 __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, const double* B, int ldb, int b_rows, int K,
                                           const double* sign, double* smem, double (&acc)[4][4][2]) {
     double* sa = smem;
@@ -360,7 +649,7 @@ __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, 
             for (int i = 0; i < 4; ++i) a[i] = pa[8 * i * kKld + k];
 #pragma unroll
             for (int j = 0; j < 4; ++j) b[j] = pb[8 * j * kKld + k];
-            if (SIGN) {
+            if (sign) {
                 const int kc = it * kKc + k + kk;
                 const double sg = kc < K ? sign[kc] : 0.0;
 #pragma unroll
@@ -385,7 +674,7 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
     if (!w.active[F.tissue]) return;
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.p - j * kT);
     double acc[4][4][2];
-    gemm_tile<false>(w.scratch + F.a21 + (size_t)i * kT * F.ldp, F.ldp, ni, w.factor + F.x11 + (size_t)j * kT * F.ldp, F.ldp, nj,
+    gemm_tile(w.scratch + F.a21 + (size_t)i * kT * F.ldp, F.ldp, ni, w.factor + F.x11 + (size_t)j * kT * F.ldp, F.ldp, nj,
                      min(F.p, (j + 1) * kT), nullptr, s_dyn, acc);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
@@ -422,16 +711,16 @@ __global__ void __launch_bounds__(128) k_fc_schur(FcWork w, int begin, int parit
     }
     double acc[4][4][2];
     const double* L = w.factor + F.l21;
-    gemm_tile<true>(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p, w.sign + F.piv, s_dyn, acc);
+    gemm_tile(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p,
+              w.neg[tk.front] ? w.sign + F.piv : nullptr, s_dyn, acc);
     __syncthreads();
     const double* C[2] = {nullptr, nullptr};
     int ldc[2] = {0, 0};
 #pragma unroll
     for (int q = 0; q < 2; ++q)
         if (F.child[q] >= 0) {
-            const FcFront& ch = w.fronts[F.child[q]];
-            C[q] = w.contrib[parity ^ 1] + ch.c;
-            ldc[q] = ch.ldb;
+            C[q] = w.contrib[parity ^ 1] + F.child_c[q];
+            ldc[q] = F.child_ldb[q];
         }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
@@ -464,7 +753,7 @@ __device__ __forceinline__ double from_children(const FcWork& w, const FcFront& 
     for (int q = 0; q < 2; ++q)
         if (F.child[q] >= 0) {
             const int k = w.maps[F.map[q] + v];
-            if (k >= 0) s += w.vec[w.fronts[F.child[q]].vec + k * w.gd + r];
+            if (k >= 0) s += w.vec[F.child_vec[q] + k * w.gd + r];
         }
     return s;
 }
@@ -475,14 +764,119 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// z = x11 v_P for 32 pivots, v_P the right-hand side plus the children's vectors.
+// The passes of a front that one CTA reads alone. Forward: z = x11 v_P, v_B = children - l21 z.
+__global__ void __launch_bounds__(256) k_fc_fwd(FcWork w, const double* __restrict__ in, int begin) {
+    extern __shared__ double s_v[];  // v_P, then z
+    const FcTask tk = w.tasks[begin + blockIdx.x];
+    const FcFront F = w.fronts[tk.front];
+    if (!w.active[F.tissue]) return;
+    double* s_z = s_v + F.p;
+    for (int c = threadIdx.x; c < F.p; c += 256) {
+        const int v = c / w.gd;
+        s_v[c] = in[(size_t)w.verts[F.verts + v] * w.gd + (c - v * w.gd)] + from_children(w, F, c);
+    }
+    __syncthreads();
+    // a row per 8 lanes: the fronts of this kernel have few pivots
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
+    for (int r0 = warp * 4; r0 < F.p; r0 += 32) {
+        const int r = r0 + (lane >> 3);
+        double s = 0.0;
+        if (r < F.p) {
+            const double* X = w.factor + F.x11 + (size_t)r * F.ldp;
+#pragma unroll 8
+            for (int c = sub; c <= r; c += 8) s += X[c] * s_v[c];
+        }
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (sub == 0 && r < F.p) s_z[r] = w.z[F.piv + r] = s;
+    }
+    __syncthreads();
+    for (int r0 = warp * 4; r0 < F.b; r0 += 64) {  // two rows per 8 lanes at a time
+        const int r = r0 + (lane >> 3), r2 = r + 32;
+        double s = 0.0, s2 = 0.0, kid = 0.0, kid2 = 0.0;
+        if (sub == 0 && r < F.b) kid = from_children(w, F, F.p + r);
+        if (sub == 0 && r2 < F.b) kid2 = from_children(w, F, F.p + r2);
+        const double* L = w.factor + F.l21 + (size_t)(r < F.b ? r : 0) * F.ldp;
+        const double* L2 = w.factor + F.l21 + (size_t)(r2 < F.b ? r2 : 0) * F.ldp;
+        if (r < F.b)
+#pragma unroll 8
+            for (int c = sub; c < F.p; c += 8) {
+                s += L[c] * s_z[c];
+                s2 += L2[c] * s_z[c];
+            }
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, off);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, off);
+        }
+        if (sub == 0 && r < F.b) w.vec[F.vec + r] = kid - s;
+        if (sub == 0 && r2 < F.b) w.vec[F.vec + r2] = kid2 - s2;
+    }
+}
+
+// Backward: x_P = x11^T (S z - l21^T x_B).
+__global__ void __launch_bounds__(256) k_fc_bwd(FcWork w, double* __restrict__ x, int begin) {
+    extern __shared__ double s_v[];  // x_B, then t (p)
+    __shared__ double s_p[8][64];
+    const FcTask tk = w.tasks[begin + blockIdx.x];
+    const FcFront F = w.fronts[tk.front];
+    if (!w.active[F.tissue]) return;
+    double* s_t = s_v + F.b;
+    for (int r = threadIdx.x; r < F.b; r += 256) {
+        const int idx = F.p + r, v = idx / w.gd;
+        s_v[r] = x[(size_t)w.verts[F.verts + v] * w.gd + (idx - v * w.gd)];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int pass = 0; pass < 2; ++pass) {  // columns of l21, then of x11, 64 at a time
+        for (int c0 = 0; c0 < F.p; c0 += 64) {
+            const int col = c0 + lane, col2 = col + 32;
+            double s = 0.0, s2 = 0.0;
+            if (pass == 0) {
+                const double* L = w.factor + F.l21 + (col < F.p ? col : 0);
+                const double* L2 = w.factor + F.l21 + (col2 < F.p ? col2 : 0);
+#pragma unroll 8
+                for (int r = warp; r < F.b; r += 8) {
+                    s += L[(size_t)r * F.ldp] * s_v[r];
+                    s2 += L2[(size_t)r * F.ldp] * s_v[r];
+                }
+            } else {
+                const double* X = w.factor + F.x11;
+#pragma unroll 8
+                for (int r = c0 + warp; r < F.p; r += 8) {
+                    if (col <= r) s += X[(size_t)r * F.ldp + col] * s_t[r];
+                    if (col2 <= r) s2 += X[(size_t)r * F.ldp + col2] * s_t[r];
+                }
+            }
+            s_p[warp][lane] = s;
+            s_p[warp][lane + 32] = s2;
+            __syncthreads();
+            const int c = c0 + threadIdx.x;
+            if (threadIdx.x < 64 && c < F.p) {
+                double t = 0.0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) t += s_p[k][threadIdx.x];
+                if (pass == 0) {
+                    s_t[c] = w.sign[F.piv + c] * w.z[F.piv + c] - t;
+                } else {
+                    const int v = c / w.gd;
+                    x[(size_t)w.verts[F.verts + v] * w.gd + (c - v * w.gd)] = t;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// The larger fronts, each pass in two launches. z = x11 v_P for 16 pivots, v_P the right-hand side plus
+// the children's vectors.
 __global__ void __launch_bounds__(256) k_fc_fwd1(FcWork w, const double* __restrict__ in, int begin) {
     extern __shared__ double s_v[];
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
     const int r1 = min((tk.i + 1) * kFcRows, F.p);
-    for (int c = threadIdx.x; c < r1; c += blockDim.x) {
+    for (int c = threadIdx.x; c < r1; c += 256) {
         const int v = c / w.gd;
         s_v[c] = in[(size_t)w.verts[F.verts + v] * w.gd + (c - v * w.gd)] + from_children(w, F, c);
     }
@@ -491,13 +885,14 @@ __global__ void __launch_bounds__(256) k_fc_fwd1(FcWork w, const double* __restr
     for (int r = tk.i * kFcRows + (threadIdx.x >> 5); r < r1; r += 8) {
         const double* X = w.factor + F.x11 + (size_t)r * F.ldp;
         double s = 0.0;
+#pragma unroll 8
         for (int c = lane; c <= r; c += 32) s += X[c] * s_v[c];
         s = warp_sum(s);
         if (lane == 0) w.z[F.piv + r] = s;
     }
 }
 
-// v_B = the children's vectors - l21 z for 32 boundary rows.
+// v_B = the children's vectors - l21 z for 16 boundary rows.
 __global__ void __launch_bounds__(256) k_fc_fwd2(FcWork w, int begin) {
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
@@ -507,6 +902,7 @@ __global__ void __launch_bounds__(256) k_fc_fwd2(FcWork w, int begin) {
     for (int r = tk.i * kFcRows + (threadIdx.x >> 5); r < r1; r += 8) {
         const double* L = w.factor + F.l21 + (size_t)r * F.ldp;
         double s = 0.0;
+#pragma unroll 8
         for (int c = lane; c < F.p; c += 32) s += L[c] * z[c];
         s = warp_sum(s);
         if (lane == 0) w.vec[F.vec + r] = from_children(w, F, F.p + r) - s;
@@ -521,7 +917,7 @@ __global__ void __launch_bounds__(256) k_fc_bwd1(FcWork w, const double* __restr
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
     const int r0 = tk.i * kFcBackRows, n = min(kFcBackRows, F.b - r0);
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
+    for (int r = threadIdx.x; r < n; r += 256) {
         const int idx = F.p + r0 + r, v = idx / w.gd;
         s_x[r] = x[(size_t)w.verts[F.verts + v] * w.gd + (idx - v * w.gd)];
     }
@@ -530,7 +926,7 @@ __global__ void __launch_bounds__(256) k_fc_bwd1(FcWork w, const double* __restr
     double s = 0.0;
     if (col < F.p) {
         const double* L = w.factor + F.l21 + (size_t)r0 * F.ldp + col;
-#pragma unroll 4
+#pragma unroll 8
         for (int r = part; r < n; r += 4) s += L[(size_t)r * F.ldp] * s_x[r];
     }
     s_p[part][c] = s;
@@ -539,14 +935,14 @@ __global__ void __launch_bounds__(256) k_fc_bwd1(FcWork w, const double* __restr
 }
 
 // x_P = x11^T (S z - l21^T x_B) for 32 pivots.
-__global__ void __launch_bounds__(256) k_fc_bwd2(FcWork w, double* __restrict__ x, int begin) {
+__global__ void __launch_bounds__(512) k_fc_bwd2(FcWork w, double* __restrict__ x, int begin) {
     extern __shared__ double s_v[];
-    __shared__ double s_p[8][33];
+    __shared__ double s_p[16][33];
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
-    const int c0 = tk.i * kFcRows, chunks = (F.b + kFcBackRows - 1) / kFcBackRows;
-    for (int c = c0 + threadIdx.x; c < F.p; c += blockDim.x) {
+    const int c0 = tk.i * 32, chunks = (F.b + kFcBackRows - 1) / kFcBackRows;
+    for (int c = c0 + threadIdx.x; c < F.p; c += 512) {
         double t = w.sign[F.piv + c] * w.z[F.piv + c];
         for (int k = 0; k < chunks; ++k) t -= w.tp[F.tp + (size_t)k * F.ldp + c];
         s_v[c - c0] = t;
@@ -556,8 +952,8 @@ __global__ void __launch_bounds__(256) k_fc_bwd2(FcWork w, double* __restrict__ 
     double s = 0.0;
     if (col < F.p) {
         const double* X = w.factor + F.x11 + col;
-#pragma unroll 4
-        for (int r = c0 + warp; r < F.p; r += 8)
+#pragma unroll 8
+        for (int r = c0 + warp; r < F.p; r += 16)
             if (r >= col) s += X[(size_t)r * F.ldp] * s_v[r - c0];
     }
     s_p[warp][lane] = s;
@@ -565,7 +961,7 @@ __global__ void __launch_bounds__(256) k_fc_bwd2(FcWork w, double* __restrict__ 
     if (warp == 0 && col < F.p) {
         double t = 0.0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) t += s_p[k][lane];
+        for (int k = 0; k < 16; ++k) t += s_p[k][lane];
         const int v = col / w.gd;
         x[(size_t)w.verts[F.verts + v] * w.gd + (col - v * w.gd)] = t;
     }
@@ -586,33 +982,42 @@ __device__ __forceinline__ double block_total(double v, double* smem) {
 // Sum of a tissue's chunk partials, the same in every thread and every CTA.
 __device__ __forceinline__ double tissue_total(const FcCg& c, const double* part, int t, double* smem) {
     double s = 0.0;
-    for (int k = c.chunk0[t] + threadIdx.x; k < c.chunk0[t + 1]; k += blockDim.x) s += part[k];
+    for (int k = c.chunk0[t] + threadIdx.x; k < c.chunk0[t + 1]; k += blockDim.x) s += __ldcg(part + k);
     return block_total(s, smem);
 }
 
-__global__ void __launch_bounds__(256) k_fc_cg_start(KrylovWork w, FcCg c) {
+// True in every thread of the last CTA of the tissue to arrive, after all partials are visible.
+__device__ __forceinline__ bool last_of_tissue(const FcCg& c, int t) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const uint32_t n = (uint32_t)(c.chunk0[t + 1] - c.chunk0[t]);
+        last = atomicAdd(&c.sc[t].ticket[0], 1u) == n - 1;
+        if (last) c.sc[t].ticket[0] = 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    return last;
+}
+
+__global__ void __launch_bounds__(256) k_fc_cg_start(KrylovWork w, FcCg c, double rtol, int max_iter) {
     __shared__ double smem[8];
     const FcChunk ch = c.chunks[blockIdx.x];
-    if (!c.active[ch.tissue]) return;
+    const int t = ch.tissue;
+    if (!c.active[t]) {
+        if (threadIdx.x == 0 && (int)blockIdx.x == c.chunk0[t]) c.running[t] = 0;
+        return;
+    }
     double s = 0.0;
-    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += blockDim.x) {
+    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) {
         const double b = w.b[i];
         w.x[i] = 0.0;
         w.r[i] = b;
-        w.p[i] = 0.0;
         s += b * b;
     }
     s = block_total(s, smem);
     if (threadIdx.x == 0) c.part[2 * c.n_chunks + blockIdx.x] = s;
-}
-
-__global__ void __launch_bounds__(256) k_fc_cg_begin(FcCg c, double rtol, int max_iter) {
-    __shared__ double smem[8];
-    const int t = blockIdx.x;
-    if (!c.active[t]) {
-        if (threadIdx.x == 0) c.running[t] = 0;
-        return;
-    }
+    if (!last_of_tissue(c, t)) return;
     const double bb = tissue_total(c, c.part + 2 * c.n_chunks, t, smem);
     if (threadIdx.x == 0) {
         KrylovScalars& k = c.sc[t];
@@ -632,7 +1037,7 @@ __global__ void __launch_bounds__(256) k_fc_cg_dot(KrylovWork w, FcCg c, const d
     const FcChunk ch = c.chunks[blockIdx.x];
     if (!c.running[ch.tissue]) return;
     double s = 0.0;
-    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += blockDim.x) s += w.r[i] * z[i];
+    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) s += w.r[i] * z[i];
     s = block_total(s, smem);
     if (threadIdx.x == 0) c.part[blockIdx.x] = s;
 }
@@ -641,25 +1046,27 @@ __global__ void __launch_bounds__(256) k_fc_cg_p(KrylovWork w, FcCg c, const dou
     __shared__ double smem[8];
     const FcChunk ch = c.chunks[blockIdx.x];
     if (!c.running[ch.tissue]) return;
-    const double rho = tissue_total(c, c.part, ch.tissue, smem), old = c.sc[ch.tissue].rho_prev;
-    const double beta = old != 0.0 ? rho / old : 0.0;
-    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += blockDim.x) w.p[i] = z[i] + beta * w.p[i];
+    const double beta = tissue_total(c, c.part, ch.tissue, smem) / c.sc[ch.tissue].rho_prev;
+    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) w.p[i] = z[i] + beta * w.p[i];
 }
 
-// q = J p and the chunk's (p, q); eight lanes a row.
-__global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, double* __restrict__ q) {
+// q = J p and the chunk's (p, q); eight lanes a row. FIRST: the first iteration, p = z, and (r, z) as
+// well, so that it needs no kernel before this one.
+template <bool FIRST>
+__global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const double* __restrict__ z, double* __restrict__ q) {
     __shared__ double smem[8];
     const FcChunk ch = c.chunks[blockIdx.x];
     if (!c.running[ch.tissue]) return;
+    const double* __restrict__ pv = FIRST ? z : w.p;
     const int gl = threadIdx.x & 7;
-    double dot = 0.0;
+    double dot = 0.0, rho = 0.0;
     for (int base = ch.row0; base < ch.row1; base += 32) {
         const int row = base + (threadIdx.x >> 3);
         double y0 = 0.0, y1 = 0.0, y2 = 0.0;
         if (row < ch.row1)
             for (int k = w.rowptr[row] + gl; k < w.rowptr[row + 1]; k += 8) {
                 const double* B = w.vals + (size_t)k * 9;
-                const double* x = w.p + (size_t)w.colidx[k] * 3;
+                const double* x = pv + (size_t)w.colidx[k] * 3;
                 const double x0 = x[0], x1 = x[1], x2 = x[2];
                 y0 += B[0] * x0 + B[1] * x1 + B[2] * x2;
                 y1 += B[3] * x0 + B[4] * x1 + B[5] * x2;
@@ -673,23 +1080,38 @@ __global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, double
         }
         if (row < ch.row1 && gl < 3) {
             const double y = gl == 0 ? y0 : (gl == 1 ? y1 : y2);
-            q[(size_t)row * 3 + gl] = y;
-            dot += y * w.p[(size_t)row * 3 + gl];
+            const size_t i = (size_t)row * 3 + gl;
+            const double p = pv[i];
+            q[i] = y;
+            dot += y * p;
+            if (FIRST) {
+                w.p[i] = p;
+                rho += w.r[i] * p;
+            }
         }
     }
     dot = block_total(dot, smem);
-    if (threadIdx.x == 0) c.part[c.n_chunks + blockIdx.x] = dot;
+    if (FIRST) rho = block_total(rho, smem);
+    if (threadIdx.x == 0) {
+        c.part[c.n_chunks + blockIdx.x] = dot;
+        if (FIRST) c.part[blockIdx.x] = rho;
+    }
 }
 
+// x += alpha p, r -= alpha q, and the tissue's test by the last of its CTAs: converged, out of
+// iterations, or still running. A step that does not look like one of a (nearly) exact preconditioner
+// - (r, z) and (p, J p) of opposite sign, or a residual that grows - ends with KS_INDEFINITE, and
+// the caller takes another path.
 __global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const double* __restrict__ q) {
     __shared__ double smem[8];
     const FcChunk ch = c.chunks[blockIdx.x];
-    if (!c.running[ch.tissue]) return;
-    const double rho = tissue_total(c, c.part, ch.tissue, smem);
-    const double pq = tissue_total(c, c.part + c.n_chunks, ch.tissue, smem);
+    const int t = ch.tissue;
+    if (!c.running[t]) return;
+    const double rho = tissue_total(c, c.part, t, smem);
+    const double pq = tissue_total(c, c.part + c.n_chunks, t, smem);
     const double alpha = rho / pq;
     double s = 0.0;
-    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += blockDim.x) {
+    for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) {
         w.x[i] += alpha * w.p[i];
         const double r = w.r[i] - alpha * q[i];
         w.r[i] = r;
@@ -697,16 +1119,7 @@ __global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const dou
     }
     s = block_total(s, smem);
     if (threadIdx.x == 0) c.part[2 * c.n_chunks + blockIdx.x] = s;
-}
-
-// The tissue's test: converged, out of iterations, or still running. A step that does not look like
-// one of a (nearly) exact preconditioner - (r, z) and (p, J p) of opposite sign, or a residual that
-// grows - ends with KS_INDEFINITE, and the caller takes another path.
-__global__ void __launch_bounds__(256) k_fc_cg_test(FcCg c) {
-    __shared__ double smem[8];
-    const int t = blockIdx.x;
-    if (!c.running[t]) return;
-    const double rho = tissue_total(c, c.part, t, smem), pq = tissue_total(c, c.part + c.n_chunks, t, smem);
+    if (!last_of_tissue(c, t)) return;
     const double rr = tissue_total(c, c.part + 2 * c.n_chunks, t, smem);
     if (threadIdx.x) return;
     KrylovScalars& k = c.sc[t];
@@ -737,6 +1150,7 @@ cudaError_t opt_in(const void* f, int bytes) { return cudaFuncSetAttribute(f, cu
 
 cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, cudaStream_t s) {
     // per-device attributes of the kernels; cheap next to a factorisation
+    FC_CK(opt_in((const void*)k_fc_small, small_smem(kT, kFcSmallB)));
     FC_CK(opt_in((const void*)k_fc_col, kPanelSmem));
     FC_CK(opt_in((const void*)k_fc_upd, kPanelSmem));
     FC_CK(opt_in((const void*)k_fc_l21, kGemmSmem));
@@ -744,6 +1158,16 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
     int64_t n = 0;
     for (int d = (int)plan.depths.size() - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
+        for (const FcRange& r : L.small)
+            if (r.count) {
+                int smem = 0;
+                for (int k = 0; k < r.count; ++k) {
+                    const FcFront& F = plan.fronts[plan.tasks[r.begin + k].front];
+                    smem = smem < small_smem(F.p, F.b) ? small_smem(F.p, F.b) : smem;
+                }
+                k_fc_small<<<r.count, 256, smem, s>>>(w, vals, r.begin, d & 1);
+                ++n;
+            }
         if (L.gather.count) {
             const int pmax = plan.fronts[plan.tasks[L.gather.begin].front].p;  // the list starts with the largest
             k_fc_gather<<<L.gather.count, 256, pmax * sizeof(int2), s>>>(w, L.gather.begin, d & 1);
@@ -760,7 +1184,7 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
         for (int k = 0; k < L.n_panel; ++k) {
             const FcPanel& P = plan.panels[L.panel0 + k];
             if (P.col.count) {
-                k_fc_col<<<P.col.count, 256, kPanelSmem, s>>>(w, P.col.begin, k);
+                k_fc_col<<<4 * P.col.count, 256, kPanelSmem, s>>>(w, P.col.begin, k);
                 ++n;
             }
             if (P.upd.count) {
@@ -781,12 +1205,27 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
     return cudaGetLastError();
 }
 
+// Shared memory of the one-CTA passes: two vectors of the pivots (forward), boundary and pivots (back).
+static size_t solve_smem(const FcPlan& plan, const FcRange& r, bool forward) {
+    int n = 0;
+    for (int k = 0; k < r.count; ++k) {
+        const FcFront& F = plan.fronts[plan.tasks[r.begin + k].front];
+        const int m = forward ? 2 * F.p : F.p + F.b;
+        n = n < m ? m : n;
+    }
+    return sizeof(double) * (size_t)n;
+}
+
 cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
                                 cudaStream_t s) {
     int64_t n = 0;
     const int depths = (int)plan.depths.size();
     for (int d = depths - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
+        if (L.solve.count) {
+            k_fc_fwd<<<L.solve.count, 256, solve_smem(plan, L.solve, true), s>>>(w, in, L.solve.begin);
+            ++n;
+        }
         if (L.fwd1.count) {
             const int pmax = plan.fronts[plan.tasks[L.fwd1.begin].front].p;
             k_fc_fwd1<<<L.fwd1.count, 256, pmax * sizeof(double), s>>>(w, in, L.fwd1.begin);
@@ -799,13 +1238,17 @@ cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const doubl
     }
     for (int d = 0; d < depths; ++d) {
         const FcDepth& L = plan.depths[d];
+        if (L.solve.count) {
+            k_fc_bwd<<<L.solve.count, 256, solve_smem(plan, L.solve, false), s>>>(w, x, L.solve.begin);
+            ++n;
+        }
         if (L.bwd1.count) {
             k_fc_bwd1<<<L.bwd1.count, 256, 0, s>>>(w, x, L.bwd1.begin);
             ++n;
         }
         if (L.bwd2.count) {
             const int pmax = plan.fronts[plan.tasks[L.bwd2.begin].front].p;
-            k_fc_bwd2<<<L.bwd2.count, 256, pmax * sizeof(double), s>>>(w, x, L.bwd2.begin);
+            k_fc_bwd2<<<L.bwd2.count, 512, pmax * sizeof(double), s>>>(w, x, L.bwd2.begin);
             ++n;
         }
     }
@@ -814,18 +1257,20 @@ cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const doubl
 }
 
 cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int max_iter, cudaStream_t s) {
-    k_fc_cg_start<<<c.n_chunks, 256, 0, s>>>(w, c);
-    k_fc_cg_begin<<<c.T, 256, 0, s>>>(c, rtol, max_iter);
+    k_fc_cg_start<<<c.n_chunks, 256, 0, s>>>(w, c, rtol, max_iter);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fc_iteration(const KrylovWork& w, const FcCg& c, const double* z, double* q, cudaStream_t s) {
-    k_fc_cg_dot<<<c.n_chunks, 256, 0, s>>>(w, c, z);
-    k_fc_cg_p<<<c.n_chunks, 256, 0, s>>>(w, c, z);
-    k_fc_cg_spmv<<<c.n_chunks, 256, 0, s>>>(w, c, q);
+int launch_fc_iteration(const KrylovWork& w, const FcCg& c, bool first, const double* z, double* q, cudaStream_t s) {
+    if (first) {
+        k_fc_cg_spmv<true><<<c.n_chunks, 256, 0, s>>>(w, c, z, q);
+    } else {
+        k_fc_cg_dot<<<c.n_chunks, 256, 0, s>>>(w, c, z);
+        k_fc_cg_p<<<c.n_chunks, 256, 0, s>>>(w, c, z);
+        k_fc_cg_spmv<false><<<c.n_chunks, 256, 0, s>>>(w, c, z, q);
+    }
     k_fc_cg_x<<<c.n_chunks, 256, 0, s>>>(w, c, q);
-    k_fc_cg_test<<<c.T, 256, 0, s>>>(c);
-    return cudaGetLastError();
+    return first ? 2 : 4;
 }
 
 }  // namespace tfb

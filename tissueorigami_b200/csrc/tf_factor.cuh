@@ -23,7 +23,9 @@ namespace tfb {
 constexpr int kFcTile = 64;        // pivot panel width and GEMM tile
 constexpr int kFcGatherRows = 32;  // rows of a front per assembly task
 constexpr int kFcScatter = 256;    // Jacobian blocks per assembly task
-constexpr int kFcRows = 32;        // front rows per solve task
+constexpr int kFcSmallB = 288;     // boundary unknowns up to which a one-panel front is one CTA's
+constexpr int kFcSmallSolve = 49152; // entries of x11 and l21 up to which a front's solve is one CTA's
+constexpr int kFcRows = 16;        // front rows per solve task
 constexpr int kFcBackRows = 128;   // boundary rows per backward task
 constexpr int kFcMaxPivots = 5000; // pivots of one front (the solve stages them in shared memory)
 
@@ -32,6 +34,7 @@ struct FcFront {
     int32_t ldp, ldb;      // leading dimensions (even): rows of x11 / l21 / a21, rows of c
     int32_t tissue;
     int32_t child[2];      // fronts one depth below, or -1
+    int32_t child_ldb[2], child_vec[2];  // the children's ldb and vec, and below their c: one load away
     int32_t map[2];        // offsets into maps: per column of this front, its index on the child's boundary
     int32_t verts;         // offset into verts: the pivots' columns, then the boundary's
     int32_t j0, j1;        // its Jacobian blocks in jblk
@@ -39,6 +42,7 @@ struct FcFront {
     int64_t x11, l21;      // kept factors
     int64_t a21, lp;       // scratch of the front's depth: A21, and the current panel of L11 (p x 64)
     int64_t c;             // contribution (b x b, lower), in the scratch of the depth's parity
+    int64_t child_c[2];
     int64_t tp;            // scratch of the backward pass: partial sums per boundary chunk (chunks x p)
 };
 
@@ -56,7 +60,8 @@ struct FcPanel {
 };
 
 struct FcDepth {
-    FcRange gather, scatter, diag, l21, schur, fwd1, fwd2, bwd1, bwd2;
+    FcRange small[3], gather, scatter, diag, l21, schur;  // small: fronts factorised by one CTA each, by size
+    FcRange solve, fwd1, fwd2, bwd1, bwd2;             // solve: fronts whose passes are one CTA's each
     int32_t panel0 = 0, n_panel = 0;
 };
 
@@ -100,6 +105,7 @@ struct FcWork {
     double* z;
     double* sign;    // [n_piv] +1 / -1
     int32_t* flags;  // [T] 1: a zero or non-finite pivot
+    int32_t* neg;    // [fronts] 1: the front has negative pivots
 };
 
 // Numeric factorisation of J (vals: the full BSR3 values; block (row, column) is read from the row of
@@ -125,9 +131,10 @@ struct FcCg {
     int32_t* running;       // [T] still iterating (the preconditioner's active flags)
     double* part;           // [3][n_chunks]: (r, z), (p, J p), (r, r) / (b, b)
 };
-// x = 0, r = b, p = 0; every active tissue running (unless b = 0)
+// x = 0, r = b; every active tissue running (unless b = 0)
 cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int max_iter, cudaStream_t s);
-// one iteration after z = M^-1 r: p = z + beta p, q = J p, x += alpha p, r -= alpha q, and the test
-cudaError_t launch_fc_iteration(const KrylovWork& w, const FcCg& c, const double* z, double* q, cudaStream_t s);
+// one iteration after z = M^-1 r: p = z + beta p (p = z in the first), q = J p, x += alpha p,
+// r -= alpha q, and the test. Returns the kernels launched.
+int launch_fc_iteration(const KrylovWork& w, const FcCg& c, bool first, const double* z, double* q, cudaStream_t s);
 
 }  // namespace tfb

@@ -298,7 +298,7 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             F.l21 = F.x11 + (int64_t)F.p * F.ldp;
             plan.n_factor = F.l21 + (int64_t)F.b * F.ldp;
             F.a21 = scratch;
-            F.lp = F.a21 + (int64_t)F.b * F.ldp;
+            F.lp = F.a21 + (int64_t)F.b * F.ldp;  // a21, lp: not used by the fronts of one CTA
             scratch = F.lp + (F.p > kFcTile ? (int64_t)F.p * kFcTile : 0);
             F.c = contrib;
             contrib += (int64_t)F.b * F.ldb;
@@ -310,6 +310,13 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
         plan.n_contrib[d & 1] = std::max(plan.n_contrib[d & 1], contrib);
         plan.n_tp = std::max(plan.n_tp, tp);
     }
+    for (FcFront& F : plan.fronts)
+        for (int k = 0; k < 2; ++k) {
+            const FcFront* c = F.child[k] >= 0 ? &plan.fronts[F.child[k]] : nullptr;
+            F.child_ldb[k] = c ? c->ldb : 0;
+            F.child_vec[k] = c ? c->vec : 0;
+            F.child_c[k] = c ? c->c : 0;
+        }
     if (n_map > INT32_MAX || n_vert > INT32_MAX || plan.n_vec > INT32_MAX || plan.n_piv > INT32_MAX) return;
     plan.maps.resize(n_map);
     plan.verts.resize(n_vert);
@@ -376,6 +383,21 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             r.count = (int32_t)plan.tasks.size() - r.begin;
         };
         auto push = [&](int32_t f, int i, int j) { plan.tasks.push_back(FcTask{f, (int16_t)i, (int16_t)j}); };
+        auto is_small = [](const FcFront& F) { return F.p > 0 && F.p <= kFcTile && F.b <= kFcSmallB; };
+        auto one_cta = [](const FcFront& F) { return (int64_t)F.p * (F.p + F.b) <= kFcSmallSolve; };
+        std::vector<int32_t> all = fs, rest;
+        for (int32_t fi : fs)
+            if (!is_small(plan.fronts[fi])) rest.push_back(fi);
+        std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) { return plan.fronts[a].b > plan.fronts[b].b; });
+        // in three launches by the shared memory they need, so that small fronts share an SM (the
+        // bounds leave room for two and three of them)
+        auto entries = [](const FcFront& F) { return (int64_t)(F.p + F.b + 39) * (((F.p + 15) & ~15) + 4); };
+        const int64_t bound[4] = {INT64_MAX, 12800, 8200, 0};
+        for (int c = 0; c < 3; ++c)
+            list(L.small[c], [&](int32_t fi, const FcFront& F) {
+                if (is_small(F) && entries(F) <= bound[c] && entries(F) > bound[c + 1]) push(fi, 0, 0);
+            });
+        fs = rest;
         list(L.gather, [&](int32_t fi, const FcFront& F) {
             if (F.p > 0)
                 for (int i = 0; i < cdiv(F.p + F.b, kFcGatherRows); ++i) push(fi, i, 0);
@@ -419,6 +441,16 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             for (int i = 0; i < cdiv(F.b, kFcTile); ++i)
                 for (int j = 0; j <= i; ++j) push(fi, i, j);
         });
+        fs.clear();
+        for (int32_t fi : all)
+            if (one_cta(plan.fronts[fi])) fs.push_back(fi);
+        std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) {
+            return (int64_t)plan.fronts[a].p * plan.fronts[a].b > (int64_t)plan.fronts[b].p * plan.fronts[b].b;
+        });
+        list(L.solve, [&](int32_t fi, const FcFront&) { push(fi, 0, 0); });
+        fs.clear();
+        for (int32_t fi : all)
+            if (!one_cta(plan.fronts[fi])) fs.push_back(fi);
         list(L.fwd1, [&](int32_t fi, const FcFront& F) {
             for (int i = cdiv(F.p, kFcRows) - 1; i >= 0; --i) push(fi, i, 0);
         });
@@ -430,7 +462,7 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
                 for (int j = 0; j < cdiv(F.p, kFcTile); ++j) push(fi, i, j);
         });
         list(L.bwd2, [&](int32_t fi, const FcFront& F) {
-            for (int i = 0; i < cdiv(F.p, kFcRows); ++i) push(fi, i, 0);
+            for (int i = 0; i < cdiv(F.p, 32); ++i) push(fi, i, 0);
         });
     }
     if (plan.tasks.size() > (size_t)INT32_MAX) return;
