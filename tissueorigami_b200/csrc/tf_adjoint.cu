@@ -257,6 +257,27 @@ __global__ void k_set_inv_fg(ElemRecord* elems, int32_t n_elems, const double* f
         for (int j = 0; j < 3; ++j) elems[e].inv_fg[i * 3 + j] = o[i][j];
 }
 
+// *flag = 1 when some Fg is singular or not finite.
+__global__ void k_check_fg(int32_t n_elems, const double* fg, int32_t* flag) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_elems) return;
+    double m[3][3];
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j) m[i][j] = fg[(size_t)e * 9 + i * 3 + j];
+    const double det = det3(m);
+    if (det == 0.0 || !isfinite(det)) *flag = 1;
+}
+
+// field (a double offset in the records) of every record = src [E][ncomp]; one double per thread, so the
+// reads are contiguous and a record's field is written by consecutive threads. Bound by the records' sectors
+// (416 bytes apart): 3 M prisms in 0.1 ms, where taking the records to the host and back took 830.
+__global__ void k_set_field(ElemRecord* elems, int64_t n, int field, int ncomp, const double* __restrict__ src) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int64_t e = k / ncomp;
+    reinterpret_cast<double*>(elems + e)[field + (int)(k - e * ncomp)] = src[k];
+}
+
 __global__ void k_mask_fixed(int32_t n_nodes, const uint8_t* fixmask, double* v) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_nodes) return;
@@ -285,6 +306,19 @@ cudaError_t launch_position_vjp(const ElemRecord* elems, int32_t n_elems, int32_
 
 cudaError_t launch_set_inv_fg(ElemRecord* elems, int32_t n_elems, const double* fg, cudaStream_t s) {
     k_set_inv_fg<<<(n_elems + 255) / 256, 256, 0, s>>>(elems, n_elems, fg);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_check_fg(int32_t n_elems, const double* fg, int32_t* flag, cudaStream_t s) {
+    cudaError_t err = cudaMemsetAsync(flag, 0, sizeof(int32_t), s);
+    if (err != cudaSuccess) return err;
+    k_check_fg<<<(n_elems + 255) / 256, 256, 0, s>>>(n_elems, fg, flag);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_set_field(ElemRecord* elems, int32_t n_elems, int field, int ncomp, const double* src, cudaStream_t s) {
+    const int64_t n = (int64_t)n_elems * ncomp;
+    k_set_field<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(elems, n, field, ncomp, src);
     return cudaGetLastError();
 }
 

@@ -2378,13 +2378,19 @@ int check_ctx(tf_ctx* ctx) {
     return TF_OK;
 }
 
-// Per-element field setter: writes `ncomp` doubles at byte offset `off` of every record.
+// Per-element field setter: writes `ncomp` doubles at byte offset `off` of every record. The values go
+// through the Jacobian's buffer (every call that reads J assembles or copies it first).
 int set_record_field(tf_ctx* ctx, size_t off, int ncomp, const double* src) {
-    std::vector<ElemRecord> rec(ctx->E);
-    TF_CK(cudaMemcpy(rec.data(), ctx->elems.p, sizeof(ElemRecord) * (size_t)ctx->E, cudaMemcpyDeviceToHost));
-    for (int e = 0; e < ctx->E; ++e)
-        std::memcpy(reinterpret_cast<char*>(&rec[e]) + off, src + (size_t)e * ncomp, sizeof(double) * ncomp);
-    TF_CK(cudaMemcpy(ctx->elems.p, rec.data(), sizeof(ElemRecord) * (size_t)ctx->E, cudaMemcpyHostToDevice));
+    const size_t bytes = sizeof(double) * (size_t)ncomp * ctx->E;
+    DevBuf own;  // for a mesh with fewer blocks than prisms
+    if (ctx->vals.bytes < bytes) TF_CK(dalloc(own, bytes));
+    double* stage = dptr<double>(own.p ? own : ctx->vals);
+    cudaError_t e = cudaMemcpyAsync(stage, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess)
+        e = launch_set_field(dptr<ElemRecord>(ctx->elems), ctx->E, (int)(off / sizeof(double)), ncomp, stage, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    dfree(own);
+    TF_CK(e);
     return TF_OK;
 }
 
@@ -3139,28 +3145,14 @@ int tf_set_growth(tf_ctx* ctx, const double* fg, const double* rates, const doub
     if (rc != TF_OK) return rc;
     const size_t E = ctx->E;
     if (fg) {
-        TF_CK(cudaMemcpy(ctx->fg.p, fg, sizeof(double) * 9 * E, cudaMemcpyHostToDevice));
+        TF_CK(cudaMemcpyAsync(ctx->fg.p, fg, sizeof(double) * 9 * E, cudaMemcpyHostToDevice, ctx->stream));
         // keep InvFg consistent with Fg (growShapeByFg leaves both in step)
-        std::vector<double> inv(9 * E);
-        for (size_t e = 0; e < E; ++e) {
-            const double* m = fg + e * 9;
-            const double det = m[0] * (m[4] * m[8] - m[5] * m[7]) - m[1] * (m[3] * m[8] - m[5] * m[6]) +
-                               m[2] * (m[3] * m[7] - m[4] * m[6]);
-            if (det == 0.0 || !std::isfinite(det)) return TF_ERR_ARGUMENT;
-            const double id = 1.0 / det;
-            double* o = &inv[e * 9];
-            o[0] = (m[4] * m[8] - m[5] * m[7]) * id;
-            o[1] = (m[2] * m[7] - m[1] * m[8]) * id;
-            o[2] = (m[1] * m[5] - m[2] * m[4]) * id;
-            o[3] = (m[5] * m[6] - m[3] * m[8]) * id;
-            o[4] = (m[0] * m[8] - m[2] * m[6]) * id;
-            o[5] = (m[2] * m[3] - m[0] * m[5]) * id;
-            o[6] = (m[3] * m[7] - m[4] * m[6]) * id;
-            o[7] = (m[1] * m[6] - m[0] * m[7]) * id;
-            o[8] = (m[0] * m[4] - m[1] * m[3]) * id;
-        }
-        rc = set_record_field(ctx, offsetof(ElemRecord, inv_fg), 9, inv.data());
+        TF_CK(launch_check_fg(ctx->E, dptr<double>(ctx->fg), dptr<int32_t>(ctx->dflags), ctx->stream));
+        rc = read_flags(ctx);
         if (rc != TF_OK) return rc;
+        if (*ctx->h_flags) return TF_ERR_ARGUMENT;
+        TF_CK(launch_set_inv_fg(dptr<ElemRecord>(ctx->elems), ctx->E, dptr<double>(ctx->fg), ctx->stream));
+        TF_CK(cudaStreamSynchronize(ctx->stream));
     }
     if (rates) TF_CK(cudaMemcpy(ctx->rates.p, rates, sizeof(double) * 3 * E, cudaMemcpyHostToDevice));
     if (angles) TF_CK(cudaMemcpy(ctx->angles.p, angles, sizeof(double) * E, cudaMemcpyHostToDevice));

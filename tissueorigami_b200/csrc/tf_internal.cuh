@@ -268,6 +268,10 @@ cudaError_t launch_position_vjp(const ElemRecord* elems, int32_t n_elems, int32_
                                 const double* ext_visc, const uint8_t* exposed, const uint8_t* peripodial, double dt,
                                 double* q, double* abar, cudaStream_t s);
 cudaError_t launch_set_inv_fg(ElemRecord* elems, int32_t n_elems, const double* fg, cudaStream_t s);
+// *flag = 1 when the growth tensor of some element is singular or not finite, else 0
+cudaError_t launch_check_fg(int32_t n_elems, const double* fg, int32_t* flag, cudaStream_t s);
+// ncomp doubles from double `field` on of every record = src [n_elems][ncomp] (device)
+cudaError_t launch_set_field(ElemRecord* elems, int32_t n_elems, int field, int ncomp, const double* src, cudaStream_t s);
 cudaError_t launch_mask_fixed(int32_t n_nodes, const uint8_t* fixmask, double* v, cudaStream_t s);
 
 // --- direct solve (tf_direct.cu) -----------------------------------------------------------
