@@ -130,3 +130,47 @@ def test_batch_matches_single_runs(count):
                 y, rc, st = s.runOneStep(y, t.dt)
                 assert rc == capi.TF_OK and st["newton_iters"] == its[k][i]
         assert np.abs(xs[i] - y).max() <= 1e-9 * t.size
+
+
+@pytest.mark.parametrize("eta", [4.0, 1e5])
+def test_viscous_steps_match_bicgstab(eta):
+    """Internal viscosity makes J unsymmetric: the factor of its symmetric part in a minimal residual
+    iteration against BiCGStab, two steps, 1e-9 of the size and equal Newton counts; and back to a
+    symmetric J on the same solver."""
+    t = mesh.wing_disc(n_surface_points=700)
+    t.eta[:] = eta
+    out = {}
+    for method in (capi.TF_KRYLOV_AUTO, capi.TF_KRYLOV_BICGSTAB):
+        with NewtonRaphsonSolver.from_tissue(t, krylov_rtol=1e-13, krylov_method=method) as s:
+            x, its = t.x, []
+            for _ in range(2):
+                x, rc, st = s.runOneStep(x, t.dt)
+                assert rc == capi.TF_OK
+                assert st["krylov_method"] == (5 if method == capi.TF_KRYLOV_AUTO else 1)
+                its.append(st["newton_iters"])
+            s.set_material(t.lam, t.mu, None)
+            s.set_growth(fg=t.fg)
+            y, rc, st = s.runOneStep(t.x, t.dt)
+            assert rc == capi.TF_OK
+        out[method] = (x, its, y)
+    a, b = out.values()
+    assert a[1] == b[1]
+    assert np.abs(a[0] - b[0]).max() <= 1e-9 * t.size
+    assert np.abs(a[2] - b[2]).max() <= 1e-9 * t.size
+
+
+@pytest.mark.parametrize("bad", [0.0, np.nan])
+def test_set_growth_rejects_singular_tensors_and_keeps_the_inverse(bad):
+    """A singular or non-finite Fg is refused and leaves InvFg as it was; a valid one sets it."""
+    t = mesh.small_disc(5, 301, 1000.0)
+    rng = np.random.default_rng(3)
+    fg = np.tile(np.eye(3), (t.n_elems, 1, 1)) + rng.uniform(-0.1, 0.1, (t.n_elems, 3, 3))
+    with NewtonRaphsonSolver.from_tissue(t) as s:
+        s.set_growth(fg=fg)
+        inv = s.get_growth()[1].reshape(-1, 3, 3)
+        assert np.abs(inv - np.linalg.inv(fg)).max() <= 1e-13
+        wrong = fg.copy()
+        wrong[-1] = bad
+        with pytest.raises(capi.TFError):
+            s.set_growth(fg=wrong)
+        assert np.array_equal(s.get_growth()[1].reshape(-1, 3, 3), inv)

@@ -183,7 +183,7 @@ struct tf_ctx {
     // whose launch alone, 3.4 us each, took longer than many of them): replayed as graphs (0.75 us each)
     cudaGraphExec_t fc_graph[2] = {nullptr, nullptr};
     int64_t fc_graph_launches[2] = {0, 0};
-    DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_tp, fc_vec, fc_z,
+    DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_jblk_t, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_tp, fc_vec, fc_z,
         fc_sign, fc_flags, fc_neg, fc_chunks, fc_chunk0_d, fc_running, fc_part;
 
     // adjoint: forward checkpoints every adj_k steps, segment recompute buffers, adjoint state
@@ -1687,10 +1687,12 @@ bool use_persistent(tf_ctx* ctx) {
 // sparse factorisation of J where the tissue is small enough for one: the separators' Schur
 // complement is the coarse operator then, eliminated exactly.
 
+// An unsymmetric J (internal viscosity) takes the factor of its symmetric part: the asymmetry comes from the
+// velocity gradient times the time step, a few per cent of the viscous blocks.
 // Whether this solve may take the factorisation. Packing pairs add blocks outside the pattern and make
 // J indefinite (MINRES); krylov_warm_start = 0 asks for solves that keep nothing from earlier ones.
 bool factor_wanted(const tf_ctx* c) {
-    return c->params.precond == TF_PRECOND_TWO_LEVEL && c->params.krylov_method == TF_KRYLOV_AUTO && !c->has_visc &&
+    return c->params.precond == TF_PRECOND_TWO_LEVEL && c->params.krylov_method == TF_KRYLOV_AUTO &&
            c->params.krylov_warm_start && !(c->pk_on && c->pk_pairs_n > 0);
 }
 
@@ -1741,7 +1743,8 @@ int build_factor(tf_ctx* ctx) {
                 for (int d = 0; d < 3; ++d) X[(size_t)(n / G) * 3 + d] = ctx->xref[(size_t)e * 18 + a * 3 + d];
         }
     FcPlan& P = ctx->fc;
-    build_factor_plan(N, G, ctx->rowptr.data(), ctx->colidx.data(), X.data(), T, ctx->tissue_node0.data(), kFcMaxFlops * T, P);
+    build_factor_plan(N, G, ctx->rowptr.data(), ctx->colidx.data(), X.data(), T, ctx->tissue_node0.data(), kFcMaxFlops * T,
+                      ctx->has_visc, P);
     if (!P.ok) return TF_OK;
     std::vector<FcChunk> chunks;
     ctx->fc_chunk0.assign(1, 0);
@@ -1778,6 +1781,7 @@ int build_factor(tf_ctx* ctx) {
     TF_CK(up(ctx->fc_maps, P.maps.data(), sizeof(int32_t) * P.maps.size()));
     TF_CK(up(ctx->fc_verts, P.verts.data(), sizeof(int32_t) * P.verts.size()));
     TF_CK(up(ctx->fc_jblk, P.jblk.data(), sizeof(int2) * P.jblk.size()));
+    TF_CK(up(ctx->fc_jblk_t, P.jblk_t.data(), sizeof(int32_t) * P.jblk_t.size()));
     TF_CK(up(ctx->fc_tasks, P.tasks.data(), sizeof(FcTask) * P.tasks.size()));
     TF_CK(up(ctx->fc_chunks, chunks.data(), sizeof(FcChunk) * chunks.size()));
     TF_CK(up(ctx->fc_chunk0_d, ctx->fc_chunk0.data(), sizeof(int32_t) * ctx->fc_chunk0.size()));
@@ -1786,6 +1790,7 @@ int build_factor(tf_ctx* ctx) {
     P.maps = {};
     P.verts = {};
     P.jblk = {};
+    P.jblk_t = {};
     ctx->fc_ready = true;
     return TF_OK;
 }
@@ -1797,6 +1802,7 @@ FcWork make_factor(tf_ctx* c) {
     f.maps = dptr<int32_t>(c->fc_maps);
     f.verts = dptr<int32_t>(c->fc_verts);
     f.jblk = dptr<int2>(c->fc_jblk);
+    f.jblk_t = c->has_visc ? dptr<int32_t>(c->fc_jblk_t) : nullptr;
     f.tasks = dptr<FcTask>(c->fc_tasks);
     f.active = dptr<int32_t>(c->active_d);
     f.factor = dptr<double>(c->fc_factor);
@@ -1829,6 +1835,7 @@ int factor_solve(tf_ctx* ctx, bool* done) {
     c.active = dptr<int32_t>(ctx->active_d);
     c.running = dptr<int32_t>(ctx->fc_running);
     c.part = dptr<double>(ctx->fc_part);
+    c.minres = ctx->has_visc;
     const bool kept = ctx->fc_same || ctx->fc_near;
     if (!kept) {
         TF_CK(cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream));
@@ -1867,11 +1874,11 @@ int factor_solve(tf_ctx* ctx, bool* done) {
     ctx->last_solve_iters = 0;
     for (int t = 0; t < ctx->T; ++t)
         if (ctx->T == 1 || ctx->h_active[t]) {
-            ctx->last_method = std::max<int32_t>(ctx->last_method, KM_CG);
-            ctx->cg_iters += ctx->h_tsc[t].iter;
+            ctx->last_method = std::max<int32_t>(ctx->last_method, ctx->h_tsc[t].method);
+            if (!c.minres) ctx->cg_iters += ctx->h_tsc[t].iter;
             ctx->last_solve_iters = std::max(ctx->last_solve_iters, ctx->h_tsc[t].iter);
         }
-    ctx->last_solve_method = KM_CG;
+    ctx->last_solve_method = c.minres ? KM_MINIMAL_RESIDUAL : KM_CG;
     *done = true;
     return TF_OK;
 }
@@ -2697,7 +2704,7 @@ void tf_destroy(tf_ctx* ctx) {
                      &ctx->ml_first_cta_d, &ctx->ml_slot_a_d, &ctx->ml_out_ptr_d, &ctx->ml_out_slots_d,
                      &ctx->ml_out_set_d, &ctx->ml_out_col_d, &ctx->ml_out_dst_d, &ctx->ml_pairs_d, &ctx->ml_pos_leaf_d};
     for (DevBuf* b : mlb) dfree(*b);
-    DevBuf* fcb[] = {&ctx->fc_fronts, &ctx->fc_maps, &ctx->fc_verts, &ctx->fc_jblk, &ctx->fc_tasks, &ctx->fc_factor,
+    DevBuf* fcb[] = {&ctx->fc_fronts, &ctx->fc_maps, &ctx->fc_verts, &ctx->fc_jblk, &ctx->fc_jblk_t, &ctx->fc_tasks, &ctx->fc_factor,
                      &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1], &ctx->fc_tp, &ctx->fc_vec, &ctx->fc_z,
                      &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_neg, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
     for (DevBuf* b : fcb) dfree(*b);
@@ -2730,6 +2737,7 @@ int tf_set_material(tf_ctx* ctx, const double* lambda, const double* mu, const d
         lme[(size_t)e * 3 + 2] = eta ? eta[e] : 0.0;
         visc |= eta && eta[e] != 0.0;
     }
+    if (visc != ctx->has_visc) ctx->fc_dirty = true;  // another plan: with the transposed blocks, or without
     ctx->has_visc = visc;
     return set_record_field(ctx, offsetof(ElemRecord, lam), 3, lme.data());
 }

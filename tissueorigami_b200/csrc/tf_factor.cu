@@ -90,6 +90,13 @@ __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int pari
     }
 }
 
+// Entry (rr, cc) that Jacobian block k (of jblk) adds to a front: the block is read from the earlier pivot's row
+// of J, transposed; of an unsymmetric J the mean with its mirror image.
+__device__ __forceinline__ double j_entry(const FcWork& w, const double* __restrict__ vals, int k, int block, int cc, int rr) {
+    const double v = vals[(size_t)block * 9 + cc * 3 + rr];
+    return w.jblk_t ? 0.5 * (v + vals[(size_t)w.jblk_t[k] * 9 + rr * 3 + cc]) : v;
+}
+
 // += the front's Jacobian blocks. Block (column k, row i) of the lower triangle is read from row k of
 // J, transposed; each lands on entries of its own.
 __global__ void __launch_bounds__(256) k_fc_scatter(FcWork w, const double* __restrict__ vals, int begin) {
@@ -103,7 +110,7 @@ __global__ void __launch_bounds__(256) k_fc_scatter(FcWork w, const double* __re
         const int row = (int)((uint32_t)jb.y >> 16) + rr, col = (jb.y & 0xffff) + cc;
         double* out = row < F.p ? w.factor + F.x11 + (size_t)row * F.ldp + col
                                 : w.scratch + F.a21 + (size_t)(row - F.p) * F.ldp + col;
-        *out += vals[(size_t)jb.x * 9 + en];
+        *out += j_entry(w, vals, b0 + k, jb.x, cc, rr);
     }
 }
 
@@ -478,7 +485,7 @@ __global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __rest
             const int k = e / 9, en = e - k * 9, cc = en / 3, rr = en - cc * 3;
             const int2 jb = w.jblk[F.j0 + k];
             const int row = (int)((uint32_t)jb.y >> 16) + rr, col = (jb.y & 0xffff) + cc;
-            (row < p ? sX + row * ld : sL + (row - p) * ld)[col] = vals[(size_t)jb.x * 9 + en];
+            (row < p ? sX + row * ld : sL + (row - p) * ld)[col] = j_entry(w, vals, F.j0 + k, jb.x, cc, rr);
         }
     }
     __syncthreads();
@@ -1026,7 +1033,7 @@ __global__ void __launch_bounds__(256) k_fc_cg_start(KrylovWork w, FcCg c, doubl
         k.rho = k.rho_prev = 0.0;
         k.iter = 0;
         k.max_iter = max_iter;
-        k.method = KM_CG;
+        k.method = c.minres ? KM_MINIMAL_RESIDUAL : KM_CG;
         k.status = !isfinite(bb) ? KS_NONFINITE : (bb > 0.0 ? KS_RUNNING : KS_CONVERGED);
         c.running[t] = k.status == KS_RUNNING;
     }
@@ -1051,7 +1058,8 @@ __global__ void __launch_bounds__(256) k_fc_cg_p(KrylovWork w, FcCg c, const dou
 }
 
 // q = J p and the chunk's (p, q); eight lanes a row. FIRST: the first iteration, p = z, and (r, z) as
-// well, so that it needs no kernel before this one.
+// well, so that it needs no kernel before this one. The minimal residual iteration is all first ones, with
+// (r, q) and (q, q).
 template <bool FIRST>
 __global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const double* __restrict__ z, double* __restrict__ q) {
     __shared__ double smem[8];
@@ -1083,10 +1091,13 @@ __global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const 
             const size_t i = (size_t)row * 3 + gl;
             const double p = pv[i];
             q[i] = y;
-            dot += y * p;
             if (FIRST) {
+                const double m = c.minres ? y : p;
                 w.p[i] = p;
-                rho += w.r[i] * p;
+                dot += y * m;
+                rho += w.r[i] * m;
+            } else {
+                dot += y * p;
             }
         }
     }
@@ -1100,8 +1111,8 @@ __global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const 
 
 // x += alpha p, r -= alpha q, and the tissue's test by the last of its CTAs: converged, out of
 // iterations, or still running. A step that does not look like one of a (nearly) exact preconditioner
-// - (r, z) and (p, J p) of opposite sign, or a residual that grows - ends with KS_INDEFINITE, and
-// the caller takes another path.
+// - (r, z) and (p, J p) of opposite sign, or a residual that does not fall - ends with KS_INDEFINITE,
+// and the caller takes another path.
 __global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const double* __restrict__ q) {
     __shared__ double smem[8];
     const FcChunk ch = c.chunks[blockIdx.x];
@@ -1131,7 +1142,7 @@ __global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const dou
         k.status = KS_NONFINITE;
     else if (rr <= k.tol2)
         k.status = KS_CONVERGED;
-    else if (!(rho * pq > 0.0) || rr > before)
+    else if (!(rho * pq > 0.0) || rr > (c.minres ? 0.25 * before : before))
         k.status = KS_INDEFINITE;
     else if (k.iter >= k.max_iter)
         k.status = KS_MAXIT;
@@ -1262,6 +1273,7 @@ cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int
 }
 
 int launch_fc_iteration(const KrylovWork& w, const FcCg& c, bool first, const double* z, double* q, cudaStream_t s) {
+    first = first || c.minres;
     if (first) {
         k_fc_cg_spmv<true><<<c.n_chunks, 256, 0, s>>>(w, c, z, q);
     } else {

@@ -71,6 +71,7 @@ struct FcPlan {
     std::vector<FcFront> fronts;
     std::vector<int32_t> maps, verts;
     std::vector<int2> jblk;  // {block, row << 16 | column} in the front's [x11; a21] rows
+    std::vector<int32_t> jblk_t;  // the transposed block of each, for an unsymmetric J (else empty)
     std::vector<FcTask> tasks;
     std::vector<FcDepth> depths;  // 0: the roots
     std::vector<FcPanel> panels;
@@ -84,9 +85,10 @@ struct FcPlan {
 
 // Symbolic factorisation of the block pattern (G consecutive nodes form one column with in-plane
 // position X[3 column]); tissue t owns nodes [node0[t], node0[t+1]). plan.ok = false when a front
-// is too large for the kernels or the operation count exceeds max_flops.
+// is too large for the kernels or the operation count exceeds max_flops. transposed: with jblk_t, so that
+// the symmetric part (J + J^T) / 2 of an unsymmetric J is factorised.
 void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colidx, const double* X, int T,
-                       const int32_t* node0, double max_flops, FcPlan& plan);
+                       const int32_t* node0, double max_flops, bool transposed, FcPlan& plan);
 
 // Device side.
 struct FcWork {
@@ -95,6 +97,7 @@ struct FcWork {
     const int32_t* maps;
     const int32_t* verts;
     const int2* jblk;
+    const int32_t* jblk_t;  // NULL: J is symmetric
     const FcTask* tasks;
     const int32_t* active;  // [T]
     double* factor;
@@ -115,8 +118,9 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
 cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
                                 cudaStream_t s);
 
-// Preconditioned conjugate gradients with the factor as preconditioner, one kernel per phase, every
-// tissue with its own scalars. A chunk is a run of rows of one tissue; the dot products are summed
+// Preconditioned iterations with the factor as preconditioner, one kernel per phase, every tissue with its
+// own scalars: conjugate gradients, or for an unsymmetric J the minimal residual iteration (p = z,
+// alpha = (r, q) / (q, q)), which the factor of the symmetric part contracts by the asymmetry. A chunk is a run of rows of one tissue; the dot products are summed
 // per chunk and then per tissue in chunk order.
 struct FcChunk {
     int32_t tissue, row0, row1;
@@ -130,6 +134,7 @@ struct FcCg {
     const int32_t* active;  // [T] tissues of this solve
     int32_t* running;       // [T] still iterating (the preconditioner's active flags)
     double* part;           // [3][n_chunks]: (r, z), (p, J p), (r, r) / (b, b)
+    int32_t minres;         // 1: the minimal residual iteration (part: (r, q), (q, q), (r, r))
 };
 // x = 0, r = b; every active tissue running (unless b = 0)
 cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int max_iter, cudaStream_t s);

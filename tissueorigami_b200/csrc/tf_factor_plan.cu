@@ -206,7 +206,7 @@ void parallel_items(int n, F f) {
 }  // namespace
 
 void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colidx, const double* X, int T,
-                       const int32_t* node0, double max_flops, FcPlan& plan) {
+                       const int32_t* node0, double max_flops, bool transposed, FcPlan& plan) {
     plan = FcPlan();
     const int nc = N / G, gd = 3 * G;
     plan.gd = gd;
@@ -366,9 +366,22 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
     }
     if (nj > INT32_MAX) return;
     plan.jblk.resize(nj);
+    if (transposed) plan.jblk_t.resize(nj);
     parallel_items((nf + step - 1) / step, [&](int chunk) {
-        for (int fi = chunk * step; fi < std::min(nf, (chunk + 1) * step); ++fi)
+        for (int fi = chunk * step; fi < std::min(nf, (chunk + 1) * step); ++fi) {
             std::copy(jb[fi].begin(), jb[fi].end(), plan.jblk.begin() + plan.fronts[fi].j0);
+            if (!transposed) continue;
+            const Dissection& D = ds[of[fi].first];
+            const Node& f = D.nodes[of[fi].second];
+            const int c0 = node0[of[fi].first] / G;
+            for (size_t k = 0; k < jb[fi].size(); ++k) {  // block (node, other) -> (other, node)
+                const int e = jb[fi][k].x, col = jb[fi][k].y & 0xffff;
+                const int node = (f.piv[col / gd] + c0) * G + (col % gd) / 3, other = colidx[e];
+                const int32_t* r0 = colidx + rowptr[other];
+                const int32_t* r1 = colidx + rowptr[other + 1];
+                plan.jblk_t[plan.fronts[fi].j0 + k] = (int32_t)(std::lower_bound(r0, r1, node) - colidx);
+            }
+        }
     });
     // task lists, the tasks of a launch by falling front size (the long ones start first)
     auto cdiv = [](int a, int b) { return (a + b - 1) / b; };

@@ -46,6 +46,7 @@ enum KrylovMethod : int32_t {
     KM_CG = 2,           // preconditioned conjugate gradients (symmetric J)
     KM_CG_FALLBACK = 3,  // CG met a non-positive curvature; BiCGStab solved the system
     KM_MINRES = 4,       // MINRES with the |D| block preconditioner (symmetric J with packing pairs)
+    KM_MINIMAL_RESIDUAL = 5,  // minimal residual iteration with the factor of (J + J^T) / 2 (unsymmetric J)
 };
 
 enum KrylovStatus : int32_t {
