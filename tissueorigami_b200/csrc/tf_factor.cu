@@ -20,7 +20,7 @@ constexpr int kT = kFcTile;
 constexpr int kLd = kT + 4;  // shared leading dimension: 8-byte reads of a fragment hit distinct banks
 constexpr int kKc = 16;      // K extent of one stage of the long GEMMs
 constexpr int kKld = kKc + 4;
-constexpr int kStages = 2;
+constexpr int kStages = 3;
 
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -32,60 +32,61 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes));
 }
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N));
 }
 
+// base[off] where ok, else 0, without a branch: a load behind a branch is waited for before the next one
+// is issued, and the gathers below live on having all of theirs in flight (base is always readable).
+__device__ __forceinline__ double load_if(const double* __restrict__ base, bool ok, size_t off) {
+    const double v = base[ok ? off : 0];
+    return ok ? v : 0.0;
+}
+
 // ---- assembly of a front -------------------------------------------------------------------
 
-// Rows [32 i, 32 i + 32) of the front's pivot columns: what its children left there. Rows below p
+// Rows [i j, (i + 1) j) of the front's pivot columns (task j: 8 or 32): what its children left there. Rows below p
 // need the columns up to the diagonal only.
 __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int parity) {
     extern __shared__ int2 s_col[];  // per pivot column: its index on either child's boundary
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
-    const double* C[2] = {nullptr, nullptr};
-    int ldc[2] = {0, 0};
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-        if (F.child[q] >= 0) {
-            C[q] = w.contrib[parity ^ 1] + F.child_c[q];
-            ldc[q] = F.child_ldb[q];
-        }
+    const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
+    const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
+    const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
     for (int c = threadIdx.x; c < F.p; c += blockDim.x) {
         const int v = c / w.gd, r = c - v * w.gd;
-        int m[2] = {-1, -1};
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-            if (C[q]) {
-                const int k = w.maps[F.map[q] + v];
-                if (k >= 0) m[q] = k * w.gd + r;
-            }
-        s_col[c] = make_int2(m[0], m[1]);
+        const int k0 = F.child[0] >= 0 ? w.maps[F.map[0] + v] : -1, k1 = F.child[1] >= 0 ? w.maps[F.map[1] + v] : -1;
+        s_col[c] = make_int2(k0 >= 0 ? k0 * w.gd + r : -1, k1 >= 0 ? k1 * w.gd + r : -1);
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r1 = min((tk.i + 1) * kFcGatherRows, F.p + F.b);
-    for (int row = tk.i * kFcGatherRows + warp; row < r1; row += 8) {
+    const int r1 = min((tk.i + 1) * tk.j, F.p + F.b);
+    for (int row = tk.i * tk.j + warp; row < r1; row += 8) {
         const int v = row / w.gd, r = row - v * w.gd;
-        const double* R[2] = {nullptr, nullptr};
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-            if (C[q]) {
-                const int k = w.maps[F.map[q] + v];
-                if (k >= 0) R[q] = C[q] + (size_t)(k * w.gd + r) * ldc[q];
-            }
+        const int k0 = F.child[0] >= 0 ? w.maps[F.map[0] + v] : -1, k1 = F.child[1] >= 0 ? w.maps[F.map[1] + v] : -1;
+        const double* R0 = C0 + (k0 >= 0 ? (size_t)(k0 * w.gd + r) * ld0 : 0);
+        const double* R1 = C1 + (k1 >= 0 ? (size_t)(k1 * w.gd + r) * ld1 : 0);
         const int n = row < F.p ? row + 1 : F.p;
         double* out = row < F.p ? w.factor + F.x11 + (size_t)row * F.ldp : w.scratch + F.a21 + (size_t)(row - F.p) * F.ldp;
-#pragma unroll 4
-        for (int c = lane; c < n; c += 32) {
-            const int2 m = s_col[c];
-            const double s0 = R[0] && m.x >= 0 ? R[0][m.x] : 0.0;
-            const double s1 = R[1] && m.y >= 0 ? R[1][m.y] : 0.0;
-            out[c] = s0 + s1;
+        for (int c = lane; c < n; c += 128) {
+            double x0[4], x1[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int2 m = c + 32 * u < n ? s_col[c + 32 * u] : make_int2(-1, -1);
+                x0[u] = load_if(R0, k0 >= 0 && m.x >= 0, m.x);
+                x1[u] = load_if(R1, k1 >= 0 && m.y >= 0, m.y);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c + 32 * u < n) out[c + 32 * u] = x0[u] + x1[u];
         }
     }
 }
@@ -139,9 +140,8 @@ __device__ __forceinline__ void factor_block(const double* s, int ld, int n, Fac
             const int c = 8 * t + 2 * lk + h;
             v[t][h] = r < n && c < n ? (c <= r ? s[r * ld + c] : s[c * ld + r]) : (r == c ? 1.0 : 0.0);
         }
-#pragma unroll
-    for (int kb = 0; kb < 8; ++kb) {
-        if (8 * kb >= n) break;
+#pragma unroll 1  // one copy of the eight steps: eight of them, 64 KB of code, ran from instruction-cache misses
+    for (int kb = 0; 8 * kb < n; ++kb) {
         double(*rows)[kLd] = sh.rows[kb & 1];
         if (w == kb) {
 #pragma unroll
@@ -150,7 +150,13 @@ __device__ __forceinline__ void factor_block(const double* s, int ld, int n, Fac
         __syncthreads();
         if (w < kb) continue;
         double D[2] = {rows[lr][8 * kb + 2 * lk], rows[lr][8 * kb + 2 * lk + 1]};
-        double O[2] = {v[kb][0], v[kb][1]};
+        double O[2] = {v[0][0], v[0][1]};
+#pragma unroll
+        for (int t = 1; t < 8; ++t)
+            if (t == kb) {
+                O[0] = v[t][0];
+                O[1] = v[t][1];
+            }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const double d = __shfl_sync(0xffffffffu, D[j & 1], 4 * j + (j >> 1));
@@ -158,13 +164,11 @@ __device__ __forceinline__ void factor_block(const double* s, int ld, int n, Fac
             const double aD = __shfl_sync(0xffffffffu, D[j & 1], (lane & 28) + (j >> 1));
             const double aO = __shfl_sync(0xffffffffu, O[j & 1], (lane & 28) + (j >> 1));
             const double inv = __drcp_rn(d);
-            const double mD = aD * inv, mO = aO * inv;
+            const double mD = lr > j ? aD * inv : 0.0, mO = aO * inv;
             O[0] -= mO * p0;
             O[1] -= mO * p1;
-            if (lr > j) {
-                D[0] -= mD * p0;
-                D[1] -= mD * p1;
-            }
+            D[0] -= mD * p0;
+            D[1] -= mD * p1;
             if (lk == (j >> 1)) {
                 O[j & 1] = -mO;
                 if (lr > j) D[j & 1] = -mD;
@@ -175,8 +179,6 @@ __device__ __forceinline__ void factor_block(const double* s, int ld, int n, Fac
             O[0] = D[0];
             O[1] = D[1];
         }
-        v[kb][0] = O[0];
-        v[kb][1] = O[1];
         // the tile as an A fragment: below the pivots minus the multipliers of the published rows; for the pivot
         // rows L^-1 itself (unit diagonal)
         double a[2];
@@ -189,7 +191,11 @@ __device__ __forceinline__ void factor_block(const double* s, int ld, int n, Fac
         }
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            if (t == kb) continue;
+            if (t == kb) {
+                v[t][0] = O[0];
+                v[t][1] = O[1];
+                continue;
+            }
             if (w == kb) v[t][0] = v[t][1] = 0.0;
             mma_f64(v[t], a[0], rows[lk][8 * t + lr]);
             mma_f64(v[t], a[1], rows[4 + lk][8 * t + lr]);
@@ -441,43 +447,29 @@ __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
 // gathered, completed with the Jacobian's blocks, factorised and turned into l21 in shared memory, and the
 // contribution is formed from there. One launch per depth instead of five, and A21 never leaves the
 // SM; the bottom half of a tree is made of such fronts.
-// Dynamic shared memory: A11 / G^-1 and A21 / l21 (rows of ld doubles), the map of both children (ints).
-__device__ __host__ __forceinline__ int small_ld(int p) { return ((p + 15) & ~15) + 4; }
-__device__ __host__ __forceinline__ int small_smem(int p, int b) {
-    return (((p + 7) & ~7) + ((b + 31) & ~31)) * small_ld(p) * 8 + 2 * (p + b) * 4;
-}
-
-__global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __restrict__ vals, int begin, int parity) {
+__global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __restrict__ vals, int begin, int parity) {
     extern __shared__ __align__(16) double s_dyn[];
     __shared__ FactorShared sh;
     __shared__ double s_sign[kT];
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
-    const int p = F.p, b = F.b, n = p + b, ld = small_ld(p), p8r = (p + 7) & ~7, b32 = (b + 31) & ~31;
+    const int p = F.p, b = F.b, n = p + b, ld = fc_small_ld(p), p8r = (p + 7) & ~7, b16 = (b + 15) & ~15;
     double* sX = s_dyn;
     double* sL = sX + p8r * ld;
-    int* s_map = reinterpret_cast<int*>(sL + b32 * ld);  // [2][n]
+    int* s_map = reinterpret_cast<int*>(sL + b16 * ld);  // [2][n]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const double* C[2] = {nullptr, nullptr};
-    int ldc[2] = {0, 0};
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-        if (F.child[q] >= 0) {
-            C[q] = w.contrib[parity ^ 1] + F.child_c[q];
-            ldc[q] = F.child_ldb[q];
-        }
+    const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
+    const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
+    const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
     for (int e = tid; e < 2 * n; e += 256) {
         const int q = e >= n, c = e - q * n;
-        int m = -1;
-        if (C[q]) {
-            const int v = c / w.gd, k = w.maps[F.map[q] + v];
-            if (k >= 0) m = k * w.gd + (c - v * w.gd);
-        }
-        s_map[e] = m;
+        const int v = c / w.gd, k = F.child[q] >= 0 ? w.maps[F.map[q] + v] : -1;
+        s_map[e] = k >= 0 ? k * w.gd + (c - v * w.gd) : -1;
     }
-    for (int e = tid; e < (p8r + b32) * ld; e += 256) s_dyn[e] = 0.0;
+    for (int e = tid; e < (p8r + b16) * ld; e += 256) s_dyn[e] = 0.0;
     __syncthreads();
+    // the Jacobian's entries go straight to their places, in flight while the children's are read
     {
         const int n9 = (F.j1 - F.j0) * 9;
 #pragma unroll 4
@@ -485,34 +477,46 @@ __global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __rest
             const int k = e / 9, en = e - k * 9, cc = en / 3, rr = en - cc * 3;
             const int2 jb = w.jblk[F.j0 + k];
             const int row = (int)((uint32_t)jb.y >> 16) + rr, col = (jb.y & 0xffff) + cc;
-            (row < p ? sX + row * ld : sL + (row - p) * ld)[col] = j_entry(w, vals, F.j0 + k, jb.x, cc, rr);
+            double* dst = (row < p ? sX + row * ld : sL + (row - p) * ld) + col;
+            if (w.jblk_t)
+                *dst = j_entry(w, vals, F.j0 + k, jb.x, cc, rr);
+            else
+                cp_async8(dst, vals + (size_t)jb.x * 9 + en);
         }
+        cp_commit();
     }
-    __syncthreads();
-    if (C[0] || C[1]) {  // eight rows a warp pass, the loads of all of them in flight
+    if (F.child[0] >= 0) {  // eight rows a warp pass, the loads of all of them in flight
+        bool first = true;
         for (int r0 = warp; r0 < n; r0 += 64)
-            for (int c = lane; c < p; c += 32) {
-                const int c0 = s_map[c], c1 = s_map[n + c];
-                double x[8];
+            for (int c = lane; c < ((p + 31) & ~31); c += 32) {
+                const int c0 = c < p ? s_map[c] : -1, c1 = c < p ? s_map[n + c] : -1;
+                double x[8], y[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const int row = r0 + 8 * u;
-                    double s = 0.0;
-                    if (row < n && (row >= p || c <= row)) {
-                        const int m0 = s_map[row], m1 = s_map[n + row];
-                        if (m0 >= 0 && c0 >= 0) s = C[0][(size_t)m0 * ldc[0] + c0];
-                        if (m1 >= 0 && c1 >= 0) s += C[1][(size_t)m1 * ldc[1] + c1];
-                    }
-                    x[u] = s;
+                    const int row = min(r0 + 8 * u, n - 1), m0 = s_map[row], m1 = s_map[n + row];
+                    const bool in = r0 + 8 * u < n && (row >= p || c <= row);
+                    x[u] = load_if(C0, in && m0 >= 0 && c0 >= 0, (size_t)m0 * ld0 + c0);
+                    y[u] = load_if(C1, in && m1 >= 0 && c1 >= 0, (size_t)m1 * ld1 + c1);
+                }
+                if (first) {  // the same pass in every thread: the Jacobian's entries are in place
+                    cp_wait<0>();
+                    __syncthreads();
+                    first = false;
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int row = r0 + 8 * u;
-                    if (row < n && (row >= p || c <= row)) (row < p ? sX + row * ld : sL + (row - p) * ld)[c] += x[u];
+                    if (row < n && c < p && (row >= p || c <= row)) (row < p ? sX + row * ld : sL + (row - p) * ld)[c] += x[u] + y[u];
                 }
             }
-        __syncthreads();
+        if (first) {  // a warp without rows
+            cp_wait<0>();
+            __syncthreads();
+        }
+    } else {
+        cp_wait<0>();
     }
+    __syncthreads();
     {
         double v[8][2];
         factor_block(sX, ld, p, sh, v, s_sign, w.flags + F.tissue, w.neg + tk.front);
@@ -521,7 +525,8 @@ __global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __rest
         if (r < p8r)
 #pragma unroll
             for (int t = 0; t < 8; ++t)
-                if (8 * t < p) *reinterpret_cast<double2*>(sX + r * ld + 8 * t + 2 * (lane & 3)) = make_double2(v[t][0], v[t][1]);
+                if (8 * t + 2 * (lane & 3) < ld)
+                    *reinterpret_cast<double2*>(sX + r * ld + 8 * t + 2 * (lane & 3)) = make_double2(v[t][0], v[t][1]);
         __syncthreads();
         if (tid < p) w.sign[F.piv + tid] = s_sign[tid];
     }
@@ -555,59 +560,58 @@ __global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __rest
         }
     }
     __syncthreads();
-    // contribution, 16 x 32 tiles of the lower triangle
+    // contribution, 16 x 16 tiles of the lower triangle
     const bool neg = w.neg[tk.front] != 0;
     double* Cf = w.contrib[parity] + F.c;
-    int task = 0;
-    for (int i = 0; i * 16 < b; ++i)
-        for (int j = 0; j * 32 <= i * 16 + 15 && j * 32 < b; ++j, ++task) {
-            if ((task & 7) != warp) continue;
-            // the children's entries are fetched ahead of the product
-            double acc[2][4][2], kid[2][4][2];
+    const int nt = b16 >> 4;
+    for (int task = warp; task < nt * (nt + 1) / 2; task += 8) {
+        int i = (int)((sqrtf(8.0f * task + 1.0f) - 1.0f) * 0.5f);
+        while ((i + 1) * (i + 2) / 2 <= task) ++i;
+        while (i * (i + 1) / 2 > task) --i;
+        const int j = task - i * (i + 1) / 2;
+        double acc[2][2][2];  // from minus the children's entries
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int y = 0; y < 4; ++y)
+            for (int y = 0; y < 2; ++y)
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int r = i * 16 + 8 * x + lr, c = j * 32 + 8 * y + 2 * lk + h;
-                        double s = 0.0;
-                        if (r < b && c <= r) {
-                            const int r0 = s_map[p + r], c0 = s_map[p + c], r1 = s_map[n + p + r], c1 = s_map[n + p + c];
-                            if (r0 >= 0 && c0 >= 0) s = C[0][(size_t)r0 * ldc[0] + c0];
-                            if (r1 >= 0 && c1 >= 0) s += C[1][(size_t)r1 * ldc[1] + c1];
-                        }
-                        kid[x][y][h] = s;
-                        acc[x][y][h] = 0.0;
-                    }
-            const double* A = sL + (i * 16 + lr) * ld + lk;
-            const double* B = sL + (j * 32 + lr) * ld + lk;
-            for (int k = 0; k < p; k += 4) {
-                double av[2], bv[4];
-#pragma unroll
-                for (int x = 0; x < 2; ++x) av[x] = A[8 * x * ld + k];
-#pragma unroll
-                for (int y = 0; y < 4; ++y) bv[y] = B[8 * y * ld + k];
-                if (neg) {
-                    const double sg = k + lk < p ? s_sign[k + lk] : 0.0;
-#pragma unroll
-                    for (int y = 0; y < 4; ++y) bv[y] *= sg;
+                for (int h = 0; h < 2; ++h) {
+                    const int r = i * 16 + 8 * x + lr, c = j * 16 + 8 * y + 2 * lk + h;
+                    const bool in = r < b && c <= r;
+                    const int rr = in ? p + r : 0, cc = in ? p + c : 0;
+                    const int r0 = s_map[rr], c0 = s_map[cc], r1 = s_map[n + rr], c1 = s_map[n + cc];
+                    acc[x][y][h] = -load_if(C0, in && r0 >= 0 && c0 >= 0, (size_t)r0 * ld0 + c0) -
+                                   load_if(C1, in && r1 >= 0 && c1 >= 0, (size_t)r1 * ld1 + c1);
                 }
+        const double* A = sL + (i * 16 + lr) * ld + lk;
+        const double* B = sL + (j * 16 + lr) * ld + lk;
+#pragma unroll 2
+        for (int k = 0; k < p; k += 4) {
+            double av[2], bv[2];
 #pragma unroll
-                for (int x = 0; x < 2; ++x)
+            for (int x = 0; x < 2; ++x) av[x] = A[8 * x * ld + k];
 #pragma unroll
-                    for (int y = 0; y < 4; ++y) mma_f64(acc[x][y], av[x], bv[y]);
+            for (int y = 0; y < 2; ++y) bv[y] = B[8 * y * ld + k];
+            if (neg) {
+                const double sg = k + lk < p ? s_sign[k + lk] : 0.0;
+#pragma unroll
+                for (int y = 0; y < 2; ++y) bv[y] *= sg;
             }
 #pragma unroll
             for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int y = 0; y < 4; ++y)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int r = i * 16 + 8 * x + lr, c = j * 32 + 8 * y + 2 * lk + h;
-                        if (r < b && c <= r) Cf[(size_t)r * F.ldb + c] = kid[x][y][h] - acc[x][y][h];
-                    }
+                for (int y = 0; y < 2; ++y) mma_f64(acc[x][y], av[x], bv[y]);
         }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = i * 16 + 8 * x + lr, c = j * 16 + 8 * y + 2 * lk + h;
+                    if (r < b && c <= r) Cf[(size_t)r * F.ldb + c] = -acc[x][y][h];
+                }
+    }
 }
 
 // ---- boundary GEMMs ---------------------------------------------------------------------------
@@ -615,8 +619,9 @@ __global__ void __launch_bounds__(256) k_fc_small(FcWork w, const double* __rest
 // 64 x 64 tile of A B^T, both row-major with K contiguous, by 4 warps (32 x 32 each: 16 accumulator
 // tiles hide the tensor instruction's latency), K in stages of 16 through a 3-stage cp.async ring.
 // a_rows / b_rows: valid rows (0 outside); K: valid columns; B's columns times sign unless it is null.
+template <class Init>
 __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, const double* B, int ldb, int b_rows, int K,
-                                          const double* sign, double* smem, double (&acc)[4][4][2]) {
+                                          const double* sign, double* smem, double (&acc)[4][4][2], Init init) {
     double* sa = smem;
     double* sb = smem + kStages * kT * kKld;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -633,14 +638,11 @@ __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, 
         }
     };
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-#pragma unroll
     for (int st = 0; st < kStages - 1; ++st) {
         if (st < n_it) load(st);
         cp_commit();
     }
+    init();  // the accumulators, while the first stages are on their way
     const int ra = (warp >> 1) * 32 + (lane >> 2), rb = (warp & 1) * 32 + (lane >> 2), kk = lane & 3;
     for (int it = 0; it < n_it; ++it) {
         cp_wait<kStages - 2>();
@@ -682,7 +684,12 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.p - j * kT);
     double acc[4][4][2];
     gemm_tile(w.scratch + F.a21 + (size_t)i * kT * F.ldp, F.ldp, ni, w.factor + F.x11 + (size_t)j * kT * F.ldp, F.ldp, nj,
-                     min(F.p, (j + 1) * kT), nullptr, s_dyn, acc);
+                     min(F.p, (j + 1) * kT), nullptr, s_dyn, acc, [&] {
+#pragma unroll
+                 for (int a = 0; a < 4; ++a)
+#pragma unroll
+                     for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+             });
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
     double* out = w.factor + F.l21 + (size_t)i * kT * F.ldp + j * kT;
@@ -699,7 +706,7 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
 }
 
 // Contribution tile (i, j <= i): what the children left there minus l21 S l21^T.
-__global__ void __launch_bounds__(128) k_fc_schur(FcWork w, int begin, int parity) {
+__global__ void __launch_bounds__(128, 3) k_fc_schur(FcWork w, int begin, int parity) {
     extern __shared__ __align__(16) double s_dyn[];
     __shared__ int s_map[2][2][kT];  // child, rows / columns
     const FcTask tk = w.tasks[begin + blockIdx.x];
@@ -708,29 +715,35 @@ __global__ void __launch_bounds__(128) k_fc_schur(FcWork w, int begin, int parit
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.b - j * kT);
     for (int e = threadIdx.x; e < 4 * kT; e += blockDim.x) {
         const int q = e >> 7, side = (e >> 6) & 1, c = e & 63, idx = (side ? j : i) * kT + c;
-        int m = -1;
-        if (F.child[q] >= 0 && idx < F.b) {
-            const int v = (F.p + idx) / w.gd, r = F.p + idx - v * w.gd;
-            const int k = w.maps[F.map[q] + v];
-            if (k >= 0) m = k * w.gd + r;
-        }
-        s_map[q][side][c] = m;
+        const int v = (F.p + idx) / w.gd, r = F.p + idx - v * w.gd;
+        const int k = F.child[q] >= 0 && idx < F.b ? w.maps[F.map[q] + v] : -1;
+        s_map[q][side][c] = k >= 0 ? k * w.gd + r : -1;
     }
-    double acc[4][4][2];
-    const double* L = w.factor + F.l21;
-    gemm_tile(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p,
-              w.neg[tk.front] ? w.sign + F.piv : nullptr, s_dyn, acc);
-    __syncthreads();
-    const double* C[2] = {nullptr, nullptr};
-    int ldc[2] = {0, 0};
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-        if (F.child[q] >= 0) {
-            C[q] = w.contrib[parity ^ 1] + F.child_c[q];
-            ldc[q] = F.child_ldb[q];
-        }
+    const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
+    const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
+    const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
+    double acc[4][4][2];
+    const double* L = w.factor + F.l21;
+    // the product accumulates onto minus the children's entries, so that nothing but stores follows it
+    gemm_tile(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p,
+              w.neg[tk.front] ? w.sign + F.piv : nullptr, s_dyn, acc, [&] {
+                  __syncthreads();  // s_map
+#pragma unroll
+                  for (int a = 0; a < 4; ++a) {
+                      const int r = r0 + 8 * a, m0 = s_map[0][0][r], m1 = s_map[1][0][r];
+#pragma unroll
+                      for (int b = 0; b < 4; ++b)
+#pragma unroll
+                          for (int h = 0; h < 2; ++h) {
+                              const int c = c0 + 8 * b + h, k0 = s_map[0][1][c], k1 = s_map[1][1][c];
+                              const bool in = i != j || c <= r;
+                              acc[a][b][h] = -load_if(C0, in && m0 >= 0 && k0 >= 0, (size_t)m0 * ld0 + k0) -
+                                             load_if(C1, in && m1 >= 0 && k1 >= 0, (size_t)m1 * ld1 + k1);
+                          }
+                  }
+              });
     double* out = w.contrib[parity] + F.c + (size_t)i * kT * F.ldb + j * kT;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -739,14 +752,7 @@ __global__ void __launch_bounds__(128) k_fc_schur(FcWork w, int begin, int parit
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = r0 + 8 * a, c = c0 + 8 * b + h;
-                if (r >= ni || c >= nj || (i == j && c > r)) continue;
-                double s = -acc[a][b][h];
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int mr = s_map[q][0][r], mc = s_map[q][1][c];
-                    if (mr >= 0 && mc >= 0) s += C[q][(size_t)mr * ldc[q] + mc];
-                }
-                out[(size_t)r * F.ldb + c] = s;
+                if (r < ni && c < nj && (i != j || c <= r)) out[(size_t)r * F.ldb + c] = -acc[a][b][h];
             }
 }
 
@@ -755,14 +761,10 @@ __global__ void __launch_bounds__(128) k_fc_schur(FcWork w, int begin, int parit
 // The children's share of entry `idx` (pivots, then boundary) of a front's right-hand side.
 __device__ __forceinline__ double from_children(const FcWork& w, const FcFront& F, int idx) {
     const int v = idx / w.gd, r = idx - v * w.gd;
-    double s = 0.0;
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-        if (F.child[q] >= 0) {
-            const int k = w.maps[F.map[q] + v];
-            if (k >= 0) s += w.vec[F.child_vec[q] + k * w.gd + r];
-        }
-    return s;
+    const int k0 = w.maps[F.child[0] >= 0 ? F.map[0] + v : 0], k1 = w.maps[F.child[1] >= 0 ? F.map[1] + v : 0];
+    const bool ok0 = F.child[0] >= 0 && k0 >= 0, ok1 = F.child[1] >= 0 && k1 >= 0;
+    const double x = w.vec[ok0 ? F.child_vec[0] + k0 * w.gd + r : 0], y = w.vec[ok1 ? F.child_vec[1] + k1 * w.gd + r : 0];
+    return (ok0 ? x : 0.0) + (ok1 ? y : 0.0);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -1161,7 +1163,7 @@ cudaError_t opt_in(const void* f, int bytes) { return cudaFuncSetAttribute(f, cu
 
 cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, cudaStream_t s) {
     // per-device attributes of the kernels; cheap next to a factorisation
-    FC_CK(opt_in((const void*)k_fc_small, small_smem(kT, kFcSmallB)));
+    FC_CK(opt_in((const void*)k_fc_small, fc_small_smem(kT, kFcSmallB)));
     FC_CK(opt_in((const void*)k_fc_col, kPanelSmem));
     FC_CK(opt_in((const void*)k_fc_upd, kPanelSmem));
     FC_CK(opt_in((const void*)k_fc_l21, kGemmSmem));
@@ -1174,7 +1176,7 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
                 int smem = 0;
                 for (int k = 0; k < r.count; ++k) {
                     const FcFront& F = plan.fronts[plan.tasks[r.begin + k].front];
-                    smem = smem < small_smem(F.p, F.b) ? small_smem(F.p, F.b) : smem;
+                    smem = smem < fc_small_smem(F.p, F.b) ? fc_small_smem(F.p, F.b) : smem;
                 }
                 k_fc_small<<<r.count, 256, smem, s>>>(w, vals, r.begin, d & 1);
                 ++n;

@@ -21,7 +21,6 @@
 namespace tfb {
 
 constexpr int kFcTile = 64;        // pivot panel width and GEMM tile
-constexpr int kFcGatherRows = 32;  // rows of a front per assembly task
 constexpr int kFcScatter = 256;    // Jacobian blocks per assembly task
 constexpr int kFcSmallB = 288;     // boundary unknowns up to which a one-panel front is one CTA's
 constexpr int kFcSmallSolve = 49152; // entries of x11 and l21 up to which a front's solve is one CTA's
@@ -50,6 +49,16 @@ struct FcTask {
     int32_t front;
     int16_t i, j;
 };
+
+// One-CTA fronts keep [A11; A21] in shared memory: leading dimension (4 mod 8: the fragments' reads hit
+// distinct banks) and bytes, with the two children's maps.
+__host__ __device__ inline int fc_small_ld(int p) {
+    const int l = (p + 3) & ~3;
+    return l % 8 ? l : l + 4;
+}
+__host__ __device__ inline int fc_small_smem(int p, int b) {
+    return (((p + 7) & ~7) + ((b + 15) & ~15)) * fc_small_ld(p) * 8 + 2 * (p + b) * 4;
+}
 
 struct FcRange {
     int32_t begin = 0, count = 0;

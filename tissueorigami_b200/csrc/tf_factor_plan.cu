@@ -402,18 +402,20 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
         for (int32_t fi : fs)
             if (!is_small(plan.fronts[fi])) rest.push_back(fi);
         std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) { return plan.fronts[a].b > plan.fronts[b].b; });
-        // in three launches by the shared memory they need, so that small fronts share an SM (the
-        // bounds leave room for two and three of them)
-        auto entries = [](const FcFront& F) { return (int64_t)(F.p + F.b + 39) * (((F.p + 15) & ~15) + 4); };
-        const int64_t bound[4] = {INT64_MAX, 12800, 8200, 0};
+        // in three launches by the shared memory they need, so that two and three small ones share an SM
+        // (228 KB, 10 KB of it static per CTA)
+        const int bound[4] = {INT32_MAX, 102000, 64000, 0};
         for (int c = 0; c < 3; ++c)
             list(L.small[c], [&](int32_t fi, const FcFront& F) {
-                if (is_small(F) && entries(F) <= bound[c] && entries(F) > bound[c + 1]) push(fi, 0, 0);
+                if (!is_small(F)) return;
+                const int bytes = fc_small_smem(F.p, F.b);
+                if (bytes <= bound[c] && bytes > bound[c + 1]) push(fi, 0, 0);
             });
         fs = rest;
         list(L.gather, [&](int32_t fi, const FcFront& F) {
+            const int rows = F.p > 128 ? 8 : 32;  // long rows: one a warp
             if (F.p > 0)
-                for (int i = 0; i < cdiv(F.p + F.b, kFcGatherRows); ++i) push(fi, i, 0);
+                for (int i = 0; i < cdiv(F.p + F.b, rows); ++i) push(fi, i, rows);
         });
         list(L.scatter, [&](int32_t fi, const FcFront& F) {
             for (int i = 0; i < cdiv(F.j1 - F.j0, kFcScatter); ++i) push(fi, i, 0);
