@@ -183,7 +183,7 @@ struct tf_ctx {
     // whose launch alone, 3.4 us each, took longer than many of them): replayed as graphs (0.75 us each)
     cudaGraphExec_t fc_graph[2] = {nullptr, nullptr};
     int64_t fc_graph_launches[2] = {0, 0};
-    DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_jblk_t, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_tp, fc_vec, fc_z,
+    DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_jblk_t, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_kids, fc_dofs, fc_vec, fc_z,
         fc_sign, fc_flags, fc_neg, fc_chunks, fc_chunk0_d, fc_running, fc_part;
 
     // adjoint: forward checkpoints every adj_k steps, segment recompute buffers, adjoint state
@@ -1727,6 +1727,8 @@ int replay_factor(tf_ctx* ctx, int which, F launch) {
     return TF_OK;
 }
 
+FcWork make_factor(tf_ctx* c);
+
 int build_factor(tf_ctx* ctx) {
     ctx->fc_dirty = false;
     ctx->fc_ready = false;
@@ -1763,7 +1765,6 @@ int build_factor(tf_ctx* ctx) {
     if (e == cudaSuccess) e = room(ctx->fc_scratch, P.n_scratch);
     for (int q = 0; q < 2; ++q)
         if (e == cudaSuccess) e = room(ctx->fc_contrib[q], P.n_contrib[q]);
-    if (e == cudaSuccess) e = room(ctx->fc_tp, P.n_tp);
     if (e == cudaSuccess) e = room(ctx->fc_vec, P.n_vec);
     if (e == cudaSuccess) e = room(ctx->fc_z, P.n_piv);
     if (e == cudaSuccess) e = room(ctx->fc_sign, P.n_piv);
@@ -1783,9 +1784,14 @@ int build_factor(tf_ctx* ctx) {
     TF_CK(up(ctx->fc_jblk, P.jblk.data(), sizeof(int2) * P.jblk.size()));
     TF_CK(up(ctx->fc_jblk_t, P.jblk_t.data(), sizeof(int32_t) * P.jblk_t.size()));
     TF_CK(up(ctx->fc_tasks, P.tasks.data(), sizeof(FcTask) * P.tasks.size()));
+    TF_CK(dalloc(ctx->fc_kids, sizeof(int2) * (size_t)P.n_ent));
+    TF_CK(dalloc(ctx->fc_dofs, sizeof(int32_t) * (size_t)P.n_ent));
     TF_CK(up(ctx->fc_chunks, chunks.data(), sizeof(FcChunk) * chunks.size()));
     TF_CK(up(ctx->fc_chunk0_d, ctx->fc_chunk0.data(), sizeof(int32_t) * ctx->fc_chunk0.size()));
+    TF_CK(launch_factor_expand(P, make_factor(ctx), dptr<int32_t>(ctx->fc_maps), dptr<int32_t>(ctx->fc_verts), ctx->stream));
     TF_CK(cudaStreamSynchronize(ctx->stream));
+    dfree(ctx->fc_maps);
+    dfree(ctx->fc_verts);
     // the launches need the task ranges and the fronts' sizes only
     P.maps = {};
     P.verts = {};
@@ -1799,8 +1805,8 @@ FcWork make_factor(tf_ctx* c) {
     FcWork f{};
     f.gd = c->fc.gd;
     f.fronts = dptr<FcFront>(c->fc_fronts);
-    f.maps = dptr<int32_t>(c->fc_maps);
-    f.verts = dptr<int32_t>(c->fc_verts);
+    f.kids = dptr<int2>(c->fc_kids);
+    f.dofs = dptr<int32_t>(c->fc_dofs);
     f.jblk = dptr<int2>(c->fc_jblk);
     f.jblk_t = c->has_visc ? dptr<int32_t>(c->fc_jblk_t) : nullptr;
     f.tasks = dptr<FcTask>(c->fc_tasks);
@@ -1809,7 +1815,6 @@ FcWork make_factor(tf_ctx* c) {
     f.scratch = dptr<double>(c->fc_scratch);
     f.contrib[0] = dptr<double>(c->fc_contrib[0]);
     f.contrib[1] = dptr<double>(c->fc_contrib[1]);
-    f.tp = dptr<double>(c->fc_tp);
     f.vec = dptr<double>(c->fc_vec);
     f.z = dptr<double>(c->fc_z);
     f.sign = dptr<double>(c->fc_sign);
@@ -2705,7 +2710,7 @@ void tf_destroy(tf_ctx* ctx) {
                      &ctx->ml_out_set_d, &ctx->ml_out_col_d, &ctx->ml_out_dst_d, &ctx->ml_pairs_d, &ctx->ml_pos_leaf_d};
     for (DevBuf* b : mlb) dfree(*b);
     DevBuf* fcb[] = {&ctx->fc_fronts, &ctx->fc_maps, &ctx->fc_verts, &ctx->fc_jblk, &ctx->fc_jblk_t, &ctx->fc_tasks, &ctx->fc_factor,
-                     &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1], &ctx->fc_tp, &ctx->fc_vec, &ctx->fc_z,
+                     &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1], &ctx->fc_kids, &ctx->fc_dofs, &ctx->fc_vec, &ctx->fc_z,
                      &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_neg, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
     for (DevBuf* b : fcb) dfree(*b);
     drop_factor_graphs(ctx);

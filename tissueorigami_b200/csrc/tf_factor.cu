@@ -20,7 +20,7 @@ constexpr int kT = kFcTile;
 constexpr int kLd = kT + 4;  // shared leading dimension: 8-byte reads of a fragment hit distinct banks
 constexpr int kKc = 16;      // K extent of one stage of the long GEMMs
 constexpr int kKld = kKc + 4;
-constexpr int kStages = 3;
+constexpr int kStages = 2;
 
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -61,19 +61,15 @@ __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int pari
     const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
     const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
     const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
-    for (int c = threadIdx.x; c < F.p; c += blockDim.x) {
-        const int v = c / w.gd, r = c - v * w.gd;
-        const int k0 = F.child[0] >= 0 ? w.maps[F.map[0] + v] : -1, k1 = F.child[1] >= 0 ? w.maps[F.map[1] + v] : -1;
-        s_col[c] = make_int2(k0 >= 0 ? k0 * w.gd + r : -1, k1 >= 0 ? k1 * w.gd + r : -1);
-    }
+    const int2* kids = w.kids + F.ent;
+    for (int c = threadIdx.x; c < F.p; c += blockDim.x) s_col[c] = kids[c];
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r1 = min((tk.i + 1) * tk.j, F.p + F.b);
     for (int row = tk.i * tk.j + warp; row < r1; row += 8) {
-        const int v = row / w.gd, r = row - v * w.gd;
-        const int k0 = F.child[0] >= 0 ? w.maps[F.map[0] + v] : -1, k1 = F.child[1] >= 0 ? w.maps[F.map[1] + v] : -1;
-        const double* R0 = C0 + (k0 >= 0 ? (size_t)(k0 * w.gd + r) * ld0 : 0);
-        const double* R1 = C1 + (k1 >= 0 ? (size_t)(k1 * w.gd + r) * ld1 : 0);
+        const int2 k = kids[row];
+        const double* R0 = C0 + (k.x >= 0 ? (size_t)k.x * ld0 : 0);
+        const double* R1 = C1 + (k.y >= 0 ? (size_t)k.y * ld1 : 0);
         const int n = row < F.p ? row + 1 : F.p;
         double* out = row < F.p ? w.factor + F.x11 + (size_t)row * F.ldp : w.scratch + F.a21 + (size_t)(row - F.p) * F.ldp;
         for (int c = lane; c < n; c += 128) {
@@ -81,8 +77,8 @@ __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int pari
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int2 m = c + 32 * u < n ? s_col[c + 32 * u] : make_int2(-1, -1);
-                x0[u] = load_if(R0, k0 >= 0 && m.x >= 0, m.x);
-                x1[u] = load_if(R1, k1 >= 0 && m.y >= 0, m.y);
+                x0[u] = load_if(R0, k.x >= 0 && m.x >= 0, m.x);
+                x1[u] = load_if(R1, k.y >= 0 && m.y >= 0, m.y);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -444,8 +440,8 @@ __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
 // ---- small fronts --------------------------------------------------------------------------------
 
 // A front of at most 64 pivots and kFcSmallB boundary unknowns, all of it in one CTA: its [A11; A21] is
-// gathered, completed with the Jacobian's blocks, factorised and turned into l21 in shared memory, and the
-// contribution is formed from there. One launch per depth instead of five, and A21 never leaves the
+// gathered, completed with the Jacobian's blocks, factorised and turned into l21 in shared memory; w21 and
+// the contribution are formed from there. One launch per depth instead of five, and A21 never leaves the
 // SM; the bottom half of a tree is made of such fronts.
 __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __restrict__ vals, int begin, int parity) {
     extern __shared__ __align__(16) double s_dyn[];
@@ -462,10 +458,10 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
     const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
     const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
     const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
-    for (int e = tid; e < 2 * n; e += 256) {
-        const int q = e >= n, c = e - q * n;
-        const int v = c / w.gd, k = F.child[q] >= 0 ? w.maps[F.map[q] + v] : -1;
-        s_map[e] = k >= 0 ? k * w.gd + (c - v * w.gd) : -1;
+    for (int e = tid; e < n; e += 256) {
+        const int2 k = w.kids[F.ent + e];
+        s_map[e] = k.x;
+        s_map[n + e] = k.y;
     }
     for (int e = tid; e < (p8r + b16) * ld; e += 256) s_dyn[e] = 0.0;
     __syncthreads();
@@ -552,10 +548,32 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
             for (int h = 0; h < 2; ++h) {
                 const int c = 8 * j + 2 * lk + h;
                 if (c < p) {
-                    const double x = (d[h] + d2[h]) * s_sign[c];
-                    strip[lr * ld + c] = x;
-                    if (r0 + lr < b) w.factor[F.l21 + (size_t)(r0 + lr) * F.ldp + c] = x;
+                    strip[lr * ld + c] = (d[h] + d2[h]) * s_sign[c];
                 }
+            }
+        }
+    }
+    // w21 = l21 G^-1 straight to memory, strips again (a warp's own)
+    __syncwarp();
+    for (int r0 = warp * 8; r0 < b; r0 += 64) {
+        const double* strip = sL + (size_t)r0 * ld;
+        double a[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) a[k] = 4 * k < p ? strip[lr * ld + 4 * k + lk] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j >= p8) break;
+            double d[2] = {0.0, 0.0}, d2[2] = {0.0, 0.0};
+#pragma unroll
+            for (int k = 2 * j; k < 16; k += 2) {
+                if (4 * k >= p) break;
+                mma_f64(d, a[k], 4 * k + lk < p ? sX[(4 * k + lk) * ld + 8 * j + lr] : 0.0);
+                mma_f64(d2, a[k + 1], 4 * k + 4 + lk < p ? sX[(4 * k + 4 + lk) * ld + 8 * j + lr] : 0.0);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = 8 * j + 2 * lk + h;
+                if (c < p && r0 + lr < b) w.factor[F.w21 + (size_t)(r0 + lr) * F.ldp + c] = d[h] + d2[h];
             }
         }
     }
@@ -616,10 +634,10 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
 
 // ---- boundary GEMMs ---------------------------------------------------------------------------
 
-// 64 x 64 tile of A B^T, both row-major with K contiguous, by 4 warps (32 x 32 each: 16 accumulator
+// 64 x 64 tile of A B^T (BT: B as [column][k]) or A B (B as [k][column], b_rows columns valid), row-major, by 4 warps (32 x 32 each: 16 accumulator
 // tiles hide the tensor instruction's latency), K in stages of 16 through a 3-stage cp.async ring.
 // a_rows / b_rows: valid rows (0 outside); K: valid columns; B's columns times sign unless it is null.
-template <class Init>
+template <bool BT, class Init>
 __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, const double* B, int ldb, int b_rows, int K,
                                           const double* sign, double* smem, double (&acc)[4][4][2], Init init) {
     double* sa = smem;
@@ -632,9 +650,16 @@ __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, 
         for (int e = 0; e < 4; ++e) {  // 64 rows x 8 chunks of two doubles
             const int id = threadIdx.x + e * 128, r = id >> 3, c = (id & 7) * 2, left = K - (k0 + c);
             const int nb = left >= 2 ? 16 : (left > 0 ? 8 : 0);
-            const int na_ = r < a_rows ? nb : 0, nb_ = r < b_rows ? nb : 0;
+            const int na_ = r < a_rows ? nb : 0;
             cp_async16(sa + (st * kT + r) * kKld + c, na_ ? A + (size_t)r * lda + k0 + c : A, na_);
-            cp_async16(sb + (st * kT + r) * kKld + c, nb_ ? B + (size_t)r * ldb + k0 + c : B, nb_);
+            if (BT) {
+                const int nb_ = r < b_rows ? nb : 0;
+                cp_async16(sb + (st * kT + r) * kKld + c, nb_ ? B + (size_t)r * ldb + k0 + c : B, nb_);
+            } else {  // 16 rows x 32 chunks
+                const int kr = id >> 5, bc = (id & 31) * 2, bl = k0 + kr < K ? b_rows - bc : 0;
+                const int nb_ = bl >= 2 ? 16 : (bl > 0 ? 8 : 0);
+                cp_async16(sb + st * kT * kKld + kr * kLd + bc, nb_ ? B + (size_t)(k0 + kr) * ldb + bc : B, nb_);
+            }
         }
     };
 #pragma unroll
@@ -650,14 +675,14 @@ __device__ __forceinline__ void gemm_tile(const double* A, int lda, int a_rows, 
         if (it + kStages - 1 < n_it) load(it + kStages - 1);
         cp_commit();
         const double* pa = sa + ((it % kStages) * kT + ra) * kKld + kk;
-        const double* pb = sb + ((it % kStages) * kT + rb) * kKld + kk;
+        const double* pb = BT ? sb + ((it % kStages) * kT + rb) * kKld + kk : sb + (it % kStages) * kT * kKld + kk * kLd + rb;
 #pragma unroll
         for (int k = 0; k < kKc; k += 4) {
             double a[4], b[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) a[i] = pa[8 * i * kKld + k];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = pb[8 * j * kKld + k];
+            for (int j = 0; j < 4; ++j) b[j] = BT ? pb[8 * j * kKld + k] : pb[k * kLd + 8 * j];
             if (sign) {
                 const int kc = it * kKc + k + kk;
                 const double sg = kc < K ? sign[kc] : 0.0;
@@ -683,7 +708,7 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
     if (!w.active[F.tissue]) return;
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.p - j * kT);
     double acc[4][4][2];
-    gemm_tile(w.scratch + F.a21 + (size_t)i * kT * F.ldp, F.ldp, ni, w.factor + F.x11 + (size_t)j * kT * F.ldp, F.ldp, nj,
+    gemm_tile<true>(w.scratch + F.a21 + (size_t)i * kT * F.ldp, F.ldp, ni, w.factor + F.x11 + (size_t)j * kT * F.ldp, F.ldp, nj,
                      min(F.p, (j + 1) * kT), nullptr, s_dyn, acc, [&] {
 #pragma unroll
                  for (int a = 0; a < 4; ++a)
@@ -692,7 +717,7 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
              });
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
-    double* out = w.factor + F.l21 + (size_t)i * kT * F.ldp + j * kT;
+    double* out = w.scratch + F.l21 + (size_t)i * kT * F.ldp + j * kT;
     const double* sg = w.sign + F.piv + j * kT;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -705,29 +730,49 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
             }
 }
 
-// Contribution tile (i, j <= i): what the children left there minus l21 S l21^T.
-__global__ void __launch_bounds__(128, 3) k_fc_schur(FcWork w, int begin, int parity) {
+// Contribution tile (i, j <= i): what the children left there minus l21 S l21^T. Or (j < 0) a tile of w21.
+__global__ void __launch_bounds__(128, 4) k_fc_schur(FcWork w, int begin, int parity) {
     extern __shared__ __align__(16) double s_dyn[];
     __shared__ int s_map[2][2][kT];  // child, rows / columns
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.b - j * kT);
+    const double* L = w.scratch + F.l21;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
+    double acc[4][4][2];
+    if (j < 0) {  // w21 tile: l21 x11, x11 lower triangular
+        const int k0 = (-1 - j) * kT, np = min(kT, F.p - k0);
+        gemm_tile<false>(L + (size_t)i * kT * F.ldp + k0, F.ldp, ni, w.factor + F.x11 + (size_t)k0 * F.ldp + k0, F.ldp, np,
+                         F.p - k0, nullptr, s_dyn, acc, [&] {
+#pragma unroll
+                             for (int a = 0; a < 4; ++a)
+#pragma unroll
+                                 for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+                         });
+        double* out = w.factor + F.w21 + (size_t)i * kT * F.ldp + k0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = r0 + 8 * a, c = c0 + 8 * b + h;
+                    if (r < ni && c < np) out[(size_t)r * F.ldp + c] = acc[a][b][h];
+                }
+        return;
+    }
     for (int e = threadIdx.x; e < 4 * kT; e += blockDim.x) {
         const int q = e >> 7, side = (e >> 6) & 1, c = e & 63, idx = (side ? j : i) * kT + c;
-        const int v = (F.p + idx) / w.gd, r = F.p + idx - v * w.gd;
-        const int k = F.child[q] >= 0 && idx < F.b ? w.maps[F.map[q] + v] : -1;
-        s_map[q][side][c] = k >= 0 ? k * w.gd + r : -1;
+        const int2 k = idx < F.b ? w.kids[F.ent + F.p + idx] : make_int2(-1, -1);
+        s_map[q][side][c] = q ? k.y : k.x;
     }
     const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
     const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
     const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r0 = (warp >> 1) * 32 + (lane >> 2), c0 = (warp & 1) * 32 + 2 * (lane & 3);
-    double acc[4][4][2];
-    const double* L = w.factor + F.l21;
     // the product accumulates onto minus the children's entries, so that nothing but stores follows it
-    gemm_tile(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p,
+    gemm_tile<true>(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p,
               w.neg[tk.front] ? w.sign + F.piv : nullptr, s_dyn, acc, [&] {
                   __syncthreads();  // s_map
 #pragma unroll
@@ -758,13 +803,14 @@ __global__ void __launch_bounds__(128, 3) k_fc_schur(FcWork w, int begin, int pa
 
 // ---- solve -------------------------------------------------------------------------------------
 
-// The children's share of entry `idx` (pivots, then boundary) of a front's right-hand side.
-__device__ __forceinline__ double from_children(const FcWork& w, const FcFront& F, int idx) {
-    const int v = idx / w.gd, r = idx - v * w.gd;
-    const int k0 = w.maps[F.child[0] >= 0 ? F.map[0] + v : 0], k1 = w.maps[F.child[1] >= 0 ? F.map[1] + v : 0];
-    const bool ok0 = F.child[0] >= 0 && k0 >= 0, ok1 = F.child[1] >= 0 && k1 >= 0;
-    const double x = w.vec[ok0 ? F.child_vec[0] + k0 * w.gd + r : 0], y = w.vec[ok1 ? F.child_vec[1] + k1 * w.gd + r : 0];
-    return (ok0 ? x : 0.0) + (ok1 ? y : 0.0);
+__global__ void k_fc_expand(FcWork w, const int32_t* __restrict__ maps, const int32_t* __restrict__ verts) {
+    const FcFront F = w.fronts[blockIdx.x];
+    for (int e = threadIdx.x; e < F.p + F.b; e += blockDim.x) {
+        const int v = e / w.gd, r = e - v * w.gd;
+        const int k0 = F.child[0] >= 0 ? maps[F.map[0] + v] : -1, k1 = F.child[1] >= 0 ? maps[F.map[1] + v] : -1;
+        w.kids[F.ent + e] = make_int2(k0 >= 0 ? k0 * w.gd + r : -1, k1 >= 0 ? k1 * w.gd + r : -1);
+        w.dofs[F.ent + e] = verts[F.verts + v] * w.gd + r;
+    }
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -773,206 +819,128 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// The passes of a front that one CTA reads alone. Forward: z = x11 v_P, v_B = children - l21 z.
-__global__ void __launch_bounds__(256) k_fc_fwd(FcWork w, const double* __restrict__ in, int begin) {
-    extern __shared__ double s_v[];  // v_P, then z
-    const FcTask tk = w.tasks[begin + blockIdx.x];
-    const FcFront F = w.fronts[tk.front];
-    if (!w.active[F.tissue]) return;
-    double* s_z = s_v + F.p;
-    for (int c = threadIdx.x; c < F.p; c += 256) {
-        const int v = c / w.gd;
-        s_v[c] = in[(size_t)w.verts[F.verts + v] * w.gd + (c - v * w.gd)] + from_children(w, F, c);
-    }
-    __syncthreads();
-    // a row per 8 lanes: the fronts of this kernel have few pivots
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
-    for (int r0 = warp * 4; r0 < F.p; r0 += 32) {
-        const int r = r0 + (lane >> 3);
+// Up: rows [i j, (i + 1) j) of [z; v_B] = [x11; children - w21] v_P, v_P the right-hand side plus the children's
+// vectors. A row is read by 8 lanes (few pivots) or by a warp. Both passes are bound by the bytes in flight:
+// every lane issues eight reads before it uses one.
+template <int LANES>
+__device__ __forceinline__ void up_rows(const FcWork& w, const FcFront& F, const double* s_v, int r0, int r1) {
+    constexpr int PER = 32 / LANES;  // rows of a warp side by side
+    const int lane = threadIdx.x & 31, sub = lane % LANES;
+    const double* X = w.factor + F.x11;  // rows p .. p + b - 1 of the kept factor are w21
+    for (int base = r0 + (threadIdx.x >> 5) * PER; base < r1; base += 8 * PER) {
+        const int r = base + lane / LANES;
+        const bool in = r < r1;
+        const double* A = X + (size_t)(in ? r : r0) * F.ldp;
+        double kid = 0.0;
+        if (sub == 0) {
+            const int2 q = in && r >= F.p ? w.kids[F.ent + r] : make_int2(-1, -1);
+            kid = load_if(w.vec, q.x >= 0, F.child_vec[0] + q.x) + load_if(w.vec, q.y >= 0, F.child_vec[1] + q.y);
+        }
+        const int n = !in ? 0 : (r < F.p ? r + 1 : F.p);
         double s = 0.0;
-        if (r < F.p) {
-            const double* X = w.factor + F.x11 + (size_t)r * F.ldp;
-#pragma unroll 8
-            for (int c = sub; c <= r; c += 8) s += X[c] * s_v[c];
+        for (int c0 = sub; c0 < F.p; c0 += 8 * LANES) {
+            double x[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[u] = load_if(A, c0 + u * LANES < n, c0 + u * LANES);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += x[u] * (c0 + u * LANES < n ? s_v[c0 + u * LANES] : 0.0);
         }
 #pragma unroll
-        for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        if (sub == 0 && r < F.p) s_z[r] = w.z[F.piv + r] = s;
-    }
-    __syncthreads();
-    for (int r0 = warp * 4; r0 < F.b; r0 += 64) {  // two rows per 8 lanes at a time
-        const int r = r0 + (lane >> 3), r2 = r + 32;
-        double s = 0.0, s2 = 0.0, kid = 0.0, kid2 = 0.0;
-        if (sub == 0 && r < F.b) kid = from_children(w, F, F.p + r);
-        if (sub == 0 && r2 < F.b) kid2 = from_children(w, F, F.p + r2);
-        const double* L = w.factor + F.l21 + (size_t)(r < F.b ? r : 0) * F.ldp;
-        const double* L2 = w.factor + F.l21 + (size_t)(r2 < F.b ? r2 : 0) * F.ldp;
-        if (r < F.b)
-#pragma unroll 8
-            for (int c = sub; c < F.p; c += 8) {
-                s += L[c] * s_z[c];
-                s2 += L2[c] * s_z[c];
-            }
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) {
-            s += __shfl_xor_sync(0xffffffffu, s, off);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-        }
-        if (sub == 0 && r < F.b) w.vec[F.vec + r] = kid - s;
-        if (sub == 0 && r2 < F.b) w.vec[F.vec + r2] = kid2 - s2;
+        for (int off = LANES / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (sub == 0 && in) *(r < F.p ? w.z + F.piv + r : w.vec + F.vec + r - F.p) = r < F.p ? s : kid - s;
     }
 }
 
-// Backward: x_P = x11^T (S z - l21^T x_B).
-__global__ void __launch_bounds__(256) k_fc_bwd(FcWork w, double* __restrict__ x, int begin) {
-    extern __shared__ double s_v[];  // x_B, then t (p)
-    __shared__ double s_p[8][64];
+__global__ void __launch_bounds__(256) k_fc_up(FcWork w, const double* __restrict__ in, int begin) {
+    extern __shared__ double s_v[];  // v_P
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
-    double* s_t = s_v + F.b;
-    for (int r = threadIdx.x; r < F.b; r += 256) {
-        const int idx = F.p + r, v = idx / w.gd;
-        s_v[r] = x[(size_t)w.verts[F.verts + v] * w.gd + (idx - v * w.gd)];
+    for (int c0 = threadIdx.x; c0 < F.p; c0 += 4 * 256) {
+        int2 k[4];
+        int d[4];
+        double x[4], y[4], z[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = min(c0 + u * 256, F.p - 1);
+            k[u] = w.kids[F.ent + c];
+            d[u] = w.dofs[F.ent + c];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x[u] = in[d[u]];
+            y[u] = load_if(w.vec, k[u].x >= 0, F.child_vec[0] + k[u].x);
+            z[u] = load_if(w.vec, k[u].y >= 0, F.child_vec[1] + k[u].y);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c0 + u * 256 < F.p) s_v[c0 + u * 256] = x[u] + y[u] + z[u];
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int pass = 0; pass < 2; ++pass) {  // columns of l21, then of x11, 64 at a time
-        for (int c0 = 0; c0 < F.p; c0 += 64) {
-            const int col = c0 + lane, col2 = col + 32;
-            double s = 0.0, s2 = 0.0;
-            if (pass == 0) {
-                const double* L = w.factor + F.l21 + (col < F.p ? col : 0);
-                const double* L2 = w.factor + F.l21 + (col2 < F.p ? col2 : 0);
-#pragma unroll 8
-                for (int r = warp; r < F.b; r += 8) {
-                    s += L[(size_t)r * F.ldp] * s_v[r];
-                    s2 += L2[(size_t)r * F.ldp] * s_v[r];
-                }
-            } else {
-                const double* X = w.factor + F.x11;
-#pragma unroll 8
-                for (int r = c0 + warp; r < F.p; r += 8) {
-                    if (col <= r) s += X[(size_t)r * F.ldp + col] * s_t[r];
-                    if (col2 <= r) s2 += X[(size_t)r * F.ldp + col2] * s_t[r];
-                }
-            }
-            s_p[warp][lane] = s;
-            s_p[warp][lane + 32] = s2;
-            __syncthreads();
-            const int c = c0 + threadIdx.x;
-            if (threadIdx.x < 64 && c < F.p) {
-                double t = 0.0;
+    const int r0 = tk.i * tk.j, r1 = min(r0 + tk.j, F.p + F.b);
+    if (F.p <= 128)
+        up_rows<8>(w, F, s_v, r0, r1);
+    else
+        up_rows<32>(w, F, s_v, r0, r1);
+}
+
+// Down: columns [i j, (i + 1) j) of x_P = [x11; w21]^T [S z; -x_B], a lane per column (two for 64 columns), the
+// warps splitting the rows.
+template <bool TWO>
+__device__ __forceinline__ void down_columns(const double* A, const double* B, int ldp, const double* s_u, int rows, double& sa,
+                                             double& sb) {
+    const int nw = blockDim.x >> 5;
+    for (int r0 = threadIdx.x >> 5; r0 < rows; r0 += 8 * nw) {
+        double x[8], y[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) t += s_p[k][threadIdx.x];
-                if (pass == 0) {
-                    s_t[c] = w.sign[F.piv + c] * w.z[F.piv + c] - t;
-                } else {
-                    const int v = c / w.gd;
-                    x[(size_t)w.verts[F.verts + v] * w.gd + (c - v * w.gd)] = t;
-                }
-            }
-            __syncthreads();
+        for (int u = 0; u < 8; ++u) {
+            const size_t r = (size_t)min(r0 + u * nw, rows - 1) * ldp;
+            x[u] = A[r];
+            if (TWO) y[u] = B[r];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const double v = r0 + u * nw < rows ? s_u[r0 + u * nw] : 0.0;
+            sa += x[u] * v;
+            if (TWO) sb += y[u] * v;
         }
     }
 }
 
-// The larger fronts, each pass in two launches. z = x11 v_P for 16 pivots, v_P the right-hand side plus
-// the children's vectors.
-__global__ void __launch_bounds__(256) k_fc_fwd1(FcWork w, const double* __restrict__ in, int begin) {
-    extern __shared__ double s_v[];
+__global__ void __launch_bounds__(1024) k_fc_down(FcWork w, double* __restrict__ x, int begin) {
+    extern __shared__ double s_u[];  // [S z; -x_B] from row c0 on
+    __shared__ double s_p[32][64];
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
-    const int r1 = min((tk.i + 1) * kFcRows, F.p);
-    for (int c = threadIdx.x; c < r1; c += 256) {
-        const int v = c / w.gd;
-        s_v[c] = in[(size_t)w.verts[F.verts + v] * w.gd + (c - v * w.gd)] + from_children(w, F, c);
+    const int c0 = tk.i * tk.j, n = F.p + F.b, nt = blockDim.x, nw = nt >> 5;
+    for (int r = c0 + threadIdx.x; r < F.p; r += nt) s_u[r - c0] = w.sign[F.piv + r] * w.z[F.piv + r];
+    for (int r = threadIdx.x; r < F.b; r += 4 * nt) {
+        int d[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) d[u] = w.dofs[F.ent + F.p + min(r + u * nt, F.b - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const double v = x[d[u]];
+            if (r + u * nt < F.b) s_u[F.p + r + u * nt - c0] = -v;
+        }
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    for (int r = tk.i * kFcRows + (threadIdx.x >> 5); r < r1; r += 8) {
-        const double* X = w.factor + F.x11 + (size_t)r * F.ldp;
-        double s = 0.0;
-#pragma unroll 8
-        for (int c = lane; c <= r; c += 32) s += X[c] * s_v[c];
-        s = warp_sum(s);
-        if (lane == 0) w.z[F.piv + r] = s;
-    }
-}
-
-// v_B = the children's vectors - l21 z for 16 boundary rows.
-__global__ void __launch_bounds__(256) k_fc_fwd2(FcWork w, int begin) {
-    const FcTask tk = w.tasks[begin + blockIdx.x];
-    const FcFront F = w.fronts[tk.front];
-    if (!w.active[F.tissue]) return;
-    const int r1 = min((tk.i + 1) * kFcRows, F.b), lane = threadIdx.x & 31;
-    const double* z = w.z + F.piv;
-    for (int r = tk.i * kFcRows + (threadIdx.x >> 5); r < r1; r += 8) {
-        const double* L = w.factor + F.l21 + (size_t)r * F.ldp;
-        double s = 0.0;
-#pragma unroll 8
-        for (int c = lane; c < F.p; c += 32) s += L[c] * z[c];
-        s = warp_sum(s);
-        if (lane == 0) w.vec[F.vec + r] = from_children(w, F, F.p + r) - s;
-    }
-}
-
-// Partial sums of l21^T x_B: 128 boundary rows (task i) x 64 pivots (task j).
-__global__ void __launch_bounds__(256) k_fc_bwd1(FcWork w, const double* __restrict__ x, int begin) {
-    __shared__ double s_x[kFcBackRows];
-    __shared__ double s_p[4][kT];
-    const FcTask tk = w.tasks[begin + blockIdx.x];
-    const FcFront F = w.fronts[tk.front];
-    if (!w.active[F.tissue]) return;
-    const int r0 = tk.i * kFcBackRows, n = min(kFcBackRows, F.b - r0);
-    for (int r = threadIdx.x; r < n; r += 256) {
-        const int idx = F.p + r0 + r, v = idx / w.gd;
-        s_x[r] = x[(size_t)w.verts[F.verts + v] * w.gd + (idx - v * w.gd)];
-    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ca = min(c0 + lane, F.p - 1), cb = min(ca + 32, F.p - 1);
+    // x11 is lower triangular, and zero above its diagonal within the 64 x 64 diagonal blocks
+    const double* X = w.factor + F.x11 + (size_t)c0 * F.ldp;
+    double sa = 0.0, sb = 0.0;
+    if (tk.j == 64)
+        down_columns<true>(X + ca, X + cb, F.ldp, s_u, n - c0, sa, sb);
+    else
+        down_columns<false>(X + ca, X + cb, F.ldp, s_u, n - c0, sa, sb);
+    s_p[warp][lane] = sa;
+    s_p[warp][lane + 32] = sb;
     __syncthreads();
-    const int c = threadIdx.x & 63, part = threadIdx.x >> 6, col = tk.j * kT + c;
-    double s = 0.0;
-    if (col < F.p) {
-        const double* L = w.factor + F.l21 + (size_t)r0 * F.ldp + col;
-#pragma unroll 8
-        for (int r = part; r < n; r += 4) s += L[(size_t)r * F.ldp] * s_x[r];
-    }
-    s_p[part][c] = s;
-    __syncthreads();
-    if (part == 0 && col < F.p) w.tp[F.tp + (size_t)tk.i * F.ldp + col] = s_p[0][c] + s_p[1][c] + s_p[2][c] + s_p[3][c];
-}
-
-// x_P = x11^T (S z - l21^T x_B) for 32 pivots.
-__global__ void __launch_bounds__(512) k_fc_bwd2(FcWork w, double* __restrict__ x, int begin) {
-    extern __shared__ double s_v[];
-    __shared__ double s_p[16][33];
-    const FcTask tk = w.tasks[begin + blockIdx.x];
-    const FcFront F = w.fronts[tk.front];
-    if (!w.active[F.tissue]) return;
-    const int c0 = tk.i * 32, chunks = (F.b + kFcBackRows - 1) / kFcBackRows;
-    for (int c = c0 + threadIdx.x; c < F.p; c += 512) {
-        double t = w.sign[F.piv + c] * w.z[F.piv + c];
-        for (int k = 0; k < chunks; ++k) t -= w.tp[F.tp + (size_t)k * F.ldp + c];
-        s_v[c - c0] = t;
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = c0 + lane;
-    double s = 0.0;
-    if (col < F.p) {
-        const double* X = w.factor + F.x11 + col;
-#pragma unroll 8
-        for (int r = c0 + warp; r < F.p; r += 16)
-            if (r >= col) s += X[(size_t)r * F.ldp] * s_v[r - c0];
-    }
-    s_p[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0 && col < F.p) {
+    if ((int)threadIdx.x < tk.j && c0 + (int)threadIdx.x < F.p) {
         double t = 0.0;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) t += s_p[k][lane];
-        const int v = col / w.gd;
-        x[(size_t)w.verts[F.verts + v] * w.gd + (col - v * w.gd)] = t;
+        for (int k = 0; k < nw; ++k) t += s_p[k][threadIdx.x];
+        x[w.dofs[F.ent + c0 + threadIdx.x]] = t;
     }
 }
 
@@ -1218,52 +1186,28 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
     return cudaGetLastError();
 }
 
-// Shared memory of the one-CTA passes: two vectors of the pivots (forward), boundary and pivots (back).
-static size_t solve_smem(const FcPlan& plan, const FcRange& r, bool forward) {
-    int n = 0;
-    for (int k = 0; k < r.count; ++k) {
-        const FcFront& F = plan.fronts[plan.tasks[r.begin + k].front];
-        const int m = forward ? 2 * F.p : F.p + F.b;
-        n = n < m ? m : n;
-    }
-    return sizeof(double) * (size_t)n;
+cudaError_t launch_factor_expand(const FcPlan& plan, const FcWork& w, const int32_t* maps, const int32_t* verts,
+                                 cudaStream_t s) {
+    k_fc_expand<<<(unsigned)plan.fronts.size(), 128, 0, s>>>(w, maps, verts);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
                                 cudaStream_t s) {
+    FC_CK(opt_in((const void*)k_fc_down, kFcMaxFront * (int)sizeof(double)));
     int64_t n = 0;
     const int depths = (int)plan.depths.size();
     for (int d = depths - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
-        if (L.solve.count) {
-            k_fc_fwd<<<L.solve.count, 256, solve_smem(plan, L.solve, true), s>>>(w, in, L.solve.begin);
-            ++n;
-        }
-        if (L.fwd1.count) {
-            const int pmax = plan.fronts[plan.tasks[L.fwd1.begin].front].p;
-            k_fc_fwd1<<<L.fwd1.count, 256, pmax * sizeof(double), s>>>(w, in, L.fwd1.begin);
-            ++n;
-        }
-        if (L.fwd2.count) {
-            k_fc_fwd2<<<L.fwd2.count, 256, 0, s>>>(w, L.fwd2.begin);
-            ++n;
-        }
+        if (!L.fwd.count) continue;
+        k_fc_up<<<L.fwd.count, 256, L.fwd_smem, s>>>(w, in, L.fwd.begin);
+        ++n;
     }
     for (int d = 0; d < depths; ++d) {
         const FcDepth& L = plan.depths[d];
-        if (L.solve.count) {
-            k_fc_bwd<<<L.solve.count, 256, solve_smem(plan, L.solve, false), s>>>(w, x, L.solve.begin);
-            ++n;
-        }
-        if (L.bwd1.count) {
-            k_fc_bwd1<<<L.bwd1.count, 256, 0, s>>>(w, x, L.bwd1.begin);
-            ++n;
-        }
-        if (L.bwd2.count) {
-            const int pmax = plan.fronts[plan.tasks[L.bwd2.begin].front].p;
-            k_fc_bwd2<<<L.bwd2.count, 512, pmax * sizeof(double), s>>>(w, x, L.bwd2.begin);
-            ++n;
-        }
+        if (!L.bwd.count) continue;
+        k_fc_down<<<L.bwd.count, L.bwd_threads, L.bwd_smem, s>>>(w, x, L.bwd.begin);
+        ++n;
     }
     *launches += n;
     return cudaGetLastError();

@@ -9,9 +9,11 @@
 // of the tree are processed together, the deepest first.
 //
 // With the front's matrix [A11 A21^T; A21 A22], A11 = G S G^T (G lower triangular, S = diag(+-1)):
-//   x11 = G^-1 (p x p, lower), l21 = A21 G^-T S (b x p), contribution C = A22 - l21 S l21^T.
-// A solve is then one pass up the tree, z = x11 v_P, v_B -= l21 z, and one down,
-// x_P = x11^T (S z - l21^T x_B): matrix-vector products only, no triangular solves.
+//   x11 = G^-1 (p x p, lower), l21 = A21 G^-T S (b x p), contribution C = A22 - l21 S l21^T,
+//   w21 = l21 x11 = A21 A11^-1 (b x p), kept in l21's place.
+// A solve is then one pass up the tree, z = x11 v_P and v_B -= w21 v_P, and one down,
+// x_P = x11^T S z - w21^T x_B: matrix-vector products whose rows (columns) do not wait for each other,
+// one launch per depth and pass.
 #pragma once
 
 #include <vector>
@@ -23,10 +25,9 @@ namespace tfb {
 constexpr int kFcTile = 64;        // pivot panel width and GEMM tile
 constexpr int kFcScatter = 256;    // Jacobian blocks per assembly task
 constexpr int kFcSmallB = 288;     // boundary unknowns up to which a one-panel front is one CTA's
-constexpr int kFcSmallSolve = 49152; // entries of x11 and l21 up to which a front's solve is one CTA's
-constexpr int kFcRows = 16;        // front rows per solve task
-constexpr int kFcBackRows = 128;   // boundary rows per backward task
-constexpr int kFcMaxPivots = 5000; // pivots of one front (the solve stages them in shared memory)
+constexpr int kFcRowEntries = 8192; // entries of [x11; w21] per task of the upward pass
+constexpr int kFcMaxPivots = 5000; // pivots of one front, and unknowns of one front: the passes stage
+constexpr int kFcMaxFront = 24000; // vectors of them in shared memory
 
 struct FcFront {
     int32_t p, b;          // pivot and boundary unknowns
@@ -37,12 +38,12 @@ struct FcFront {
     int32_t map[2];        // offsets into maps: per column of this front, its index on the child's boundary
     int32_t verts;         // offset into verts: the pivots' columns, then the boundary's
     int32_t j0, j1;        // its Jacobian blocks in jblk
+    int32_t ent;           // offset of its p + b entries in kids / dofs
     int32_t vec, piv;      // offsets of the boundary vector (b) and of z / the signs (p)
-    int64_t x11, l21;      // kept factors
-    int64_t a21, lp;       // scratch of the front's depth: A21, and the current panel of L11 (p x 64)
+    int64_t x11, w21;      // kept factors
+    int64_t a21, l21, lp;  // scratch of the front's depth: A21, l21 and the current panel of L11 (p x 64)
     int64_t c;             // contribution (b x b, lower), in the scratch of the depth's parity
     int64_t child_c[2];
-    int64_t tp;            // scratch of the backward pass: partial sums per boundary chunk (chunks x p)
 };
 
 struct FcTask {
@@ -70,7 +71,8 @@ struct FcPanel {
 
 struct FcDepth {
     FcRange small[3], gather, scatter, diag, l21, schur;  // small: fronts factorised by one CTA each, by size
-    FcRange solve, fwd1, fwd2, bwd1, bwd2;             // solve: fronts whose passes are one CTA's each
+    FcRange fwd, bwd;  // tasks (i, j): rows [i j, (i + 1) j); columns [i j, (i + 1) j)
+    int32_t fwd_smem = 0, bwd_smem = 0, bwd_threads = 256;  // bytes; threads of a downward CTA
     int32_t panel0 = 0, n_panel = 0;
 };
 
@@ -84,8 +86,8 @@ struct FcPlan {
     std::vector<FcTask> tasks;
     std::vector<FcDepth> depths;  // 0: the roots
     std::vector<FcPanel> panels;
-    int64_t n_factor = 0, n_scratch = 0, n_contrib[2] = {0, 0}, n_tp = 0;  // doubles
-    int64_t n_vec = 0, n_piv = 0;
+    int64_t n_factor = 0, n_scratch = 0, n_contrib[2] = {0, 0};  // doubles
+    int64_t n_vec = 0, n_piv = 0, n_ent = 0;
     int64_t n_root = 0;   // pivots of the root fronts
     double flops = 0.0;   // multiplications and additions of one factorisation
     int chain = 0;        // dependent 64-pivot panels over the depths
@@ -103,8 +105,8 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
 struct FcWork {
     int gd;
     const FcFront* fronts;
-    const int32_t* maps;
-    const int32_t* verts;
+    int2* kids;     // [n_ent] every entry's index on the boundary of either child, or -1
+    int32_t* dofs;  // [n_ent] every entry's unknown
     const int2* jblk;
     const int32_t* jblk_t;  // NULL: J is symmetric
     const FcTask* tasks;
@@ -112,7 +114,6 @@ struct FcWork {
     double* factor;
     double* scratch;
     double* contrib[2];
-    double* tp;
     double* vec;
     double* z;
     double* sign;    // [n_piv] +1 / -1
@@ -120,6 +121,9 @@ struct FcWork {
     int32_t* neg;    // [fronts] 1: the front has negative pivots
 };
 
+// kids and dofs of every front from the plan's columns (maps, verts on the device)
+cudaError_t launch_factor_expand(const FcPlan& plan, const FcWork& w, const int32_t* maps, const int32_t* verts,
+                                 cudaStream_t s);
 // Numeric factorisation of J (vals: the full BSR3 values; block (row, column) is read from the row of
 // the earlier pivot, transposed). Returns the kernels launched in *launches.
 cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, cudaStream_t s);

@@ -190,6 +190,9 @@ struct Dissection {
     }
 };
 
+// Fronts that one CTA factorises in shared memory.
+bool one_cta(const FcFront& F) { return F.p > 0 && F.p <= kFcTile && F.b <= kFcSmallB; }
+
 template <class F>
 void parallel_items(int n, F f) {
     const int nt = std::min<int>(n, (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
@@ -257,7 +260,7 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             at[f.depth].push_back({t, k});
             const double p = (double)f.piv.size() * gd, b = (double)f.bnd.size() * gd;
             flops += p * p * p * (2.0 / 3.0) + p * p * b + b * b * p;
-            if (p > kFcMaxPivots || p + b >= 65536) return;
+            if (p > kFcMaxPivots || p + b > kFcMaxFront) return;
         }
     plan.flops = flops;
     if (flops > max_flops) return;
@@ -271,7 +274,7 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
     std::vector<std::pair<int, int>> of(nf);
     int64_t n_map = 0, n_vert = 0;
     for (int d = 0; d < depths; ++d) {
-        int64_t scratch = 0, contrib = 0, tp = 0;
+        int64_t scratch = 0, contrib = 0;
         for (auto& q : at[d]) {
             const int fi = id[q.first][q.second];
             of[fi] = q;
@@ -294,21 +297,25 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             F.piv = (int32_t)plan.n_piv;
             plan.n_vec += F.b;
             plan.n_piv += F.ldp;
+            F.ent = (int32_t)plan.n_ent;
+            plan.n_ent += F.p + F.b;
             F.x11 = plan.n_factor;
-            F.l21 = F.x11 + (int64_t)F.p * F.ldp;
-            plan.n_factor = F.l21 + (int64_t)F.b * F.ldp;
-            F.a21 = scratch;
-            F.lp = F.a21 + (int64_t)F.b * F.ldp;  // a21, lp: not used by the fronts of one CTA
-            scratch = F.lp + (F.p > kFcTile ? (int64_t)F.p * kFcTile : 0);
+            F.w21 = F.x11 + (int64_t)F.p * F.ldp;
+            plan.n_factor = F.w21 + (int64_t)F.b * F.ldp;
+            if (one_cta(F)) {  // these live in shared memory
+                F.a21 = F.l21 = F.lp = scratch;
+            } else {
+                F.a21 = scratch;
+                F.l21 = F.a21 + (int64_t)F.b * F.ldp;
+                F.lp = F.l21 + (int64_t)F.b * F.ldp;
+                scratch = F.lp + (F.p > kFcTile ? (int64_t)F.p * kFcTile : 0);
+            }
             F.c = contrib;
             contrib += (int64_t)F.b * F.ldb;
-            F.tp = tp;
-            tp += (int64_t)((F.b + kFcBackRows - 1) / kFcBackRows) * F.ldp;
             if (d == 0) plan.n_root += F.p;
         }
         plan.n_scratch = std::max(plan.n_scratch, scratch);
         plan.n_contrib[d & 1] = std::max(plan.n_contrib[d & 1], contrib);
-        plan.n_tp = std::max(plan.n_tp, tp);
     }
     for (FcFront& F : plan.fronts)
         for (int k = 0; k < 2; ++k) {
@@ -317,7 +324,7 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             F.child_vec[k] = c ? c->vec : 0;
             F.child_c[k] = c ? c->c : 0;
         }
-    if (n_map > INT32_MAX || n_vert > INT32_MAX || plan.n_vec > INT32_MAX || plan.n_piv > INT32_MAX) return;
+    if (n_map > INT32_MAX || n_vert > INT32_MAX || plan.n_ent > INT32_MAX || plan.n_vec > INT32_MAX || plan.n_piv > INT32_MAX) return;
     plan.maps.resize(n_map);
     plan.verts.resize(n_vert);
     // columns, child maps and Jacobian blocks of every front
@@ -396,18 +403,16 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             r.count = (int32_t)plan.tasks.size() - r.begin;
         };
         auto push = [&](int32_t f, int i, int j) { plan.tasks.push_back(FcTask{f, (int16_t)i, (int16_t)j}); };
-        auto is_small = [](const FcFront& F) { return F.p > 0 && F.p <= kFcTile && F.b <= kFcSmallB; };
-        auto one_cta = [](const FcFront& F) { return (int64_t)F.p * (F.p + F.b) <= kFcSmallSolve; };
         std::vector<int32_t> all = fs, rest;
         for (int32_t fi : fs)
-            if (!is_small(plan.fronts[fi])) rest.push_back(fi);
+            if (!one_cta(plan.fronts[fi])) rest.push_back(fi);
         std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) { return plan.fronts[a].b > plan.fronts[b].b; });
         // in three launches by the shared memory they need, so that two and three small ones share an SM
         // (228 KB, 10 KB of it static per CTA)
         const int bound[4] = {INT32_MAX, 102000, 64000, 0};
         for (int c = 0; c < 3; ++c)
             list(L.small[c], [&](int32_t fi, const FcFront& F) {
-                if (!is_small(F)) return;
+                if (!one_cta(F)) return;
                 const int bytes = fc_small_smem(F.p, F.b);
                 if (bytes <= bound[c] && bytes > bound[c + 1]) push(fi, 0, 0);
             });
@@ -453,31 +458,28 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
                 for (int j = cdiv(F.p, kFcTile) - 1; j >= 0; --j) push(fi, i, j);
         });
         list(L.schur, [&](int32_t fi, const FcFront& F) {
+            // with them, from the same l21, the tiles of w21 (j < 0: column tile -1 - j)
+            for (int j = 0; j < cdiv(F.p, kFcTile); ++j)
+                for (int i = 0; i < cdiv(F.b, kFcTile); ++i) push(fi, i, -1 - j);
             for (int i = 0; i < cdiv(F.b, kFcTile); ++i)
                 for (int j = 0; j <= i; ++j) push(fi, i, j);
         });
-        fs.clear();
-        for (int32_t fi : all)
-            if (one_cta(plan.fronts[fi])) fs.push_back(fi);
+        fs = all;
         std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) {
             return (int64_t)plan.fronts[a].p * plan.fronts[a].b > (int64_t)plan.fronts[b].p * plan.fronts[b].b;
         });
-        list(L.solve, [&](int32_t fi, const FcFront&) { push(fi, 0, 0); });
-        fs.clear();
-        for (int32_t fi : all)
-            if (!one_cta(plan.fronts[fi])) fs.push_back(fi);
-        list(L.fwd1, [&](int32_t fi, const FcFront& F) {
-            for (int i = cdiv(F.p, kFcRows) - 1; i >= 0; --i) push(fi, i, 0);
+        // up: rows of [x11; w21] by entries; down: 64 columns, or 32 and more threads where there are many rows
+        list(L.fwd, [&](int32_t fi, const FcFront& F) {
+            const int n = F.p + F.b, rows = F.p > 128 ? std::max(8, kFcRowEntries / F.p / 8 * 8)
+                                                     : std::max(32, kFcRowEntries / std::max(F.p, 1) / 32 * 32);
+            for (int i = 0; i < cdiv(n, rows); ++i) push(fi, i, std::min(rows, 32736));
+            L.fwd_smem = std::max(L.fwd_smem, (int32_t)(F.p * sizeof(double)));
         });
-        list(L.fwd2, [&](int32_t fi, const FcFront& F) {
-            for (int i = 0; i < cdiv(F.b, kFcRows); ++i) push(fi, i, 0);
-        });
-        list(L.bwd1, [&](int32_t fi, const FcFront& F) {
-            for (int i = 0; i < cdiv(F.b, kFcBackRows); ++i)
-                for (int j = 0; j < cdiv(F.p, kFcTile); ++j) push(fi, i, j);
-        });
-        list(L.bwd2, [&](int32_t fi, const FcFront& F) {
-            for (int i = 0; i < cdiv(F.p, 32); ++i) push(fi, i, 0);
+        list(L.bwd, [&](int32_t fi, const FcFront& F) {
+            const int cols = F.p > 256 ? 32 : 64;
+            for (int i = 0; i < cdiv(F.p, cols); ++i) push(fi, i, cols);
+            L.bwd_smem = std::max(L.bwd_smem, (int32_t)((F.p + F.b) * sizeof(double)));
+            if (F.p + F.b > 300) L.bwd_threads = std::max(L.bwd_threads, F.p + F.b > 700 ? 1024 : 512);
         });
     }
     if (plan.tasks.size() > (size_t)INT32_MAX) return;
