@@ -1761,7 +1761,7 @@ int build_factor(tf_ctx* ctx) {
         if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(b.p, h, bytes, cudaMemcpyHostToDevice, ctx->stream);
         return e;
     };
-    cudaError_t e = room(ctx->fc_factor, P.n_factor);
+    cudaError_t e = room(ctx->fc_factor, P.n_factor + 64);  // the downward pass reads past the last row's columns
     if (e == cudaSuccess) e = room(ctx->fc_scratch, P.n_scratch);
     for (int q = 0; q < 2; ++q)
         if (e == cudaSuccess) e = room(ctx->fc_contrib[q], P.n_contrib[q]);
@@ -1775,6 +1775,8 @@ int build_factor(tf_ctx* ctx) {
         return TF_OK;
     }
     TF_CK(e);
+    // the padding of the rows, and x11 above its diagonal blocks, stay zero: no kernel writes there
+    TF_CK(cudaMemsetAsync(ctx->fc_factor.p, 0, sizeof(double) * (size_t)(P.n_factor + 64), ctx->stream));
     TF_CK(dalloc(ctx->fc_flags, sizeof(int32_t) * T));
     TF_CK(dalloc(ctx->fc_neg, sizeof(int32_t) * P.fronts.size()));
     TF_CK(dalloc(ctx->fc_running, sizeof(int32_t) * T));

@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(256) k_fc_scatter(FcWork w, const double* __re
         const int k = e / 9, en = e - k * 9, cc = en / 3, rr = en - cc * 3;
         const int2 jb = w.jblk[b0 + k];
         const int row = (int)((uint32_t)jb.y >> 16) + rr, col = (jb.y & 0xffff) + cc;
+        if (col > row) continue;  // the upper half of a node's own block
         double* out = row < F.p ? w.factor + F.x11 + (size_t)row * F.ldp + col
                                 : w.scratch + F.a21 + (size_t)(row - F.p) * F.ldp + col;
         *out += j_entry(w, vals, b0 + k, jb.x, cc, rr);
@@ -820,31 +821,50 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Up: rows [i j, (i + 1) j) of [z; v_B] = [x11; children - w21] v_P, v_P the right-hand side plus the children's
-// vectors. A row is read by 8 lanes (few pivots) or by a warp. Both passes are bound by the bytes in flight:
-// every lane issues eight reads before it uses one.
+// vectors. A row is read by 8 lanes (few pivots) or by a warp, two entries at a time, four such reads in
+// flight: one entry at a time both passes were bound by their instructions (58 % issue slots busy).
+// Rows are zero from the diagonal to the end of its 64-column block, and in the padding to ldp.
 template <int LANES>
-__device__ __forceinline__ void up_rows(const FcWork& w, const FcFront& F, const double* s_v, int r0, int r1) {
+__device__ __forceinline__ void up_rows(const FcWork& w, const FcFront& F, const double2* s_v, int r0, int r1) {
     constexpr int PER = 32 / LANES;  // rows of a warp side by side
     const int lane = threadIdx.x & 31, sub = lane % LANES;
     const double* X = w.factor + F.x11;  // rows p .. p + b - 1 of the kept factor are w21
     for (int base = r0 + (threadIdx.x >> 5) * PER; base < r1; base += 8 * PER) {
         const int r = base + lane / LANES;
         const bool in = r < r1;
-        const double* A = X + (size_t)(in ? r : r0) * F.ldp;
+        const double2* A = reinterpret_cast<const double2*>(X + (size_t)(in ? r : r0) * F.ldp);
         double kid = 0.0;
         if (sub == 0) {
             const int2 q = in && r >= F.p ? w.kids[F.ent + r] : make_int2(-1, -1);
             kid = load_if(w.vec, q.x >= 0, F.child_vec[0] + q.x) + load_if(w.vec, q.y >= 0, F.child_vec[1] + q.y);
         }
-        const int n = !in ? 0 : (r < F.p ? r + 1 : F.p);
-        double s = 0.0;
-        for (int c0 = sub; c0 < F.p; c0 += 8 * LANES) {
-            double x[8];
+        const int n = !in ? 0 : (r < F.p ? min(F.ldp, (r | (kT - 1)) + 1) : F.ldp) >> 1;
+        double s = 0.0, s2 = 0.0;
+        int c = sub;
+        for (; c + 3 * LANES < n; c += 4 * LANES) {
+            double2 x[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) x[u] = load_if(A, c0 + u * LANES < n, c0 + u * LANES);
+            for (int u = 0; u < 4; ++u) x[u] = A[c + u * LANES];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) s += x[u] * (c0 + u * LANES < n ? s_v[c0 + u * LANES] : 0.0);
+            for (int u = 0; u < 4; ++u) {
+                const double2 v = s_v[c + u * LANES];
+                s += x[u].x * v.x;
+                s2 += x[u].y * v.y;
+            }
         }
+        if (c < n) {
+            double2 x[3];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) x[u] = A[min(c + u * LANES, n - 1)];
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+                if (c + u * LANES < n) {
+                    const double2 v = s_v[c + u * LANES];
+                    s += x[u].x * v.x;
+                    s2 += x[u].y * v.y;
+                }
+        }
+        s += s2;
 #pragma unroll
         for (int off = LANES / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
         if (sub == 0 && in) *(r < F.p ? w.z + F.piv + r : w.vec + F.vec + r - F.p) = r < F.p ? s : kid - s;
@@ -852,7 +872,8 @@ __device__ __forceinline__ void up_rows(const FcWork& w, const FcFront& F, const
 }
 
 __global__ void __launch_bounds__(256) k_fc_up(FcWork w, const double* __restrict__ in, int begin) {
-    extern __shared__ double s_v[];  // v_P
+    extern __shared__ __align__(16) double s_vec[];  // v_P, padded with zero
+    double* s_v = s_vec;
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
@@ -876,44 +897,60 @@ __global__ void __launch_bounds__(256) k_fc_up(FcWork w, const double* __restric
         for (int u = 0; u < 4; ++u)
             if (c0 + u * 256 < F.p) s_v[c0 + u * 256] = x[u] + y[u] + z[u];
     }
+    if (threadIdx.x == 0 && (F.p & 1)) s_v[F.p] = 0.0;
     __syncthreads();
     const int r0 = tk.i * tk.j, r1 = min(r0 + tk.j, F.p + F.b);
     if (F.p <= 128)
-        up_rows<8>(w, F, s_v, r0, r1);
+        up_rows<8>(w, F, reinterpret_cast<const double2*>(s_v), r0, r1);
     else
-        up_rows<32>(w, F, s_v, r0, r1);
+        up_rows<32>(w, F, reinterpret_cast<const double2*>(s_v), r0, r1);
 }
 
-// Down: columns [i j, (i + 1) j) of x_P = [x11; w21]^T [S z; -x_B], a lane per column (two for 64 columns), the
-// warps splitting the rows.
-template <bool TWO>
-__device__ __forceinline__ void down_columns(const double* A, const double* B, int ldp, const double* s_u, int rows, double& sa,
-                                             double& sb) {
-    const int nw = blockDim.x >> 5;
-    for (int r0 = threadIdx.x >> 5; r0 < rows; r0 += 8 * nw) {
-        double x[8], y[8];
+// Down: columns [i j, (i + 1) j) of x_P = [x11; w21]^T [S z; -x_B], j = 64 or 32: two columns a lane, one or two
+// rows a warp at a time, the warps splitting the rows.
+template <int COLS>
+__device__ __forceinline__ void down_columns(const double* X, int ldp, const double* s_u, int rows, double* s_p) {
+    constexpr int PER = 64 / COLS;  // rows of a warp side by side
+    const int lane = threadIdx.x & 31, col = 2 * (lane % (COLS / 2)), group = (threadIdx.x >> 5) * PER + lane / (COLS / 2);
+    const int step = (blockDim.x >> 5) * PER;
+    const double* A = X + col + (size_t)group * ldp;
+    const size_t hop = (size_t)step * ldp;
+    double sa = 0.0, sb = 0.0;
+    int r = group;
+    for (; r + 3 * step < rows; r += 4 * step, A += 4 * hop) {
+        double2 x[4];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const size_t r = (size_t)min(r0 + u * nw, rows - 1) * ldp;
-            x[u] = A[r];
-            if (TWO) y[u] = B[r];
-        }
+        for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const double2*>(A + u * hop);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const double v = r0 + u * nw < rows ? s_u[r0 + u * nw] : 0.0;
-            sa += x[u] * v;
-            if (TWO) sb += y[u] * v;
+        for (int u = 0; u < 4; ++u) {
+            const double v = s_u[r + u * step];
+            sa += x[u].x * v;
+            sb += x[u].y * v;
         }
     }
+    if (r < rows) {
+        double2 x[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) x[u] = *reinterpret_cast<const double2*>(r + u * step < rows ? A + u * hop : A);
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (r + u * step < rows) {
+                const double v = s_u[r + u * step];
+                sa += x[u].x * v;
+                sb += x[u].y * v;
+            }
+    }
+    *reinterpret_cast<double2*>(s_p + group * COLS + col) = make_double2(sa, sb);
 }
 
 __global__ void __launch_bounds__(1024) k_fc_down(FcWork w, double* __restrict__ x, int begin) {
     extern __shared__ double s_u[];  // [S z; -x_B] from row c0 on
-    __shared__ double s_p[32][64];
+    __shared__ __align__(16) double s_p[32 * 64];
+    __shared__ double s_q[4][64];
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
     if (!w.active[F.tissue]) return;
-    const int c0 = tk.i * tk.j, n = F.p + F.b, nt = blockDim.x, nw = nt >> 5;
+    const int cols = tk.j, c0 = tk.i * cols, n = F.p + F.b, nt = blockDim.x;
     for (int r = c0 + threadIdx.x; r < F.p; r += nt) s_u[r - c0] = w.sign[F.piv + r] * w.z[F.piv + r];
     for (int r = threadIdx.x; r < F.b; r += 4 * nt) {
         int d[4];
@@ -926,22 +963,22 @@ __global__ void __launch_bounds__(1024) k_fc_down(FcWork w, double* __restrict__
         }
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ca = min(c0 + lane, F.p - 1), cb = min(ca + 32, F.p - 1);
-    // x11 is lower triangular, and zero above its diagonal within the 64 x 64 diagonal blocks
-    const double* X = w.factor + F.x11 + (size_t)c0 * F.ldp;
-    double sa = 0.0, sb = 0.0;
-    if (tk.j == 64)
-        down_columns<true>(X + ca, X + cb, F.ldp, s_u, n - c0, sa, sb);
+    // x11 is lower triangular, and zero above its diagonal within the 64 x 64 diagonal blocks; columns past the
+    // last one read the next rows' entries (the last row's: the padding behind the factors) and are dropped
+    const double* X = w.factor + F.x11 + (size_t)c0 * F.ldp + c0;
+    if (cols == 64)
+        down_columns<64>(X, F.ldp, s_u, n - c0, s_p);
     else
-        down_columns<false>(X + ca, X + cb, F.ldp, s_u, n - c0, sa, sb);
-    s_p[warp][lane] = sa;
-    s_p[warp][lane + 32] = sb;
+        down_columns<32>(X, F.ldp, s_u, n - c0, s_p);
     __syncthreads();
-    if ((int)threadIdx.x < tk.j && c0 + (int)threadIdx.x < F.p) {
+    const int groups = nt / cols * 2, c = threadIdx.x % cols, part = threadIdx.x / cols;
+    if (part < 4) {
         double t = 0.0;
-        for (int k = 0; k < nw; ++k) t += s_p[k][threadIdx.x];
-        x[w.dofs[F.ent + c0 + threadIdx.x]] = t;
+        for (int k = part; k < groups; k += 4) t += s_p[k * cols + c];
+        s_q[part][c] = t;
     }
+    __syncthreads();
+    if (part == 0 && c0 + c < F.p) x[w.dofs[F.ent + c0 + c]] = s_q[0][c] + s_q[1][c] + s_q[2][c] + s_q[3][c];
 }
 
 // ---- conjugate gradients ------------------------------------------------------------------------

@@ -473,7 +473,7 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             const int n = F.p + F.b, rows = F.p > 128 ? std::max(8, kFcRowEntries / F.p / 8 * 8)
                                                      : std::max(32, kFcRowEntries / std::max(F.p, 1) / 32 * 32);
             for (int i = 0; i < cdiv(n, rows); ++i) push(fi, i, std::min(rows, 32736));
-            L.fwd_smem = std::max(L.fwd_smem, (int32_t)(F.p * sizeof(double)));
+            L.fwd_smem = std::max(L.fwd_smem, (int32_t)(F.ldp * sizeof(double)));
         });
         list(L.bwd, [&](int32_t fi, const FcFront& F) {
             const int cols = F.p > 256 ? 32 : 64;
