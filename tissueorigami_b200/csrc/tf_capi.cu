@@ -41,7 +41,10 @@ constexpr int kFcMaxIters = 8;       // iterations after which a factorised solv
 constexpr double kFcKeepFlops = 5e7; // factorisations from this size on are kept from the second Newton iteration
                                      // (342 prisms, 1e7: 1.18 ms a step anew, 1.54 kept; 2,713 prisms,
                                      // 2e8: 4.6 and 3.9; 79,650 prisms, 4.3e10: 26.5 and 19.6)
-constexpr double kFcMaxFlops = 4e11; // largest factorisation (operations of one tissue, or mean of a batch)
+// Largest factorisation (operations of one tissue, or the mean of a batch). ms a step, factorised and
+// conjugate gradients: slab of 86,400 nodes 24.9 and 81, 125,000 nodes (1.6e11) 38.7 and 47, 174,000 nodes
+// (2.7e11) 53 and 58; wing disc of 135,651 nodes 36.6 and 139.
+constexpr double kFcMaxFlops = 3e11;
 
 struct DevBuf {
     void* p = nullptr;
@@ -1750,9 +1753,10 @@ int build_factor(tf_ctx* ctx) {
     if (!P.ok) return TF_OK;
     std::vector<FcChunk> chunks;
     ctx->fc_chunk0.assign(1, 0);
+    const int rows = fc_chunk_rows(N);
     for (int t = 0; t < T; ++t) {
-        for (int r = ctx->tissue_node0[t]; r < ctx->tissue_node0[t + 1]; r += kFcChunkRows)
-            chunks.push_back({t, r, std::min(r + kFcChunkRows, ctx->tissue_node0[t + 1])});
+        for (int r = ctx->tissue_node0[t]; r < ctx->tissue_node0[t + 1]; r += rows)
+            chunks.push_back({t, r, std::min(r + rows, ctx->tissue_node0[t + 1])});
         ctx->fc_chunk0.push_back((int32_t)chunks.size());
     }
     auto room = [&](DevBuf& b, int64_t doubles) { return dalloc(b, sizeof(double) * (size_t)std::max<int64_t>(doubles, 2)); };

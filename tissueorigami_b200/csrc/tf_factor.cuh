@@ -138,7 +138,12 @@ cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const doubl
 struct FcChunk {
     int32_t tissue, row0, row1;
 };
-constexpr int kFcChunkRows = 256;
+// Rows of a chunk: two chunks per SM, between 32 (one pass of a CTA's 8-lane rows) and 256 (few partial sums).
+inline int fc_chunk_rows(int n_nodes) {
+    const int r = (n_nodes / 296 + 31) / 32 * 32;
+    return r < 32 ? 32 : (r > 256 ? 256 : r);
+}
+
 struct FcCg {
     int n_chunks, T;
     const FcChunk* chunks;
