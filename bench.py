@@ -257,7 +257,7 @@ def run_b200(args) -> None:
     if args.profile_region:
         torch.cuda.cudart().cudaProfilerStart()
     ms, iters, kry, launches, worst = 0.0, 0, 0, 0, 0
-    solve_ms, solve_launches, kry_cg, methods = 0.0, 0, 0, set()
+    solve_ms, all_solve_ms, solve_launches, kry_cg, methods = 0.0, 0.0, 0, 0, set()
     for _ in range(args.steps):
         flush.zero_()  # L2 flush between timed steps (outside the step's event window)
         torch.cuda.synchronize()
@@ -267,6 +267,7 @@ def run_b200(args) -> None:
         kry += st.krylov_iters_total
         launches += st.gpu_launches
         solve_ms += st.ms_solve_kernel
+        all_solve_ms += st.ms_solve
         solve_launches += st.solve_launches
         kry_cg += st.krylov_iters_cg
         methods.add(int(st.krylov_method))
@@ -311,14 +312,16 @@ def run_b200(args) -> None:
     else:
         direct = {"skipped": f"{nnz_scalar} scalar non-zeros: beyond a single cusolverSp factorisation",
                   "note": "cuDSS is unavailable on this box (not in the image)"}
-    direct["krylov_ms_per_solve"] = solve_ms / max(solve_launches, 1)
+    # a factorised tissue's solves are no launches of the persistent kernel: their share of the step instead
+    direct["krylov_ms_per_solve"] = solve_ms / solve_launches if solve_launches else all_solve_ms / max(iters, 1)
 
     # the preconditioner as built by the solves (two-level stands down to block-Jacobi when it cannot help)
     pc_eff, n_coarse, refreshes = s.preconditioner()
     sched["precond_effective"] = {0: "block_jacobi", 1: "ilu0", 2: "two_level", 3: "multilevel"}.get(pc_eff, pc_eff)
     sched["krylov_method"] = {1: "bicgstab", 2: "conjugate gradients",
                               3: "conjugate gradients, finished by bicgstab on indefinite solves",
-                              4: "minres on steps with packing pairs"}.get(max(methods), "none")
+                              4: "minres on steps with packing pairs",
+                              5: "minimal residual iteration with the factor of J's symmetric part"}.get(max(methods), "none")
     sched["krylov_iters_cg_share"] = kry_cg / max(kry, 1)
     # the reference detects node-node packing after every step's growth; the pairs it finds add
     # forces and Jacobian blocks to the Newton iterations

@@ -64,7 +64,11 @@ extern "C" {
                                   /* (a batch uses TF_PRECOND_TWO_LEVEL's space)             */
 
 #define TF_KRYLOV_AUTO 0      /* conjugate gradients when J is symmetric (no internal     */
-                              /* viscosity), else BiCGStab (persistent solve)             */
+                              /* viscosity), else BiCGStab (persistent solve). With       */
+                              /* TF_PRECOND_TWO_LEVEL and warm starts on, tissues whose   */
+                              /* factorisation is below 3e11 operations are preconditioned */
+                              /* by the sparse factor of J's symmetric part instead: one  */
+                              /* or two iterations (not on steps with packing pairs)      */
 #define TF_KRYLOV_BICGSTAB 1  /* BiCGStab                                                 */
 #define TF_KRYLOV_CG 2        /* preconditioned conjugate gradients; a tissue whose J turns */
                               /* out indefinite is solved again with BiCGStab              */
@@ -112,7 +116,8 @@ typedef struct tf_params {
                               /* gradients start from the previous step's solution of the   */
                               /* same Newton iteration (x0, r0 = g - J x0; from zero if that */
                               /* residual is not below ||g||); 0: every solve from zero.    */
-                              /* Same stopping rule either way; the adjoint runs cold       */
+                              /* Same stopping rule either way; the adjoint runs cold. 0    */
+                              /* also keeps the solves off the sparse factor               */
 } tf_params;
 
 typedef struct tf_step_stats {
@@ -127,11 +132,13 @@ typedef struct tf_step_stats {
     double ms_total;            /* device time of the whole call, host copies included      */
     int64_t gpu_launches;       /* kernels this call launched (graph nodes counted)         */
     double ms_solve_kernel;     /* device time inside the persistent BiCGStab launches      */
-    int32_t solve_launches;     /* number of those launches                                 */
+    int32_t solve_launches;     /* number of those launches (0 where the sparse factor      */
+                                /* solved every system)                                     */
     int32_t krylov_method;      /* 1 BiCGStab, 2 conjugate gradients, 3 CG fell back to     */
                                 /* BiCGStab on some solve, 4 MINRES (a symmetric J with    */
-                                /* packing pairs; block preconditioner |D|); the largest    */
-                                /* over the call                                            */
+                                /* packing pairs; block preconditioner |D|), 5 minimal      */
+                                /* residual iteration with the sparse factor (internal      */
+                                /* viscosity); the largest over the call                    */
     int32_t krylov_iters_cg;    /* the conjugate-gradient iterations in krylov_iters_total  */
                                 /* (persistent solves; the rest are BiCGStab's)            */
 } tf_step_stats;
@@ -320,12 +327,14 @@ int tf_get_schedule(tf_ctx* ctx, int32_t* n_colours, int32_t* scatter, int32_t* 
  * took the multilevel space), the number of coarse unknowns of the
  * two-level space summed over the tissues (0 until the first solve, and 0 when a single tissue's
  * aggregates would be too large to help), and how many times the coarse operators have been
- * refactorised. */
+ * refactorised. Where the last solve used the sparse factor: the unknowns of the tissues' top
+ * separators, and the factorisations. */
 int tf_get_preconditioner(tf_ctx* ctx, int32_t* precond, int32_t* n_coarse, int32_t* coarse_refreshes);
 
 /* The Krylov method of the last call's linear solves (no counterpart in the reference, whose
  * Pardiso solve is direct): 1 BiCGStab, 2 conjugate gradients, 3 conjugate gradients that met a
- * non-positive curvature on some tissue, solved again by BiCGStab; 0 before any solve. */
+ * non-positive curvature on some tissue, solved again by BiCGStab, 4 MINRES, 5 the minimal
+ * residual iteration with the sparse factor; 0 before any solve. */
 int tf_get_krylov_method(tf_ctx* ctx, int32_t* method);
 
 /* Nodes per block of the block-Jacobi smoother the context uses (1: 3x3 node blocks; G > 1:

@@ -279,14 +279,16 @@ class NewtonRaphsonSolver:
         return {"n_colours": nc.value, "scatter": sc.value, "elems_per_block": t.value}
 
     def preconditioner(self):
-        """(effective preconditioner, coarse unknowns, coarse refactorisations so far)."""
+        """(effective preconditioner, coarse unknowns, coarse refactorisations so far); with the sparse
+        factor the unknowns of the top separators and the factorisations."""
         pc, nc, rf = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
         capi.check(self._L.tf_get_preconditioner(self._h, ctypes.byref(pc), ctypes.byref(nc), ctypes.byref(rf)),
                    "tf_get_preconditioner", self._h)
         return pc.value, nc.value, rf.value
 
     def krylov_method(self) -> int:
-        """Krylov method of the last call's solves: 1 BiCGStab, 2 CG, 3 CG that fell back to BiCGStab."""
+        """Krylov method of the last call's solves: 1 BiCGStab, 2 CG, 3 CG that fell back to BiCGStab,
+        4 MINRES, 5 minimal residual iteration with the sparse factor."""
         m = ctypes.c_int32()
         capi.check(self._L.tf_get_krylov_method(self._h, ctypes.byref(m)), "tf_get_krylov_method", self._h)
         return m.value
