@@ -337,6 +337,11 @@ int tf_get_preconditioner(tf_ctx* ctx, int32_t* precond, int32_t* n_coarse, int3
  * residual iteration with the sparse factor; 0 before any solve. */
 int tf_get_krylov_method(tf_ctx* ctx, int32_t* method);
 
+/* Page-lock a host buffer that results are copied to, and undo it (no counterpart in the reference).
+ * The buffer outlives the context if need be; copies in flight must have ended before the second call. */
+int tf_host_register(tf_ctx* ctx, void* p, uint64_t bytes);
+int tf_host_unregister(void* p);
+
 /* Nodes per block of the block-Jacobi smoother the context uses (1: 3x3 node blocks; G > 1:
  * the 3G x 3G diagonal sub-block of G consecutive nodes, a prism column). No counterpart in the
  * reference, whose Pardiso solve needs no smoother. */

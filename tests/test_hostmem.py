@@ -1,0 +1,78 @@
+"""The pool of page-locked result arrays: blocks that are in use are not handed out again, what is dropped is
+reused, what does not fit its bound is an ordinary array. On the CPU with a library that only counts."""
+import gc
+
+import numpy as np
+import pytest
+
+from tissueorigami_b200 import capi, hostmem, mesh
+
+MB = 1 << 20
+
+
+class _Lib:
+    def __init__(self):
+        self.live = {}
+
+    def tf_host_register(self, handle, p, n):
+        assert handle == "ctx" and p % 4096 == 0 and p not in self.live
+        self.live[p] = n
+        return 0
+
+    def tf_host_unregister(self, p):
+        del self.live[p]
+        return 0
+
+
+@pytest.mark.parametrize("doubles", [MB // 8 - 1, MB // 8, MB // 8 + 1, 5 * MB // 8 + 3, 40 * MB // 8])
+def test_pool_reuses_only_what_was_dropped(doubles):
+    pool, lib = hostmem._Pool(), _Lib()
+    a = pool.take(lib, "ctx", (doubles,))
+    if 8 * doubles < hostmem.MIN_BYTES:
+        assert a is None
+        return
+    b = pool.take(lib, "ctx", (doubles,))
+    a[:], b[:] = 1.0, 2.0
+    assert (a == 1.0).all() and (b == 2.0).all() and len(lib.live) == 2
+    view, where = a[5:9], a.ctypes.data
+    del a
+    gc.collect()
+    c = pool.take(lib, "ctx", (doubles,))  # the view still holds the first block
+    assert c.ctypes.data not in (where, b.ctypes.data) and (view == 1.0).all()
+    del view
+    gc.collect()
+    d = pool.take(lib, "ctx", (doubles,))
+    assert d.ctypes.data == where and len(lib.live) == 3
+
+
+def test_pool_is_bounded():
+    pool, lib = hostmem._Pool(), _Lib()
+    held = [pool.take(lib, "ctx", (30 * MB // 8,)) for _ in range(8)]
+    assert all(h is not None for h in held) and sum(lib.live.values()) <= hostmem.LIMIT
+    assert pool.take(lib, "ctx", (30 * MB // 8,)) is None
+    assert pool.take(lib, "ctx", (hostmem.LIMIT // 8 + 1,)) is None
+    del held
+    gc.collect()
+    assert sum(lib.live.values()) <= hostmem.KEEP
+    other = pool.take(lib, "ctx", (250 * MB // 8,))  # gives the kept blocks back
+    assert other is not None and sum(lib.live.values()) <= hostmem.LIMIT
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(11, 11), (41, 40)])
+def test_results_equal_those_in_ordinary_arrays(nx, ny):
+    """J of 0.7 and 9 MB, assembled in the coloured scatter's fixed order."""
+    from tissueorigami_b200.newton import NewtonRaphsonSolver
+
+    t = mesh.large_slab(nx=nx, ny=ny)
+    with NewtonRaphsonSolver.from_tissue(t, scatter=2) as s:
+        first = s.assemble(t.x, t.x, t.dt)
+        keep = first[1].copy()
+        second = s.assemble(t.x * 1.001, t.x, t.dt)
+        np.testing.assert_array_equal(first[1], keep)
+        assert np.abs(second[1] - first[1]).max() > 0
+        x = np.ascontiguousarray(t.x, dtype=np.float64).reshape(-1)
+        g, vals = np.empty(x.shape), np.empty(keep.shape)
+        capi.check(s._L.tf_assemble(s._h, capi.dptr(x), capi.dptr(x), t.dt, capi.dptr(g), capi.dptr(vals)), "tf_assemble", s._h)
+        np.testing.assert_array_equal(vals, keep)
+    np.testing.assert_array_equal(first[1], keep)  # the arrays outlive the context

@@ -56,7 +56,7 @@ EXPORTS = [
     "tf_solve_direct", "tf_get_preconditioner", "tf_get_smoother_block", "tf_measure_fp64", "tf_invert_dense", "tf_set_packing", "tf_detect_packing",
     "tf_get_packing", "tf_set_lumen", "tf_get_lumen",
     "tf_set_grid_growth", "tf_set_time", "tf_get_time", "tf_set_external_force", "tf_newton_iteration",
-    "tf_get_krylov_method",
+    "tf_get_krylov_method", "tf_host_register", "tf_host_unregister",
 ]
 
 
@@ -170,6 +170,8 @@ def load(build_if_missing: bool = True):
     L.tf_get_krylov_method.argtypes = [_P, _I]
     L.tf_newton_iteration.argtypes = [_P, _D, _D, c_double, _D, _I, _D]
     L.tf_get_time.argtypes = [_P, _D]
+    L.tf_host_register.argtypes = [_P, _P, ctypes.c_uint64]
+    L.tf_host_unregister.argtypes = [_P]
     L.tf_last_error.argtypes = [_P]
     L.tf_last_error.restype = ctypes.c_char_p
     for name in EXPORTS:

@@ -3354,6 +3354,21 @@ int tf_get_krylov_method(tf_ctx* ctx, int32_t* method) {
     return TF_OK;
 }
 
+int tf_host_register(tf_ctx* ctx, void* p, uint64_t bytes) {
+    const int rc = check_ctx(ctx);
+    if (rc != TF_OK) return rc;
+    if (!p || bytes == 0) return TF_ERR_ARGUMENT;
+    TF_CK(cudaHostRegister(p, (size_t)bytes, cudaHostRegisterPortable));
+    return TF_OK;
+}
+
+int tf_host_unregister(void* p) {
+    if (!p) return TF_ERR_ARGUMENT;
+    if (cudaHostUnregister(p) == cudaSuccess) return TF_OK;
+    cudaGetLastError();
+    return TF_ERR_CUDA;
+}
+
 int tf_get_smoother_block(tf_ctx* ctx, int32_t* nodes) {
     if (!ctx || !nodes) return TF_ERR_ARGUMENT;
     *nodes = use_persistent(ctx) ? ctx->smooth_G : 1;

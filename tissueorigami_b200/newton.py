@@ -13,7 +13,7 @@ from typing import Optional
 
 import numpy as np
 
-from . import capi
+from . import capi, hostmem
 from .mesh import Tissue
 
 
@@ -185,8 +185,8 @@ class NewtonRaphsonSolver:
     # -- the path -------------------------------------------------------------------------------
     def updateStepNR(self, x_n, dt: float):
         """Simulation::updateStepNR: returns (positions, status, stats dict)."""
-        x = _f64(x_n).reshape(self.n_nodes, 3).copy()
-        out = np.empty_like(x)
+        x = _f64(x_n).reshape(self.n_nodes, 3)
+        out = hostmem.result(self._L, self._h, x.shape)
         st = capi.StepStats()
         rc = capi.check(self._L.tf_newton_step(self._h, capi.dptr(x), float(dt), capi.dptr(out), ctypes.byref(st)),
                         "tf_newton_step", self._h)
@@ -195,8 +195,8 @@ class NewtonRaphsonSolver:
 
     def runOneStep(self, x_n, dt: float):
         """Growth prologue + viscosity surfaces + updateStepNR (Simulation::runOneStep subset)."""
-        x = _f64(x_n).reshape(self.n_nodes, 3).copy()
-        out = np.empty_like(x)
+        x = _f64(x_n).reshape(self.n_nodes, 3)
+        out = hostmem.result(self._L, self._h, x.shape)
         st = capi.StepStats()
         rc = capi.check(self._L.tf_time_step(self._h, capi.dptr(x), float(dt), capi.dptr(out), ctypes.byref(st)),
                         "tf_time_step", self._h)
@@ -215,7 +215,7 @@ class NewtonRaphsonSolver:
         """One Newton iteration's residual gSum and Jacobian J = K^T (BSR3 values)."""
         rowptr, colidx = self.pattern()
         g = np.zeros(3 * self.n_nodes)
-        vals = np.zeros((colidx.shape[0], 3, 3)) if want_matrix else None
+        vals = hostmem.result(self._L, self._h, (colidx.shape[0], 3, 3)) if want_matrix else None
         rc = capi.check(self._L.tf_assemble(self._h, capi.dptr(_f64(uk).reshape(-1)), capi.dptr(_f64(un).reshape(-1)),
                                             float(dt), capi.dptr(g), capi.dptr(vals)), "tf_assemble", self._h)
         return g, vals, rowptr, colidx, rc
