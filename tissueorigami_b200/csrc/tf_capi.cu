@@ -184,6 +184,7 @@ struct tf_ctx {
     std::vector<int32_t> fc_chunk0;
     // the launches of a factorisation and of a solve are the same every time (50 to 300 short kernels
     // whose launch alone, 3.4 us each, took longer than many of them): replayed as graphs (0.75 us each)
+    FcStreams fc_streams;
     cudaGraphExec_t fc_graph[2] = {nullptr, nullptr};
     int64_t fc_graph_launches[2] = {0, 0};
     DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_jblk_t, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_kids, fc_dofs, fc_vec, fc_z,
@@ -1781,6 +1782,13 @@ int build_factor(tf_ctx* ctx) {
     TF_CK(e);
     // the padding of the rows, and x11 above its diagonal blocks, stay zero: no kernel writes there
     TF_CK(cudaMemsetAsync(ctx->fc_factor.p, 0, sizeof(double) * (size_t)(P.n_factor + 64), ctx->stream));
+    FcStreams& st = ctx->fc_streams;
+    st.main = ctx->stream;
+    if (!st.fork) TF_CK(cudaEventCreateWithFlags(&st.fork, cudaEventDisableTiming));
+    for (int q = 0; q < 3; ++q) {
+        if (!st.side[q]) TF_CK(cudaStreamCreateWithFlags(&st.side[q], cudaStreamNonBlocking));
+        if (!st.join[q]) TF_CK(cudaEventCreateWithFlags(&st.join[q], cudaEventDisableTiming));
+    }
     TF_CK(dalloc(ctx->fc_flags, sizeof(int32_t) * T));
     TF_CK(dalloc(ctx->fc_neg, sizeof(int32_t) * P.fronts.size()));
     TF_CK(dalloc(ctx->fc_running, sizeof(int32_t) * T));
@@ -1851,7 +1859,7 @@ int factor_solve(tf_ctx* ctx, bool* done) {
     if (!kept) {
         TF_CK(cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream));
         TF_CK(cudaMemsetAsync(ctx->fc_neg.p, 0, sizeof(int32_t) * ctx->fc.fronts.size(), ctx->stream));
-        const int rc = replay_factor(ctx, 0, [&](int64_t* n) { return launch_factor(ctx->fc, f, w.vals, n, ctx->stream); });
+        const int rc = replay_factor(ctx, 0, [&](int64_t* n) { return launch_factor(ctx->fc, f, w.vals, n, ctx->fc_streams); });
         if (rc != TF_OK) return rc;
         ++ctx->coarse_refreshes;
     }
@@ -2720,6 +2728,11 @@ void tf_destroy(tf_ctx* ctx) {
                      &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_neg, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
     for (DevBuf* b : fcb) dfree(*b);
     drop_factor_graphs(ctx);
+    if (ctx->fc_streams.fork) cudaEventDestroy(ctx->fc_streams.fork);
+    for (int q = 0; q < 3; ++q) {
+        if (ctx->fc_streams.join[q]) cudaEventDestroy(ctx->fc_streams.join[q]);
+        if (ctx->fc_streams.side[q]) cudaStreamDestroy(ctx->fc_streams.side[q]);
+    }
     if (ctx->h_coarse_info) cudaFreeHost(ctx->h_coarse_info);
     if (ctx->h_active) cudaFreeHost(ctx->h_active);
     if (ctx->h_du2) cudaFreeHost(ctx->h_du2);

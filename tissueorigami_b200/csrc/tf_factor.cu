@@ -1170,7 +1170,7 @@ cudaError_t opt_in(const void* f, int bytes) { return cudaFuncSetAttribute(f, cu
         if (err_ != cudaSuccess) return err_;        \
     } while (0)
 
-cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, cudaStream_t s) {
+cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, const FcStreams& st) {
     // per-device attributes of the kernels; cheap next to a factorisation
     FC_CK(opt_in((const void*)k_fc_small, fc_small_smem(kT, kFcSmallB)));
     FC_CK(opt_in((const void*)k_fc_col, kPanelSmem));
@@ -1180,8 +1180,22 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
     int64_t n = 0;
     for (int d = (int)plan.depths.size() - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
-        for (const FcRange& r : L.small)
+        // The fronts of a depth do not depend on each other: each size of small fronts and the chain of the
+        // others has a stream of its own, else a depth takes the sum of their latencies (a wing disc of
+        // 10,000 prisms: 11 launches of small fronts, 35 to 120 us each, on 5 depths).
+        bool main_free = L.gather.count == 0;
+        bool forked[3] = {};
+        FC_CK(cudaEventRecord(st.fork, st.main));
+        for (int c = 0; c < 3; ++c) {
+            const FcRange& r = L.small[c];
             if (r.count) {
+                cudaStream_t s = st.main;
+                if (!main_free) {
+                    s = st.side[c];
+                    forked[c] = true;
+                    FC_CK(cudaStreamWaitEvent(s, st.fork, 0));
+                }
+                main_free = false;
                 int smem = 0;
                 for (int k = 0; k < r.count; ++k) {
                     const FcFront& F = plan.fronts[plan.tasks[r.begin + k].front];
@@ -1189,7 +1203,10 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
                 }
                 k_fc_small<<<r.count, 256, smem, s>>>(w, vals, r.begin, d & 1);
                 ++n;
+                if (forked[c]) FC_CK(cudaEventRecord(st.join[c], s));
             }
+        }
+        const cudaStream_t s = st.main;
         if (L.gather.count) {
             const int pmax = plan.fronts[plan.tasks[L.gather.begin].front].p;  // the list starts with the largest
             k_fc_gather<<<L.gather.count, 256, pmax * sizeof(int2), s>>>(w, L.gather.begin, d & 1);
@@ -1222,6 +1239,8 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
             k_fc_schur<<<L.schur.count, 128, kGemmSmem, s>>>(w, L.schur.begin, d & 1);
             ++n;
         }
+        for (int c = 0; c < 3; ++c)
+            if (forked[c]) FC_CK(cudaStreamWaitEvent(st.main, st.join[c], 0));
     }
     *launches += n;
     return cudaGetLastError();

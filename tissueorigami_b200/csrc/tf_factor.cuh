@@ -124,9 +124,14 @@ struct FcWork {
 // kids and dofs of every front from the plan's columns (maps, verts on the device)
 cudaError_t launch_factor_expand(const FcPlan& plan, const FcWork& w, const int32_t* maps, const int32_t* verts,
                                  cudaStream_t s);
+// Streams of a factorisation: the side streams start after and end before what is on `main`.
+struct FcStreams {
+    cudaStream_t main = nullptr, side[3] = {};
+    cudaEvent_t fork = nullptr, join[3] = {};
+};
 // Numeric factorisation of J (vals: the full BSR3 values; block (row, column) is read from the row of
 // the earlier pivot, transposed). Returns the kernels launched in *launches.
-cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, cudaStream_t s);
+cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, const FcStreams& st);
 // x = (factor)^-1 in on the active tissues' unknowns (every unknown is a pivot of one front).
 cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
                                 cudaStream_t s);
