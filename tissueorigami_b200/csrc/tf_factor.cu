@@ -53,14 +53,25 @@ __device__ __forceinline__ double load_if(const double* __restrict__ base, bool 
     return ok ? v : 0.0;
 }
 
+// Programmatic dependent launch: a kernel of a chain lets the next one start when its own CTAs have, and waits
+// for the end of the one before it after it has read its part of the plan (which nothing writes) - the launch
+// and two or three of the dependent loads of every link then overlap the previous kernel. Every CTA waits, also
+// one with nothing to do: the end of a kernel then means the end of all before it. What earlier kernels
+// of the chain write is not reached through `const __restrict__`, which would let a load move above the wait.
+__device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void prefetch(const double* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ---- assembly of a front -------------------------------------------------------------------
 
 // Rows [i j, (i + 1) j) of the front's pivot columns (task j: 8 or 32): what its children left there. Rows below p
 // need the columns up to the diagonal only.
 __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int parity) {
     extern __shared__ int2 s_col[];  // per pivot column: its index on either child's boundary
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
     const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
@@ -101,8 +112,10 @@ __device__ __forceinline__ double j_entry(const FcWork& w, const double* __restr
 // += the front's Jacobian blocks. Block (column k, row i) of the lower triangle is read from row k of
 // J, transposed; each lands on entries of its own.
 __global__ void __launch_bounds__(256) k_fc_scatter(FcWork w, const double* __restrict__ vals, int begin) {
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     const int b0 = F.j0 + tk.i * kFcScatter, b1 = min(b0 + kFcScatter, F.j1);
     for (int e = threadIdx.x; e < (b1 - b0) * 9; e += blockDim.x) {
@@ -252,8 +265,10 @@ __device__ __forceinline__ void tile_wait() {
 __global__ void __launch_bounds__(256) k_fc_diag(FcWork w, int begin) {
     __shared__ __align__(16) double s[kT][kLd];
     __shared__ FactorShared sh;
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     double* A = w.factor + F.x11;
     const int n = min(kT, F.p);
@@ -319,8 +334,10 @@ __global__ void __launch_bounds__(256) k_fc_col(FcWork w, int begin, int k) {
     extern __shared__ double s_dyn[];
     double(*sA)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn);
     double(*sB)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn + kT * kLd);
+    chain_go();
     const FcTask tk = w.tasks[begin + (blockIdx.x >> 2)];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     double* X = w.factor + F.x11;
     const int i = tk.i, part = (blockIdx.x & 3) * 16, nk = min(kT, F.p - k * kT), ni = min(kT, F.p - i * kT);
@@ -389,8 +406,10 @@ __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
     __shared__ FactorShared sh;
     double(*sA)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn);
     double(*sB)[kLd] = reinterpret_cast<double(*)[kLd]>(s_dyn + kT * kLd);
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     double* X = w.factor + F.x11;
     const int i = tk.i, j = tk.j;
@@ -452,8 +471,10 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
     extern __shared__ __align__(16) double s_dyn[];
     __shared__ FactorShared sh;
     __shared__ double s_sign[kT];
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     const int p = F.p, b = F.b, n = p + b, ld = fc_small_ld(p), p8r = (p + 7) & ~7, b16 = (b + 15) & ~15;
     double* sX = s_dyn;
@@ -708,8 +729,10 @@ constexpr int kGemmSmem = 2 * kStages * kT * kKld * (int)sizeof(double);
 // l21 tile (i, j) = A21 rows i x (x11 rows j)^T, times S; x11 is lower triangular, so K ends at the tile.
 __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
     extern __shared__ __align__(16) double s_dyn[];
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.p - j * kT);
     double acc[4][4][2];
@@ -739,8 +762,10 @@ __global__ void __launch_bounds__(128) k_fc_l21(FcWork w, int begin) {
 __global__ void __launch_bounds__(128, 4) k_fc_schur(FcWork w, int begin, int parity) {
     extern __shared__ __align__(16) double s_dyn[];
     __shared__ int s_map[2][2][kT];  // child, rows / columns
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
+    chain_wait();
     if (!w.active[F.tissue]) return;
     const int i = tk.i, j = tk.j, ni = min(kT, F.b - i * kT), nj = min(kT, F.b - j * kT);
     const double* L = w.scratch + F.l21;
@@ -875,22 +900,31 @@ __device__ __forceinline__ void up_rows(const FcWork& w, const FcFront& F, const
     }
 }
 
-__global__ void __launch_bounds__(256) k_fc_up(FcWork w, const double* __restrict__ in, int begin) {
+__global__ void __launch_bounds__(256) k_fc_up(FcWork w, const double* in, int begin) {
     extern __shared__ __align__(16) double s_vec[];  // v_P, padded with zero
     double* s_v = s_vec;
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
-    if (!w.active[F.tissue]) return;
-    for (int c0 = threadIdx.x; c0 < F.p; c0 += 4 * 256) {
-        int2 k[4];
-        int d[4];
-        double x[4], y[4], z[4];
+    const int r0 = tk.i * tk.j, r1 = min(r0 + tk.j, F.p + F.b);
+    int2 k[4];
+    int d[4];
+    auto entries = [&](int c0) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int c = min(c0 + u * 256, F.p - 1);
             k[u] = w.kids[F.ent + c];
             d[u] = w.dofs[F.ent + c];
         }
+    };
+    if ((int)threadIdx.x < F.p) entries(threadIdx.x);
+    // the factor is older than the chain: its rows may be on their way into L2 before the wait
+    for (int o = threadIdx.x * 16; o < (r1 - r0) * F.ldp; o += 256 * 16) prefetch(w.factor + F.x11 + (size_t)r0 * F.ldp + o);
+    chain_wait();
+    if (!w.active[F.tissue]) return;
+    for (int c0 = threadIdx.x; c0 < F.p; c0 += 4 * 256) {
+        double x[4], y[4], z[4];
+        if (c0 != (int)threadIdx.x) entries(c0);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             x[u] = in[d[u]];
@@ -903,7 +937,6 @@ __global__ void __launch_bounds__(256) k_fc_up(FcWork w, const double* __restric
     }
     if (threadIdx.x == 0 && (F.p & 1)) s_v[F.p] = 0.0;
     __syncthreads();
-    const int r0 = tk.i * tk.j, r1 = min(r0 + tk.j, F.p + F.b);
     if (F.p <= 128)
         up_rows<8>(w, F, reinterpret_cast<const double2*>(s_v), r0, r1);
     else
@@ -947,19 +980,27 @@ __device__ __forceinline__ void down_columns(const double* X, int ldp, const dou
     *reinterpret_cast<double2*>(s_p + group * COLS + col) = make_double2(sa, sb);
 }
 
-__global__ void __launch_bounds__(1024) k_fc_down(FcWork w, double* __restrict__ x, int begin) {
+__global__ void __launch_bounds__(1024) k_fc_down(FcWork w, double* x, int begin) {
     extern __shared__ double s_u[];  // [S z; -x_B] from row c0 on
     __shared__ __align__(16) double s_p[32 * 64];
     __shared__ double s_q[4][64];
+    chain_go();
     const FcTask tk = w.tasks[begin + blockIdx.x];
     const FcFront F = w.fronts[tk.front];
-    if (!w.active[F.tissue]) return;
     const int cols = tk.j, c0 = tk.i * cols, n = F.p + F.b, nt = blockDim.x;
-    for (int r = c0 + threadIdx.x; r < F.p; r += nt) s_u[r - c0] = w.sign[F.piv + r] * w.z[F.piv + r];
-    for (int r = threadIdx.x; r < F.b; r += 4 * nt) {
-        int d[4];
+    int d[4];
+    auto entries = [&](int r) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) d[u] = w.dofs[F.ent + F.p + min(r + u * nt, F.b - 1)];
+    };
+    if ((int)threadIdx.x < F.b) entries(threadIdx.x);
+    for (int o = threadIdx.x; o < (n - c0) * (cols / 16); o += nt)
+        prefetch(w.factor + F.x11 + (size_t)(c0 + o / (cols / 16)) * F.ldp + c0 + o % (cols / 16) * 16);
+    chain_wait();
+    if (!w.active[F.tissue]) return;
+    for (int r = c0 + threadIdx.x; r < F.p; r += nt) s_u[r - c0] = w.sign[F.piv + r] * w.z[F.piv + r];
+    for (int r = threadIdx.x; r < F.b; r += 4 * nt) {
+        if (r != (int)threadIdx.x) entries(r);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const double v = x[d[u]];
@@ -1160,6 +1201,27 @@ __global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const dou
     if (k.status != KS_RUNNING) c.running[t] = 0;
 }
 
+// Launches kernels of a stream one after the other, each but the first as a link of a chain.
+struct Chain {
+    cudaStream_t stream;
+    bool linked = false;
+    template <class... P, class... A>
+    cudaError_t operator()(void (*kernel)(P...), int grid, int threads, size_t smem, A... args) {
+        cudaLaunchAttribute a{};
+        a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        a.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3((unsigned)grid);
+        c.blockDim = dim3((unsigned)threads);
+        c.dynamicSmemBytes = smem;
+        c.stream = stream;
+        c.attrs = &a;
+        c.numAttrs = linked ? 1 : 0;
+        linked = true;
+        return cudaLaunchKernelEx(&c, kernel, P(args)...);
+    }
+};
+
 cudaError_t opt_in(const void* f, int bytes) { return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); }
 
 }  // namespace
@@ -1178,6 +1240,7 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
     FC_CK(opt_in((const void*)k_fc_l21, kGemmSmem));
     FC_CK(opt_in((const void*)k_fc_schur, kGemmSmem));
     int64_t n = 0;
+    Chain chain{st.main};
     for (int d = (int)plan.depths.size() - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
         // The fronts of a depth do not depend on each other: each size of small fronts and the chain of the
@@ -1201,46 +1264,49 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
                     const FcFront& F = plan.fronts[plan.tasks[r.begin + k].front];
                     smem = smem < fc_small_smem(F.p, F.b) ? fc_small_smem(F.p, F.b) : smem;
                 }
-                k_fc_small<<<r.count, 256, smem, s>>>(w, vals, r.begin, d & 1);
+                Chain alone{s};
+                FC_CK((forked[c] ? alone : chain)(k_fc_small, r.count, 256, smem, w, vals, r.begin, d & 1));
                 ++n;
                 if (forked[c]) FC_CK(cudaEventRecord(st.join[c], s));
             }
         }
-        const cudaStream_t s = st.main;
         if (L.gather.count) {
             const int pmax = plan.fronts[plan.tasks[L.gather.begin].front].p;  // the list starts with the largest
-            k_fc_gather<<<L.gather.count, 256, pmax * sizeof(int2), s>>>(w, L.gather.begin, d & 1);
+            FC_CK(chain(k_fc_gather, L.gather.count, 256, pmax * sizeof(int2), w, L.gather.begin, d & 1));
             ++n;
         }
         if (L.scatter.count) {
-            k_fc_scatter<<<L.scatter.count, 256, 0, s>>>(w, vals, L.scatter.begin);
+            FC_CK(chain(k_fc_scatter, L.scatter.count, 256, 0, w, vals, L.scatter.begin));
             ++n;
         }
         if (L.diag.count) {
-            k_fc_diag<<<L.diag.count, 256, 0, s>>>(w, L.diag.begin);
+            FC_CK(chain(k_fc_diag, L.diag.count, 256, 0, w, L.diag.begin));
             ++n;
         }
         for (int k = 0; k < L.n_panel; ++k) {
             const FcPanel& P = plan.panels[L.panel0 + k];
             if (P.col.count) {
-                k_fc_col<<<4 * P.col.count, 256, kPanelSmem, s>>>(w, P.col.begin, k);
+                FC_CK(chain(k_fc_col, 4 * P.col.count, 256, kPanelSmem, w, P.col.begin, k));
                 ++n;
             }
             if (P.upd.count) {
-                k_fc_upd<<<P.upd.count, 256, kPanelSmem, s>>>(w, P.upd.begin, k);
+                FC_CK(chain(k_fc_upd, P.upd.count, 256, kPanelSmem, w, P.upd.begin, k));
                 ++n;
             }
         }
         if (L.l21.count) {
-            k_fc_l21<<<L.l21.count, 128, kGemmSmem, s>>>(w, L.l21.begin);
+            FC_CK(chain(k_fc_l21, L.l21.count, 128, kGemmSmem, w, L.l21.begin));
             ++n;
         }
         if (L.schur.count) {
-            k_fc_schur<<<L.schur.count, 128, kGemmSmem, s>>>(w, L.schur.begin, d & 1);
+            FC_CK(chain(k_fc_schur, L.schur.count, 128, kGemmSmem, w, L.schur.begin, d & 1));
             ++n;
         }
         for (int c = 0; c < 3; ++c)
-            if (forked[c]) FC_CK(cudaStreamWaitEvent(st.main, st.join[c], 0));
+            if (forked[c]) {
+                FC_CK(cudaStreamWaitEvent(st.main, st.join[c], 0));
+                chain.linked = false;
+            }
     }
     *launches += n;
     return cudaGetLastError();
@@ -1256,17 +1322,18 @@ cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const doubl
                                 cudaStream_t s) {
     FC_CK(opt_in((const void*)k_fc_down, kFcMaxFront * (int)sizeof(double)));
     int64_t n = 0;
+    Chain chain{s};
     const int depths = (int)plan.depths.size();
     for (int d = depths - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
         if (!L.fwd.count) continue;
-        k_fc_up<<<L.fwd.count, 256, L.fwd_smem, s>>>(w, in, L.fwd.begin);
+        FC_CK(chain(k_fc_up, L.fwd.count, 256, L.fwd_smem, w, in, L.fwd.begin));
         ++n;
     }
     for (int d = 0; d < depths; ++d) {
         const FcDepth& L = plan.depths[d];
         if (!L.bwd.count) continue;
-        k_fc_down<<<L.bwd.count, L.bwd_threads, L.bwd_smem, s>>>(w, x, L.bwd.begin);
+        FC_CK(chain(k_fc_down, L.bwd.count, L.bwd_threads, L.bwd_smem, w, x, L.bwd.begin));
         ++n;
     }
     *launches += n;
