@@ -25,7 +25,8 @@ namespace tfb {
 constexpr int kFcTile = 64;        // pivot panel width and GEMM tile
 constexpr int kFcScatter = 256;    // Jacobian blocks per assembly task
 constexpr int kFcSmallB = 288;     // boundary unknowns up to which a one-panel front is one CTA's
-constexpr int kFcRowEntries = 8192; // entries of [x11; w21] per task of the upward pass
+constexpr int kFcRowEntries = 8192; // most entries of [x11; w21] per task of the upward pass
+constexpr int kFcSms = 148;
 constexpr int kFcMaxPivots = 5000; // pivots of one front, and unknowns of one front: the passes stage
 constexpr int kFcMaxFront = 24000; // vectors of them in shared memory
 

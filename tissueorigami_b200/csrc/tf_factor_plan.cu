@@ -468,18 +468,28 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
         std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) {
             return (int64_t)plan.fronts[a].p * plan.fronts[a].b > (int64_t)plan.fronts[b].p * plan.fronts[b].b;
         });
-        // up: rows of [x11; w21] by entries; down: 64 columns, or 32 and more threads where there are many rows
+        // Up: rows of [x11; w21] by entries, three tasks an SM where a depth is that large (the tasks of a small
+        // depth are latency: 8192 entries each took 2.53 ms a step on 2,713 prisms, 2.33 like this; smaller
+        // still, no gain). Down: 64 columns; 32 and more threads where there are many rows, or fewer tasks
+        // than SMs (2.33 to 2.25 ms; up to four times the SMs: the wing disc loses 1 %).
+        int64_t entries = 0, tiles = 0;
+        for (int32_t fi : all) {
+            entries += (int64_t)(plan.fronts[fi].p + plan.fronts[fi].b) * plan.fronts[fi].p;
+            tiles += cdiv(plan.fronts[fi].p, 64);
+        }
+        const int per = (int)std::min<int64_t>(kFcRowEntries, std::max<int64_t>(kFcRowEntries / 8, entries / (3 * kFcSms)));
+        const bool narrow = tiles < kFcSms;
         list(L.fwd, [&](int32_t fi, const FcFront& F) {
-            const int n = F.p + F.b, rows = F.p > 128 ? std::max(8, kFcRowEntries / F.p / 8 * 8)
-                                                     : std::max(32, kFcRowEntries / std::max(F.p, 1) / 32 * 32);
+            const int n = F.p + F.b, rows = F.p > 128 ? std::max(8, per / F.p / 8 * 8)
+                                                     : std::max(32, per / std::max(F.p, 1) / 32 * 32);
             for (int i = 0; i < cdiv(n, rows); ++i) push(fi, i, std::min(rows, 32736));
             L.fwd_smem = std::max(L.fwd_smem, (int32_t)(F.ldp * sizeof(double)));
         });
         list(L.bwd, [&](int32_t fi, const FcFront& F) {
-            const int cols = F.p > 256 ? 32 : 64;
+            const int cols = F.p > 256 || narrow ? 32 : 64, n = F.p + F.b;
             for (int i = 0; i < cdiv(F.p, cols); ++i) push(fi, i, cols);
             L.bwd_smem = std::max(L.bwd_smem, (int32_t)((F.p + F.b) * sizeof(double)));
-            if (F.p + F.b > 300) L.bwd_threads = std::max(L.bwd_threads, F.p + F.b > 700 ? 1024 : 512);
+            if (n > (narrow ? 128 : 300)) L.bwd_threads = std::max(L.bwd_threads, n > (narrow ? 300 : 700) ? 1024 : 512);
         });
     }
     if (plan.tasks.size() > (size_t)INT32_MAX) return;
