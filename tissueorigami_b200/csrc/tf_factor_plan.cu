@@ -454,8 +454,8 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             plan.panels.push_back(P);
         }
         list(L.l21, [&](int32_t fi, const FcFront& F) {
-            for (int i = 0; i < cdiv(F.b, kFcTile); ++i)
-                for (int j = cdiv(F.p, kFcTile) - 1; j >= 0; --j) push(fi, i, j);
+            for (int j = cdiv(F.p, kFcTile) - 1; j >= 0; --j)
+                for (int i = 0; i < cdiv(F.b, kFcTile); ++i) push(fi, i, j);
         });
         list(L.schur, [&](int32_t fi, const FcFront& F) {
             // with them, from the same l21, the tiles of w21 (j < 0: column tile -1 - j)
@@ -464,6 +464,12 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
             for (int i = 0; i < cdiv(F.b, kFcTile); ++i)
                 for (int j = 0; j <= i; ++j) push(fi, i, j);
         });
+        // the longest products first, so that short ones fill the last wave
+        auto by_length = [&](const FcTask& a, const FcTask& b) {
+            auto length = [&](const FcTask& t) { return plan.fronts[t.front].p - (t.j < 0 ? (-1 - t.j) * kFcTile : 0); };
+            return length(a) > length(b);
+        };
+        std::stable_sort(plan.tasks.begin() + L.schur.begin, plan.tasks.begin() + L.schur.begin + L.schur.count, by_length);
         fs = all;
         std::stable_sort(fs.begin(), fs.end(), [&](int32_t a, int32_t b) {
             return (int64_t)plan.fronts[a].p * plan.fronts[a].b > (int64_t)plan.fronts[b].p * plan.fronts[b].b;
