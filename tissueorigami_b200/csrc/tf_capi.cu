@@ -185,8 +185,8 @@ struct tf_ctx {
     // the launches of a factorisation and of a solve are the same every time (50 to 300 short kernels
     // whose launch alone, 3.4 us each, took longer than many of them): replayed as graphs (0.75 us each)
     FcStreams fc_streams;
-    cudaGraphExec_t fc_graph[2] = {nullptr, nullptr};
-    int64_t fc_graph_launches[2] = {0, 0};
+    cudaGraphExec_t fc_graph[3] = {};  // the factorisation, the first iteration, a further one
+    int64_t fc_graph_launches[3] = {};
     DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_jblk_t, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_kids, fc_dofs, fc_vec, fc_z,
         fc_sign, fc_flags, fc_neg, fc_chunks, fc_chunk0_d, fc_running, fc_part;
 
@@ -1843,6 +1843,8 @@ FcWork make_factor(tf_ctx* c) {
 // value, an ill-conditioned J): the caller solves them all again by the iterative path.
 int factor_solve(tf_ctx* ctx, bool* done) {
     *done = false;
+    const int cap = std::min(kFcMaxIters, ctx->params.krylov_max_iters);
+    if (cap < 1) return TF_OK;
     const KrylovWork w = make_work(ctx);
     FcWork f = make_factor(ctx);
     FcCg c;
@@ -1851,30 +1853,28 @@ int factor_solve(tf_ctx* ctx, bool* done) {
     c.chunks = dptr<FcChunk>(ctx->fc_chunks);
     c.chunk0 = dptr<int32_t>(ctx->fc_chunk0_d);
     c.sc = dptr<KrylovScalars>(ctx->tscalars);
+    c.host = ctx->h_tsc;
     c.active = dptr<int32_t>(ctx->active_d);
     c.running = dptr<int32_t>(ctx->fc_running);
     c.part = dptr<double>(ctx->fc_part);
     c.minres = ctx->has_visc;
     const bool kept = ctx->fc_same || ctx->fc_near;
     if (!kept) {
-        TF_CK(cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream));
-        TF_CK(cudaMemsetAsync(ctx->fc_neg.p, 0, sizeof(int32_t) * ctx->fc.fronts.size(), ctx->stream));
-        const int rc = replay_factor(ctx, 0, [&](int64_t* n) { return launch_factor(ctx->fc, f, w.vals, n, ctx->fc_streams); });
+        const int rc = replay_factor(ctx, 0, [&](int64_t* n) -> cudaError_t {
+            cudaError_t e = cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(ctx->fc_neg.p, 0, sizeof(int32_t) * ctx->fc.fronts.size(), ctx->stream);
+            return e == cudaSuccess ? launch_factor(ctx->fc, f, w.vals, n, ctx->fc_streams) : e;
+        });
         if (rc != TF_OK) return rc;
         ++ctx->coarse_refreshes;
     }
-    const int cap = std::min(kFcMaxIters, ctx->params.krylov_max_iters);
-    TF_CK(launch_fc_start(w, c, ctx->params.krylov_rtol, cap, ctx->stream));
-    ctx->launches += 1;
     f.active = c.running;
-    double* z = w.phat;
     bool running = true;
     for (int it = 0; it < cap && running; ++it) {
-        const int rc = replay_factor(ctx, 1, [&](int64_t* n) { return launch_factor_solve(ctx->fc, f, w.r, z, n, ctx->stream); });
+        const int rc = replay_factor(ctx, it == 0 ? 1 : 2, [&](int64_t* n) {
+            return launch_fc_iteration(ctx->fc, f, w, c, it == 0, ctx->params.krylov_rtol, cap, w.phat, w.v, n, ctx->stream);
+        });
         if (rc != TF_OK) return rc;
-        ctx->launches += launch_fc_iteration(w, c, it == 0, z, w.v, ctx->stream);
-        TF_CK(cudaGetLastError());
-        TF_CK(cudaMemcpyAsync(ctx->h_tsc, ctx->tscalars.p, sizeof(KrylovScalars) * ctx->T, cudaMemcpyDeviceToHost, ctx->stream));
         TF_CK(cudaStreamSynchronize(ctx->stream));
         running = false;
         for (int t = 0; t < ctx->T; ++t)

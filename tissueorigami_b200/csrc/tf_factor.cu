@@ -1057,6 +1057,28 @@ __device__ __forceinline__ double tissue_total(const FcCg& c, const double* part
     for (int k = c.chunk0[t] + threadIdx.x; k < c.chunk0[t + 1]; k += blockDim.x) s += __ldcg(part + k);
     return block_total(s, smem);
 }
+// Of the first two kinds of partials at once.
+__device__ __forceinline__ double2 tissue_totals(const FcCg& c, int t, double* smem) {
+    double s = 0.0, u = 0.0;
+    for (int k = c.chunk0[t] + threadIdx.x; k < c.chunk0[t + 1]; k += blockDim.x) {
+        s += __ldcg(c.part + k);
+        u += __ldcg(c.part + c.n_chunks + k);
+    }
+    s = warp_sum(s);
+    u = warp_sum(u);
+    if ((threadIdx.x & 31) == 0) {
+        smem[threadIdx.x >> 5] = s;
+        smem[8 + (threadIdx.x >> 5)] = u;
+    }
+    __syncthreads();
+    double2 r = make_double2(0.0, 0.0);
+    for (int k = 0; k < 8; ++k) {
+        r.x += smem[k];
+        r.y += smem[8 + k];
+    }
+    __syncthreads();
+    return r;
+}
 
 // True in every thread of the last CTA of the tissue to arrive, after all partials are visible.
 __device__ __forceinline__ bool last_of_tissue(const FcCg& c, int t) {
@@ -1074,8 +1096,10 @@ __device__ __forceinline__ bool last_of_tissue(const FcCg& c, int t) {
 
 __global__ void __launch_bounds__(256) k_fc_cg_start(KrylovWork w, FcCg c, double rtol, int max_iter) {
     __shared__ double smem[8];
+    chain_go();
     const FcChunk ch = c.chunks[blockIdx.x];
     const int t = ch.tissue;
+    chain_wait();
     if (!c.active[t]) {
         if (threadIdx.x == 0 && (int)blockIdx.x == c.chunk0[t]) c.running[t] = 0;
         return;
@@ -1101,12 +1125,15 @@ __global__ void __launch_bounds__(256) k_fc_cg_start(KrylovWork w, FcCg c, doubl
         k.method = c.minres ? KM_MINIMAL_RESIDUAL : KM_CG;
         k.status = !isfinite(bb) ? KS_NONFINITE : (bb > 0.0 ? KS_RUNNING : KS_CONVERGED);
         c.running[t] = k.status == KS_RUNNING;
+        c.host[t] = k;
     }
 }
 
-__global__ void __launch_bounds__(256) k_fc_cg_dot(KrylovWork w, FcCg c, const double* __restrict__ z) {
+__global__ void __launch_bounds__(256) k_fc_cg_dot(KrylovWork w, FcCg c, const double* z) {
     __shared__ double smem[8];
+    chain_go();
     const FcChunk ch = c.chunks[blockIdx.x];
+    chain_wait();
     if (!c.running[ch.tissue]) return;
     double s = 0.0;
     for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) s += w.r[i] * z[i];
@@ -1114,9 +1141,11 @@ __global__ void __launch_bounds__(256) k_fc_cg_dot(KrylovWork w, FcCg c, const d
     if (threadIdx.x == 0) c.part[blockIdx.x] = s;
 }
 
-__global__ void __launch_bounds__(256) k_fc_cg_p(KrylovWork w, FcCg c, const double* __restrict__ z) {
+__global__ void __launch_bounds__(256) k_fc_cg_p(KrylovWork w, FcCg c, const double* z) {
     __shared__ double smem[8];
+    chain_go();
     const FcChunk ch = c.chunks[blockIdx.x];
+    chain_wait();
     if (!c.running[ch.tissue]) return;
     const double beta = tissue_total(c, c.part, ch.tissue, smem) / c.sc[ch.tissue].rho_prev;
     for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) w.p[i] = z[i] + beta * w.p[i];
@@ -1126,11 +1155,15 @@ __global__ void __launch_bounds__(256) k_fc_cg_p(KrylovWork w, FcCg c, const dou
 // well, so that it needs no kernel before this one. The minimal residual iteration is all first ones, with
 // (r, q) and (q, q).
 template <bool FIRST>
-__global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const double* __restrict__ z, double* __restrict__ q) {
+__global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const double* z, double* q) {
     __shared__ double smem[8];
+    chain_go();
     const FcChunk ch = c.chunks[blockIdx.x];
+    const int k0 = w.rowptr[ch.row0], k1 = w.rowptr[ch.row1];
+    for (int o = k0 * 9 + (int)threadIdx.x * 16; o < k1 * 9; o += 256 * 16) prefetch(w.vals + o);  // J is older than the chain
+    chain_wait();
     if (!c.running[ch.tissue]) return;
-    const double* __restrict__ pv = FIRST ? z : w.p;
+    const double* pv = FIRST ? z : w.p;
     const int gl = threadIdx.x & 7;
     double dot = 0.0, rho = 0.0;
     for (int base = ch.row0; base < ch.row1; base += 32) {
@@ -1178,14 +1211,15 @@ __global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const 
 // iterations, or still running. A step that does not look like one of a (nearly) exact preconditioner
 // - (r, z) and (p, J p) of opposite sign, or a residual that does not fall - ends with KS_INDEFINITE,
 // and the caller takes another path.
-__global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const double* __restrict__ q) {
-    __shared__ double smem[8];
+__global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const double* q) {
+    __shared__ double smem[16];
+    chain_go();
     const FcChunk ch = c.chunks[blockIdx.x];
     const int t = ch.tissue;
+    chain_wait();
     if (!c.running[t]) return;
-    const double rho = tissue_total(c, c.part, t, smem);
-    const double pq = tissue_total(c, c.part + c.n_chunks, t, smem);
-    const double alpha = rho / pq;
+    const double2 both = tissue_totals(c, t, smem);
+    const double rho = both.x, pq = both.y, alpha = rho / pq;
     double s = 0.0;
     for (int i = 3 * ch.row0 + threadIdx.x; i < 3 * ch.row1; i += 256) {
         w.x[i] += alpha * w.p[i];
@@ -1212,6 +1246,7 @@ __global__ void __launch_bounds__(256) k_fc_cg_x(KrylovWork w, FcCg c, const dou
     else if (k.iter >= k.max_iter)
         k.status = KS_MAXIT;
     if (k.status != KS_RUNNING) c.running[t] = 0;
+    c.host[t] = k;
 }
 
 // Launches kernels of a stream one after the other, each but the first as a link of a chain.
@@ -1331,44 +1366,39 @@ cudaError_t launch_factor_expand(const FcPlan& plan, const FcWork& w, const int3
     return cudaGetLastError();
 }
 
-cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
-                                cudaStream_t s) {
+cudaError_t launch_fc_iteration(const FcPlan& plan, const FcWork& f, const KrylovWork& w, const FcCg& c, bool first, double rtol,
+                                int max_iter, double* z, double* q, int64_t* launches, cudaStream_t s) {
     FC_CK(opt_in((const void*)k_fc_down, kFcMaxFront * (int)sizeof(double)));
     int64_t n = 0;
     Chain chain{s};
+    if (first) {
+        FC_CK(chain(k_fc_cg_start, c.n_chunks, 256, 0, w, c, rtol, max_iter));
+        ++n;
+    }
     const int depths = (int)plan.depths.size();
     for (int d = depths - 1; d >= 0; --d) {
         const FcDepth& L = plan.depths[d];
         if (!L.fwd.count) continue;
-        FC_CK(chain(k_fc_up, L.fwd.count, 256, L.fwd_smem, w, in, L.fwd.begin));
+        FC_CK(chain(k_fc_up, L.fwd.count, 256, L.fwd_smem, f, w.r, L.fwd.begin));
         ++n;
     }
     for (int d = 0; d < depths; ++d) {
         const FcDepth& L = plan.depths[d];
         if (!L.bwd.count) continue;
-        FC_CK(chain(k_fc_down, L.bwd.count, L.bwd_threads, L.bwd_smem, w, x, L.bwd.begin));
+        FC_CK(chain(k_fc_down, L.bwd.count, L.bwd_threads, L.bwd_smem, f, z, L.bwd.begin));
         ++n;
     }
-    *launches += n;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int max_iter, cudaStream_t s) {
-    k_fc_cg_start<<<c.n_chunks, 256, 0, s>>>(w, c, rtol, max_iter);
-    return cudaGetLastError();
-}
-
-int launch_fc_iteration(const KrylovWork& w, const FcCg& c, bool first, const double* z, double* q, cudaStream_t s) {
-    first = first || c.minres;
-    if (first) {
-        k_fc_cg_spmv<true><<<c.n_chunks, 256, 0, s>>>(w, c, z, q);
+    if (first || c.minres) {
+        FC_CK(chain(k_fc_cg_spmv<true>, c.n_chunks, 256, 0, w, c, z, q));
     } else {
-        k_fc_cg_dot<<<c.n_chunks, 256, 0, s>>>(w, c, z);
-        k_fc_cg_p<<<c.n_chunks, 256, 0, s>>>(w, c, z);
-        k_fc_cg_spmv<false><<<c.n_chunks, 256, 0, s>>>(w, c, z, q);
+        FC_CK(chain(k_fc_cg_dot, c.n_chunks, 256, 0, w, c, z));
+        FC_CK(chain(k_fc_cg_p, c.n_chunks, 256, 0, w, c, z));
+        FC_CK(chain(k_fc_cg_spmv<false>, c.n_chunks, 256, 0, w, c, z, q));
+        n += 2;
     }
-    k_fc_cg_x<<<c.n_chunks, 256, 0, s>>>(w, c, q);
-    return first ? 2 : 4;
+    FC_CK(chain(k_fc_cg_x, c.n_chunks, 256, 0, w, c, q));
+    *launches += n + 2;
+    return cudaGetLastError();
 }
 
 }  // namespace tfb

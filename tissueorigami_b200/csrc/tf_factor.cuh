@@ -133,10 +133,6 @@ struct FcStreams {
 // Numeric factorisation of J (vals: the full BSR3 values; block (row, column) is read from the row of
 // the earlier pivot, transposed). Returns the kernels launched in *launches.
 cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* vals, int64_t* launches, const FcStreams& st);
-// x = (factor)^-1 in on the active tissues' unknowns (every unknown is a pivot of one front).
-cudaError_t launch_factor_solve(const FcPlan& plan, const FcWork& w, const double* in, double* x, int64_t* launches,
-                                cudaStream_t s);
-
 // Preconditioned iterations with the factor as preconditioner, one kernel per phase, every tissue with its
 // own scalars: conjugate gradients, or for an unsymmetric J the minimal residual iteration (p = z,
 // alpha = (r, q) / (q, q)), which the factor of the symmetric part contracts by the asymmetry. A chunk is a run of rows of one tissue; the dot products are summed
@@ -155,15 +151,16 @@ struct FcCg {
     const FcChunk* chunks;
     const int32_t* chunk0;  // [T+1]
     KrylovScalars* sc;      // [T]
+    KrylovScalars* host;    // [T] page-locked: sc after the start and after every iteration
     const int32_t* active;  // [T] tissues of this solve
     int32_t* running;       // [T] still iterating (the preconditioner's active flags)
     double* part;           // [3][n_chunks]: (r, z), (p, J p), (r, r) / (b, b)
     int32_t minres;         // 1: the minimal residual iteration (part: (r, q), (q, q), (r, r))
 };
-// x = 0, r = b; every active tissue running (unless b = 0)
-cudaError_t launch_fc_start(const KrylovWork& w, const FcCg& c, double rtol, int max_iter, cudaStream_t s);
-// one iteration after z = M^-1 r: p = z + beta p (p = z in the first), q = J p, x += alpha p,
-// r -= alpha q, and the test. Returns the kernels launched.
-int launch_fc_iteration(const KrylovWork& w, const FcCg& c, bool first, const double* z, double* q, cudaStream_t s);
+// One iteration: z = M^-1 r (a pass up and down the tree with the factor; every unknown is a pivot of one
+// front), p = z + beta p (p = z in the first), q = J p, x += alpha p, r -= alpha q, and the test. Before the
+// first: x = 0, r = b; every active tissue running (unless b = 0).
+cudaError_t launch_fc_iteration(const FcPlan& plan, const FcWork& f, const KrylovWork& w, const FcCg& c, bool first, double rtol,
+                                int max_iter, double* z, double* q, int64_t* launches, cudaStream_t s);
 
 }  // namespace tfb
