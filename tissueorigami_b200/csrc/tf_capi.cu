@@ -2210,9 +2210,11 @@ int newton_core(tf_ctx* ctx, double dt, tf_step_stats* st) {
         if (rc != TF_OK) return rc;
         KrylovWork w = make_work(ctx);
         if (persistent) {
-            TF_CK(launch_newton_update_batched(w, make_plan(ctx), dptr<double>(ctx->uk), dptr<int32_t>(ctx->slaves_d),
+            BatchPlan update = make_plan(ctx);
+            update.du2_host = ctx->h_du2;
+            update.flags_host = ctx->h_flags;
+            TF_CK(launch_newton_update_batched(w, update, dptr<double>(ctx->uk), dptr<int32_t>(ctx->slaves_d),
                                                dptr<int32_t>(ctx->masters_d), (int32_t)ctx->slave.size(), ctx->stream));
-            TF_CK(cudaMemcpyAsync(ctx->h_du2, ctx->tdu2.p, sizeof(double) * T, cudaMemcpyDeviceToHost, ctx->stream));
         } else {
             *ctx->h_tsc = *ctx->h_sc;
             TF_CK(launch_newton_update(w, dptr<double>(ctx->uk), dptr<int32_t>(ctx->slaves_d), dptr<int32_t>(ctx->masters_d),
@@ -2221,8 +2223,12 @@ int newton_core(tf_ctx* ctx, double dt, tf_step_stats* st) {
         }
         ctx->launches += ctx->slave.empty() ? 1 : 2;
         TF_CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-        rc = read_flags(ctx);
-        if (rc != TF_OK) return rc;
+        if (persistent) {
+            TF_CK(cudaStreamSynchronize(ctx->stream));
+        } else {
+            rc = read_flags(ctx);
+            if (rc != TF_OK) return rc;
+        }
         if (!persistent) ctx->h_du2[0] = ctx->h_sc->du2;
         TF_CK(cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]));
         st->ms_assemble += ms;

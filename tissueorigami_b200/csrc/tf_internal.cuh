@@ -148,6 +148,8 @@ struct BatchPlan {
     GridBarrier* barriers;       // [T]
     KrylovScalars* scalars;      // [T]
     double* du2;                 // [T] ||du||^2 of the last Newton update
+    double* du2_host;            // [T] page-locked, with flags_host the flags after the update; or NULL
+    int32_t* flags_host;
     // two-level preconditioner of a single tissue (agg_per_cta = 0: block-Jacobi only). Each
     // CTA's rows [r0, r1) split into agg_per_cta aggregates [r0 + L k / m, r0 + L (k+1) / m);
     // aggregate a (CTA lc, local k: a = lc m + k) owns coarse unknowns 6a .. 6a+5.

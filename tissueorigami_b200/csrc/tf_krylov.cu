@@ -1818,12 +1818,19 @@ __global__ void k_newton_update_batched(KrylovWork w, BatchPlan plan, double* uk
             last = (k == (uint32_t)nct - 1);
         }
         __syncthreads();
-        if (last && threadIdx.x == 0) {
+        if (last) {  // one load a thread: one thread's 148 took 8 us of 15
             __threadfence();
-            double sum = 0.0;
-            for (int i = 0; i < nct; ++i) sum += __ldcg(part + i);
-            plan.du2[t] = sum;
-            plan.barriers[t].count = 0u;
+            double sum[1] = {0.0};
+            for (int i = threadIdx.x; i < nct; i += blockDim.x) sum[0] += __ldcg(part + i);
+            block_sum<1>(sum, smem);
+            if (threadIdx.x == 0) {
+                plan.du2[t] = sum[0];
+                plan.barriers[t].count = 0u;
+                if (plan.du2_host) {  // page-locked: no copies between the update and the host's test
+                    plan.du2_host[t] = sum[0];
+                    *plan.flags_host = *w.dflags;
+                }
+            }
         }
         __syncthreads();
     }
