@@ -38,9 +38,10 @@ constexpr int kMlAutoNodes = 100000; // single tissues from this size take the m
 constexpr int kMlTopMaxAge = 8;      // solves between refreshes of the multilevel top inverse
 constexpr int kWarmSlots = 8;        // Newton iterations whose solutions are kept for warm starts
 constexpr int kFcMaxIters = 8;       // iterations after which a factorised solve counts as failed
-constexpr double kFcKeepFlops = 5e7; // factorisations from this size on are kept from the second Newton iteration
-                                     // (342 prisms, 1e7: 1.18 ms a step anew, 1.54 kept; 2,713 prisms,
-                                     // 2e8: 4.6 and 3.9; 79,650 prisms, 4.3e10: 26.5 and 19.6)
+// Factorisations from this size on are kept from the second Newton iteration. Anew, or the three further passes of a
+// kept one with their products and host waits, us: 342 prisms (1e7) 127 and 180; 2,661 prisms (2e8) 554 and 280;
+// 79,650 prisms (4.3e10) 5,000 and 1,300.
+constexpr double kFcKeepFlops = 5e7;
 // Largest factorisation (operations of one tissue, or the mean of a batch). ms a step, factorised and
 // conjugate gradients: slab of 86,400 nodes 24.9 and 81, 125,000 nodes (1.6e11) 38.7 and 47, 174,000 nodes
 // (2.7e11) 53 and 58; wing disc of 135,651 nodes 36.6 and 139.

@@ -11,8 +11,9 @@
 //   k_fc_l21       l21 = A21 x11^T S
 //   k_fc_schur     C = children - l21 S l21^T, and w21 = l21 x11
 //   k_fc_small     all of it for a front of one panel and a short boundary
-// A wing disc of 79,650 prisms (4.3e10 operations): 5.2 ms, of which the Schur and w21 tiles 1.7, the small
-// fronts 1.4, the chain of 72 panels 2.0 (they share the depths), l21 0.6; 1.2 ms would be the tensor rate.
+// A wing disc of 79,650 prisms (4.3e10 operations): 5.0 ms, of which the Schur and w21 tiles 2.1, the chain of
+// 68 panels 1.8, l21 0.7, the gathers 0.3, the small fronts 0.4 behind others; 1.2 ms would be the tensor rate.
+// A pass: 0.37 ms for twice the factor's 519 MB (0.16 ms at the copy rate).
 #include <math.h>
 
 #include "tf_factor.cuh"
@@ -58,6 +59,7 @@ __device__ __forceinline__ double load_if(const double* __restrict__ base, bool 
 // and two or three of the dependent loads of every link then overlap the previous kernel. Every CTA waits, also
 // one with nothing to do: the end of a kernel then means the end of all before it. What earlier kernels
 // of the chain write is not reached through `const __restrict__`, which would let a load move above the wait.
+// Step of a wing disc of 23,876 prisms 7.39 -> 6.69 ms, of a disc of 2,661 2.73 -> 2.53.
 __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void prefetch(const double* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -1293,7 +1295,8 @@ cudaError_t launch_factor(const FcPlan& plan, const FcWork& w, const double* val
         const FcDepth& L = plan.depths[d];
         // The fronts of a depth do not depend on each other: each size of small fronts and the chain of the
         // others has a stream of its own, else a depth takes the sum of their latencies (a wing disc of
-        // 10,000 prisms: 11 launches of small fronts, 35 to 120 us each, on 5 depths).
+        // 23,876 prisms: 11 launches of small fronts, 35 to 120 us each, on 5 depths; 8.15 ms a
+        // step like that, 7.39 side by side).
         bool main_free = L.gather.count == 0;
         bool forked[3] = {};
         FC_CK(cudaEventRecord(st.fork, st.main));
