@@ -2573,7 +2573,7 @@ static int create_ctx(const tf_mesh_desc* mesh, const tf_params* params, int32_t
     {
         int coop = 0;
         TF_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-        // a large single tissue: one 768-thread CTA per SM (fewest grid-barrier participants);
+        // a large single tissue: one 640-thread CTA per SM (fewest grid-barrier participants);
         // small tissues and batches: three 256-thread CTAs per SM (more, smaller row ranges, and
         // in a batch many tissues each with their own CTAs)
         int sms = 0;
@@ -2581,7 +2581,7 @@ static int create_ctx(const tf_mesh_desc* mesh, const tf_params* params, int32_t
         ctx->persist_threads = (T == 1 && ((int64_t)ctx->N >= (int64_t)sms * 256 ||
                                            ctx->params.precond == TF_PRECOND_TWO_LEVEL ||
                                            ctx->params.precond == TF_PRECOND_MULTILEVEL))
-                                   ? 768
+                                   ? kPersistWide
                                    : 256;
         ctx->persistent_grid_max = coop ? persistent_max_grid(ctx->device, ctx->persist_threads) : 0;
     }

@@ -208,7 +208,7 @@ constexpr int kMaxCoarse = 2048;  // coarse unknowns the persistent solve stages
 // rounded to FP32 (6m x n_coarse floats; the correction is accumulated in FP64 and the solve's
 // convergence test is on the FP64 residual, so this only changes the fixed preconditioner).
 // The block stays small enough that the SM keeps most of its L1 for the SpMV's matrix reuse.
-// The two-level solve runs one 768-thread CTA per SM.
+// The two-level solve runs one kPersistWide-thread CTA per SM.
 constexpr int kCoarseSmemBytes = 96 * 1024;
 
 // --- element assembly (tf_element.cu) ---------------------------------------------------
@@ -284,6 +284,10 @@ int direct_solve_bsr3(int32_t n_nodes, int64_t nnzb, const int32_t* rowptr, cons
                       const double* b, double* x, cudaStream_t s, float* ms, int* method);
 
 // --- Krylov (tf_krylov.cu) ----------------------------------------------------------------
+// Threads of the persistent solve's one-CTA-per-SM build: 20 warps of 96 registers, three of a lane's blocks in flight
+// in the row product. With 24 warps of 80 and one block in flight a CG iteration of a slab of 2,000,000 nodes took
+// 819 us instead of 742, of a wing disc of 60,867 50.5 instead of 49.2; 16 warps of 128: 794.
+constexpr int kPersistWide = 640;
 struct KrylovWork {
     int32_t n_nodes;
     const int32_t* rowptr;
@@ -335,7 +339,7 @@ cudaError_t launch_newton_update(const KrylovWork& w, double* uk, const int32_t*
 int spmv_grid(int n_nodes);
 // Persistent cooperative BiCGStab over a batch of tissues (one tissue: a plan with T = 1).
 // w.partials must hold 4 * plan.n_cta doubles.
-// threads: CTA width, 256 (three CTAs per SM, for batches of many tissues) or 768 (one per SM).
+// threads: CTA width, 256 (three CTAs per SM, for batches of many tissues) or kPersistWide (one per SM).
 int persistent_max_grid(int device, int threads);
 // Coarse operator of the two-level preconditioner, row-major dense n_coarse^2: entry
 // (6a+r, 6b+c) = sum over the Jacobian blocks k in rows of aggregate a and columns of

@@ -460,7 +460,7 @@ __device__ void write_partials(double (&v)[NDOT], double* buf, int local, double
 // y = J x for rows [r0, r1) with kGroup lanes per row; returns this thread's share of the
 // dots (rhat,y) [KIND 1], (s,y), (y,y) [KIND 2] or (p,y) [KIND 3].
 template <int KIND>
-__device__ __forceinline__ void spmv_rows(const KrylovWork& w, int r0, int r1, const double* __restrict__ xin,
+__device__ __forceinline__ void spmv_rows_narrow(const KrylovWork& w, int r0, int r1, const double* __restrict__ xin,
                                           double* __restrict__ yout, double& d0, double& d1) {
     const int gl = threadIdx.x & (kGroup - 1);
     const int groups = blockDim.x / kGroup;
@@ -508,6 +508,107 @@ __device__ __forceinline__ void spmv_rows(const KrylovWork& w, int r0, int r1, c
                 d1 += y0 * y0 + y1 * y1 + y2 * y2;
         }
     }
+}
+
+// The same with a row's first 24 blocks in flight at once, for the build that has the registers: one block a lane at
+// a time the phase waited on memory (long scoreboard) at 24 warps an SM. CG iteration of a slab of 2,000,000
+// nodes 819 -> 742 us, of 240,000 139 -> 125; BiCGStab on 600,000 673 -> 567.
+template <int KIND>
+__device__ __forceinline__ void spmv_rows_wide(const KrylovWork& w, int r0, int r1, const double* __restrict__ xin,
+                                          double* __restrict__ yout, double& d0, double& d1) {
+    const int gl = threadIdx.x & (kGroup - 1);
+    const int groups = blockDim.x / kGroup;
+    if (r0 >= r1) return;
+    // two rows ahead: block ranges; one row ahead: the first three column indices
+    auto range = [&](int row, int& a, int& z) {
+        const int q = min(row, r1 - 1);
+        a = __ldg(w.rowptr + q);
+        z = row < r1 ? __ldg(w.rowptr + q + 1) : a;
+    };
+    int row = r0 + threadIdx.x / kGroup;
+    int ka, kz, na, nz;
+    int c[3];
+    range(row, ka, kz);
+#pragma unroll
+    for (int u = 0; u < 3; ++u) c[u] = __ldg(w.colidx + min(ka + gl + u * kGroup, max(kz - 1, ka)));
+    range(row + groups, na, nz);
+    for (int rb = r0; rb < r1; rb += groups, row += groups) {
+        double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+        double a[3] = {0.0, 0.0, 0.0}, b[3] = {0.0, 0.0, 0.0};
+        int cn[3], fa, fz;
+#pragma unroll
+        for (int u = 0; u < 3; ++u) cn[u] = __ldg(w.colidx + min(na + gl + u * kGroup, max(nz - 1, na)));
+        range(row + 2 * groups, fa, fz);
+        if (row < r1 && gl == 0) {
+            const double* av = KIND == 1 ? w.rhat : (KIND == 3 || KIND == 4 ? w.p : w.s);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) a[i] = av[row * 3 + i];
+            if (KIND == 4)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) b[i] = w.r[row * 3 + i];
+        }
+        {
+            double B[3][9], x[3][3];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int k = ka + gl + u * kGroup;
+                const bool in = k < kz;
+                const double* q = w.vals + (size_t)(in ? k : ka) * 9;
+                if (in) {
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) B[u][e] = __ldg(q + e);
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) x[u][e] = __ldca(xin + c[u] * 3 + e);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) B[u][e] = 0.0;
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) x[u][e] = 0.0;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                y0 += B[u][0] * x[u][0] + B[u][1] * x[u][1] + B[u][2] * x[u][2];
+                y1 += B[u][3] * x[u][0] + B[u][4] * x[u][1] + B[u][5] * x[u][2];
+                y2 += B[u][6] * x[u][0] + B[u][7] * x[u][1] + B[u][8] * x[u][2];
+            }
+        }
+        if (row < r1) {
+            row_dot<kGroup>(w, ka + gl + 3 * kGroup, kz, xin, y0, y1, y2);
+            row_aux<kGroup>(w, row, gl, xin, y0, y1, y2);
+        }
+        ka = na;
+        kz = nz;
+        na = fa;
+        nz = fz;
+#pragma unroll
+        for (int u = 0; u < 3; ++u) c[u] = cn[u];
+#pragma unroll
+        for (int off = kGroup / 2; off > 0; off >>= 1) {
+            y0 += __shfl_xor_sync(0xffffffffu, y0, off);
+            y1 += __shfl_xor_sync(0xffffffffu, y1, off);
+            y2 += __shfl_xor_sync(0xffffffffu, y2, off);
+        }
+        if (row < r1 && gl == 0) {
+            yout[row * 3 + 0] = y0;
+            yout[row * 3 + 1] = y1;
+            yout[row * 3 + 2] = y2;
+            d0 += a[0] * y0 + a[1] * y1 + a[2] * y2;
+            if (KIND == 4)
+                d1 += a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+            else if (KIND == 2)
+                d1 += y0 * y0 + y1 * y1 + y2 * y2;
+        }
+    }
+}
+
+template <int KIND, bool WIDE>
+__device__ __forceinline__ void spmv_rows(const KrylovWork& w, int r0, int r1, const double* __restrict__ xin,
+                                          double* __restrict__ yout, double& d0, double& d1) {
+    if (WIDE)
+        spmv_rows_wide<KIND>(w, r0, r1, xin, yout, d0, d1);
+    else
+        spmv_rows_narrow<KIND>(w, r0, r1, xin, yout, d0, d1);
 }
 
 // The persistent solve keeps a node block's 3x3 inverse in FP32 at dinv32(w) + 9 n (it only
@@ -1282,6 +1383,7 @@ __device__ bool restart(const KrylovWork& w, int r0, int r1, double& rho, double
 // the tissue's group (nct = 1: a tissue solved by this CTA alone, with CTA-level barriers only).
 // The group's per-CTA partial sums live at partials[4 pbase ..) (4 nct doubles). Returns false
 // when a group barrier timed out.
+template <bool WIDE>
 __device__ bool solve_tissue(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase, double rtol,
                              int max_iter, double* smem, double* sb, double* red, double* ys, double* Ms, double* cs,
                              float* cinv_s) {
@@ -1344,7 +1446,7 @@ __device__ bool solve_tissue(const KrylovWork& w, const BatchPlan& plan, int t, 
         if (!group_barrier(bar, nct, w.dflags)) return false;
         // B: v = J phat; (rhat, v)
         double d0 = 0.0, d1 = 0.0;
-        spmv_rows<1>(w, r0, r1, w.phat, w.v, d0, d1);
+        spmv_rows<1, WIDE>(w, r0, r1, w.phat, w.v, d0, d1);
         v1[0] = d0;
         write_partials<1>(v1, part[pb], lc, smem);
         if (!group_barrier(bar, nct, w.dflags)) return false;
@@ -1367,7 +1469,7 @@ __device__ bool solve_tissue(const KrylovWork& w, const BatchPlan& plan, int t, 
         // D: t = J shat; (t, s), (t, t)
         d0 = 0.0;
         d1 = 0.0;
-        spmv_rows<2>(w, r0, r1, w.shat, w.t, d0, d1);
+        spmv_rows<2, WIDE>(w, r0, r1, w.shat, w.t, d0, d1);
         double v2[2] = {d0, d1};
         write_partials<2>(v2, part[pb], lc, smem);
         if (!group_barrier(bar, nct, w.dflags)) return false;
@@ -1436,6 +1538,7 @@ __device__ bool solve_tissue(const KrylovWork& w, const BatchPlan& plan, int t, 
 // or (r, z) <= 0 before convergence (J or M not positive definite) the tissue's status is
 // KS_INDEFINITE and the host finishes it with BiCGStab from the iterate reached. Returns false when a group barrier
 // timed out.
+template <bool WIDE>
 __device__ bool solve_tissue_cg(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase, double rtol,
                                 int max_iter, double* smem, double* sb, double* red, double* ys, double* Ms, double* cs,
                                 float* cinv_s, bool& indefinite) {
@@ -1530,7 +1633,7 @@ __device__ bool solve_tissue_cg(const KrylovWork& w, const BatchPlan& plan, int 
         if (!group_barrier(bar, nct, w.dflags)) return false;
         // q = J p, (p, q)
         double d0 = 0.0, d1 = 0.0;
-        spmv_rows<3>(w, r0, r1, w.p, w.v, d0, d1);
+        spmv_rows<3, WIDE>(w, r0, r1, w.p, w.v, d0, d1);
         v1[0] = d0;
         write_partials<1>(v1, part[pb], lc, smem);
         if (!group_barrier(bar, nct, w.dflags)) return false;
@@ -1601,6 +1704,7 @@ __device__ bool solve_tissue_cg(const KrylovWork& w, const BatchPlan& plan, int 
 // the SpMV with (v, A v) and (v, r1), after r2 / z with (r2, z). Stops when the preconditioned
 // residual estimate phibar <= rtol phibar_0 (the host reports phibar / phibar_0 as the relative
 // residual). Returns false when a group barrier timed out.
+template <bool WIDE>
 __device__ bool solve_tissue_minres(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase, double rtol,
                                     int max_iter, double* smem, double* sb) {
     if (!plan.active[t]) return true;
@@ -1649,7 +1753,7 @@ __device__ bool solve_tissue_minres(const KrylovWork& w, const BatchPlan& plan, 
     }
     while (status == KS_RUNNING) {
         double d0 = 0.0, d1 = 0.0;
-        spmv_rows<4>(w, r0, r1, w.p, w.v, d0, d1);
+        spmv_rows<4, WIDE>(w, r0, r1, w.p, w.v, d0, d1);
         double v3[2] = {d0, d1};
         write_partials<2>(v3, part[pb], lc, smem);
         if (!group_barrier(bar, nct, w.dflags)) return false;
@@ -1735,22 +1839,43 @@ __device__ bool solve_tissue_minres(const KrylovWork& w, const BatchPlan& plan, 
     return true;
 }
 
-// Two builds of the persistent solve: one 768-thread CTA per SM (single tissues with the
-// two-level preconditioner, large tissues; up to 80 registers) and four 256-thread CTAs per SM
+// Two builds of the persistent solve: one 640-thread CTA per SM (single tissues with the
+// two-level preconditioner, large tissues; up to 96 registers) and four 256-thread CTAs per SM
 // (batches, small block-Jacobi tissues; registers capped at 64 so that 32 warps per SM hide the
 // latency of the memory-bound batched solve).
 // METHOD: 0 BiCGStab, 1 conjugate gradients, 2 MINRES (each its own build, so none pays the
-// others' registers).
+// others' registers). The narrow builds call their solves: inlined twice, the 64 registers spill 2 KB of loads.
+__device__ __noinline__ bool narrow_cg(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase, double rtol,
+                                       int max_iter, double* smem, double* sb, double* red, double* ys, double* Ms, double* cs,
+                                       float* cinv_s, bool& indefinite) {
+    return solve_tissue_cg<false>(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s, indefinite);
+}
+__device__ __noinline__ bool narrow_minres(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase, double rtol,
+                                           int max_iter, double* smem, double* sb) {
+    return solve_tissue_minres<false>(w, plan, t, lc, pbase, rtol, max_iter, smem, sb);
+}
+__device__ __noinline__ bool narrow_bicgstab(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase, double rtol,
+                                             int max_iter, double* smem, double* sb, double* red, double* ys, double* Ms,
+                                             double* cs, float* cinv_s) {
+    return solve_tissue<false>(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s);
+}
+
 template <int THREADS, int MIN_BLOCKS, int METHOD>
 __device__ __forceinline__ bool solve_by(const KrylovWork& w, const BatchPlan& plan, int t, int lc, int pbase,
                                          double rtol, int max_iter, double* smem, double* sb, double* red, double* ys,
                                          double* Ms, double* cs, float* cinv_s) {
+    constexpr bool wide = THREADS > 256;
     if (METHOD == 1) {
         bool indefinite = false;
-        return solve_tissue_cg(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s, indefinite);
+        if (wide) return solve_tissue_cg<true>(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s, indefinite);
+        return narrow_cg(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s, indefinite);
     }
-    if (METHOD == 2) return solve_tissue_minres(w, plan, t, lc, pbase, rtol, max_iter, smem, sb);
-    return solve_tissue(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s);
+    if (METHOD == 2) {
+        if (wide) return solve_tissue_minres<true>(w, plan, t, lc, pbase, rtol, max_iter, smem, sb);
+        return narrow_minres(w, plan, t, lc, pbase, rtol, max_iter, smem, sb);
+    }
+    if (wide) return solve_tissue<true>(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s);
+    return narrow_bicgstab(w, plan, t, lc, pbase, rtol, max_iter, smem, sb, red, ys, Ms, cs, cinv_s);
 }
 
 template <int THREADS, int MIN_BLOCKS, int METHOD>
@@ -2158,15 +2283,15 @@ cudaError_t launch_symmetrize(double* m, int n, int ld, long long stride, int co
 
 namespace {
 void (*persist_kernel(int threads, int method))(KrylovWork, BatchPlan, double, int) {
-    if (method == 2) return threads == 768 ? k_bicgstab_batched<768, 1, 2> : k_bicgstab_batched<256, 4, 2>;
-    if (method == 1) return threads == 768 ? k_bicgstab_batched<768, 1, 1> : k_bicgstab_batched<256, 4, 1>;
-    return threads == 768 ? k_bicgstab_batched<768, 1, 0> : k_bicgstab_batched<256, 4, 0>;
+    if (method == 2) return threads == kPersistWide ? k_bicgstab_batched<kPersistWide, 1, 2> : k_bicgstab_batched<256, 4, 2>;
+    if (method == 1) return threads == kPersistWide ? k_bicgstab_batched<kPersistWide, 1, 1> : k_bicgstab_batched<256, 4, 1>;
+    return threads == kPersistWide ? k_bicgstab_batched<kPersistWide, 1, 0> : k_bicgstab_batched<256, 4, 0>;
 }
 }  // namespace
 
 int persistent_max_grid(int device, int threads) {
     int sms = 0, occ = 0;
-    if (threads != 256 && threads != 768) return 0;
+    if (threads != 256 && threads != kPersistWide) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
     occ = 1 << 30;
     for (int method = 0; method < 3; ++method) {  // every method's build must fit the same plan
@@ -2176,14 +2301,14 @@ int persistent_max_grid(int device, int threads) {
             return 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, threads, 0) != cudaSuccess) return 0;
         occ = o < occ ? o : occ;
-        if (threads == 768) {  // the two-level solve adds its coarse row block: still one CTA per SM
+        if (threads == kPersistWide) {  // the two-level solve adds its coarse row block: still one CTA per SM
             int occ_c = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, kern, threads, kCoarseSmemBytes) != cudaSuccess ||
                 occ_c < 1)
                 return 0;
         }
     }
-    const int want = threads == 768 ? 1 : 4;  // the CTAs per SM each build is compiled for
+    const int want = threads == kPersistWide ? 1 : 4;  // the CTAs per SM each build is compiled for
     return sms * (occ < want ? occ : want);
 }
 
@@ -2194,7 +2319,7 @@ cudaError_t launch_bicgstab_batched(const KrylovWork& w, const BatchPlan& plan, 
     void* args[] = {&wc, &pc, &rtol, &max_iter};
     const size_t smem = plan.agg_per_cta > 0 ? sizeof(float) * 6 * plan.agg_per_cta * (size_t)plan.n_coarse : 0;
     if (smem > (size_t)kCoarseSmemBytes) return cudaErrorInvalidValue;
-    if (threads != 256 && threads != 768) return cudaErrorInvalidValue;
+    if (threads != 256 && threads != kPersistWide) return cudaErrorInvalidValue;
     const int method = plan.minres ? 2 : (plan.cg ? 1 : 0);
     return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(persist_kernel(threads, method)), dim3(plan.n_cta),
                                        dim3(threads), args, smem, s);
