@@ -174,3 +174,31 @@ def test_set_growth_rejects_singular_tensors_and_keeps_the_inverse(bad):
         with pytest.raises(capi.TFError):
             s.set_growth(fg=wrong)
         assert np.array_equal(s.get_growth()[1].reshape(-1, 3, 3), inv)
+
+
+@pytest.mark.parametrize("rows", [(0, 1), (1, 2), (0, 2)])
+def test_set_growth_rejects_a_tensor_with_two_equal_rows(rows):
+    """Its determinant is zero where every product is rounded (the other minors cancel exactly), but not where the
+    products are contracted into fused operations."""
+    t = mesh.small_disc(5, 301, 1000.0)
+    rng = np.random.default_rng(7)
+    fg = np.tile(np.eye(3), (t.n_elems, 1, 1)) + rng.uniform(-0.1, 0.1, (t.n_elems, 3, 3))
+    i, j = rows
+
+    def det(m):
+        m = m.reshape(9)
+        return (m[0] * (m[4] * m[8] - m[5] * m[7]) - m[1] * (m[3] * m[8] - m[5] * m[6])) + m[2] * (m[3] * m[7] - m[4] * m[6])
+
+    with NewtonRaphsonSolver.from_tissue(t) as s:
+        refused = 0
+        for _ in range(20):
+            wrong = fg.copy()
+            wrong[-1] = rng.uniform(0.5, 1.5, (3, 3))
+            wrong[-1, j] = wrong[-1, i]
+            if det(wrong[-1]) == 0.0:
+                refused += 1
+                with pytest.raises(capi.TFError):
+                    s.set_growth(fg=wrong)
+            else:
+                s.set_growth(fg=wrong)
+        assert refused > 0

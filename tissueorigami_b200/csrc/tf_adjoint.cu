@@ -261,10 +261,12 @@ __global__ void k_set_inv_fg(ElemRecord* elems, int32_t n_elems, const double* f
 __global__ void k_check_fg(int32_t n_elems, const double* fg, int32_t* flag) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_elems) return;
-    double m[3][3];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) m[i][j] = fg[(size_t)e * 9 + i * 3 + j];
-    const double det = det3(m);
+    const double* m = fg + (size_t)e * 9;
+    // every product rounded: contracted, the determinant of a tensor with two equal rows is not zero
+    auto minor = [](double a, double b, double c, double d) { return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d)); };
+    const double det = __dadd_rn(__dsub_rn(__dmul_rn(m[0], minor(m[4], m[8], m[5], m[7])),
+                                           __dmul_rn(m[1], minor(m[3], m[8], m[5], m[6]))),
+                                 __dmul_rn(m[2], minor(m[3], m[7], m[4], m[6])));
     if (det == 0.0 || !isfinite(det)) *flag = 1;
 }
 
