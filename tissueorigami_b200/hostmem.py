@@ -1,6 +1,6 @@
 """Page-locked memory for large result arrays.
 
-A device-to-host copy into fresh pageable memory is bound by its page faults and by the driver's staging
+A device-to-host copy into fresh pageable memory is bound by its page faults and by CUDA's staging
 (14 MB of Jacobian: 2.1 ms, 0.28 ms into page-locked memory). Results of at least 1 MB therefore live in
 page-locked blocks that go back to a bounded pool when the last view of the array is gone.
 """
