@@ -72,6 +72,28 @@ def test_factorised_solve_of_an_indefinite_system():
         assert np.linalg.norm(du - ref) <= 1e-8 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("share", [0.02, 0.3])
+def test_negative_pivots_in_some_panels_of_a_front(share):
+    """Fronts of several 64-pivot panels (the root of 9,000 prisms has six), some of them with negative pivots and
+    some without, beside fronts with none: every panel's update takes its own signs. Five solves of one
+    system are equal to the last bit."""
+    t = mesh.small_disc(3, 9000, 800.0)
+    vals, g, _ = _system(t)
+    rowptr, colidx = O.block_pattern(t)
+    free = np.nonzero(t.fixed.sum(axis=1) == 0)[0]
+    node = np.random.default_rng(5).choice(free, int(share * len(free)), replace=False)
+    rows = np.repeat(np.arange(t.n_nodes), np.diff(rowptr))
+    vals[(rows == colidx) & np.isin(rows, node)] *= -1.0
+    ref = sla.spsolve(O.bsr_to_scipy(rowptr, colidx, vals, t.n_nodes).tocsc(), g)
+    with NewtonRaphsonSolver.from_tissue(t, krylov_rtol=1e-13) as s:
+        first, rc, iters, rr = s.solveForDeltaU(vals, g)
+        assert rc == capi.TF_OK and rr <= 1e-13 and iters <= 4
+        assert s.preconditioner()[2] == 1
+        for _ in range(4):
+            assert np.array_equal(s.solveForDeltaU(vals, g)[0], first)
+    assert np.linalg.norm(first - ref) <= 1e-8 * np.linalg.norm(ref)
+
+
 def test_singular_system_falls_back():
     """A free node cut off from everything (zero row and column): a zero pivot. The call returns what the
     iterative path makes of it, without a non-finite du on the other nodes."""
