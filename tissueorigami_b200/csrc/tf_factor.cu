@@ -1164,8 +1164,8 @@ __global__ void __launch_bounds__(256) k_fc_cg_spmv(KrylovWork w, FcCg c, const 
     __shared__ double smem[8];
     chain_go();
     const FcChunk ch = c.chunks[blockIdx.x];
-    const int k0 = w.rowptr[ch.row0], k1 = w.rowptr[ch.row1];
-    for (int o = k0 * 9 + (int)threadIdx.x * 16; o < k1 * 9; o += 256 * 16) prefetch(w.vals + o);  // J is older than the chain
+    const FcSpan js = fc_block_span(w.rowptr[ch.row0], w.rowptr[ch.row1]);
+    for (int64_t o = js.begin + threadIdx.x * 16; o < js.end; o += 256 * 16) prefetch(w.vals + o);  // J is older than the chain
     chain_wait();
     if (!c.running[ch.tissue]) return;
     const double* pv = FIRST ? z : w.p;

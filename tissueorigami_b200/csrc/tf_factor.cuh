@@ -146,6 +146,13 @@ inline int fc_chunk_rows(int n_nodes) {
     return r < 32 ? 32 : (r > 256 ? 256 : r);
 }
 
+// The doubles [begin, end) of the Jacobian blocks [k0, k1). In 64 bits: 32 end at 238.6 million blocks, a batch
+// of 243 full wing discs (17 GB of values beside 126 GB of factors).
+struct FcSpan {
+    int64_t begin, end;
+};
+__host__ __device__ inline FcSpan fc_block_span(int32_t k0, int32_t k1) { return {(int64_t)k0 * 9, (int64_t)k1 * 9}; }
+
 struct FcCg {
     int n_chunks, T;
     const FcChunk* chunks;
