@@ -1968,7 +1968,7 @@ int krylov_solve(tf_ctx* ctx) {
         const size_t bytes3 = sizeof(double) * 3 * (size_t)ctx->N;
         const int wk = ctx->warm_k;
         const bool warm_slot = ctx->params.krylov_warm_start && ctx->T == 1 && plan.cg && !plan.minres &&
-                               !ctx->reuse_precond && wk >= 0 && wk < kWarmSlots;
+                               wk >= 0 && wk < kWarmSlots;
         if (warm_slot && wk < (int)ctx->warm_valid.size() && ctx->warm_valid[wk]) {
             TF_CK(cudaMemcpyAsync(ctx->du.p, ctx->warm_hist[wk].p, bytes3, cudaMemcpyDeviceToDevice, ctx->stream));
             TF_CK(launch_residual(w, dptr<double>(ctx->du), dptr<double>(ctx->g), dptr<double>(ctx->r), ctx->stream));
@@ -2320,7 +2320,7 @@ int call_end(tf_ctx* ctx, tf_step_stats* st) {
 // The Newton system's solve: J du = g, and with a lumen (J + a G G^T) du = g by Sherman-Morrison
 // from two solves with the sparse J: y = J^-1 g, z = J^-1 G, du = y - a (G.y) / (1 + a G.z) z,
 // a = bulk / (36 V0^2) (the rank-one term of Lumen::calculateJacobian couples every lumen node,
-// so it stays out of the sparse J). The second solve reuses the first one's preconditioner; the
+// so it stays out of the sparse J). The second solve reuses the first one's preconditioner or factor; the
 // scalars left for the Newton loop carry both solves' iterations and the worse status.
 int newton_solve(tf_ctx* ctx) {
     int rc = krylov_solve(ctx);
@@ -2330,11 +2330,16 @@ int newton_solve(tf_ctx* ctx) {
     TF_CK(cudaMemcpyAsync(ctx->lm_y_d.p, ctx->du.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     TF_CK(cudaMemcpyAsync(ctx->lm_gsave_d.p, ctx->g.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     TF_CK(cudaMemcpyAsync(ctx->g.p, ctx->lm_G_d.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    ctx->reuse_precond = true;
-    ctx->fc_same = ctx->fc_used;  // the factor is of this J
+    // A factorised first solve leaves its factor: of this J, or (fc_near) of an earlier one, which a right-hand
+    // side it does not serve replaces as in any other solve. It set up no iterative preconditioner.
+    const int warm_k = ctx->warm_k;
+    ctx->warm_k = -1;  // another right-hand side
+    ctx->reuse_precond = !ctx->fc_used;
+    ctx->fc_same = ctx->fc_used && !ctx->fc_near;
     rc = krylov_solve(ctx);
     ctx->fc_same = false;
     ctx->reuse_precond = false;
+    ctx->warm_k = warm_k;
     if (rc != TF_OK) return rc;
     TF_CK(cudaMemcpyAsync(ctx->lm_z_d.p, ctx->du.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     TF_CK(launch_dot2(3 * ctx->N, dptr<double>(ctx->lm_G_d), dptr<double>(ctx->lm_y_d), dptr<double>(ctx->lm_z_d),
