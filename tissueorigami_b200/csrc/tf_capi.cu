@@ -1907,12 +1907,12 @@ int factor_solve(tf_ctx* ctx, bool* done) {
 // ctx->h_tsc[T] (persistent) or ctx->h_sc (chunked, single tissue).
 int krylov_solve(tf_ctx* ctx) {
     KrylovWork w = make_work(ctx);
+    ctx->fc_used = false;
     if (use_persistent(ctx) && factor_wanted(ctx)) {
         if (ctx->fc_dirty) {
             const int frc = build_factor(ctx);
             if (frc != TF_OK) return frc;
         }
-        ctx->fc_used = false;
         if (ctx->fc_ready) {
             const int frc = factor_solve(ctx, &ctx->fc_used);
             if (frc != TF_OK || ctx->fc_used) return frc;
