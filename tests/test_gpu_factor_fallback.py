@@ -2,9 +2,11 @@
 Jacobian is replaced, a system it cannot solve goes to the iterative solve, the others stay with it."""
 import numpy as np
 import pytest
+import scipy.sparse.linalg as sla
 
+from oracle import oracle as O
 from tissueorigami_b200 import capi, mesh
-from tissueorigami_b200.newton import NewtonRaphsonSolver
+from tissueorigami_b200.newton import BatchSolver, NewtonRaphsonSolver
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +63,93 @@ def test_packing_pairs_that_come_and_go_on_one_solver():
     for a, b in zip(one, alone):
         assert a[1:] == b[1:]
         assert np.abs(a[0] - b[0]).max() <= 1e-9 * t.size
+
+
+def _system(t):
+    """(values, right-hand side) of the oracle's first Newton iteration, and the block pattern."""
+    _, inv, _, _ = O.grow(t, t.x, t.fg)
+    rowptr, colidx = O.block_pattern(t)
+    vals, g = O.assemble_bsr(t, t.x, t.x, O.viscosity_surfaces(t, t.x), inv, rowptr, colidx)
+    return vals, g, rowptr, colidx
+
+
+def _cut_off(t, vals, g, rowptr, colidx):
+    """The system with one free node's rows, columns and forces zero (a zero pivot, and a solution all the same),
+    and the solution on the other unknowns (the node's own are free): their indices and values."""
+    node = int(np.nonzero(t.fixed.sum(axis=1) == 0)[0][3])
+    rows = np.repeat(np.arange(t.n_nodes), np.diff(rowptr))
+    vals, g = vals.copy(), g.copy()
+    vals[(rows == node) | (colidx == node)] = 0.0
+    g[3 * node:3 * node + 3] = 0.0
+    keep = np.setdiff1d(np.arange(3 * t.n_nodes), 3 * node + np.arange(3))
+    J = O.bsr_to_scipy(rowptr, colidx, vals, t.n_nodes).tocsc()
+    return vals, g, keep, sla.spsolve(J[keep][:, keep], g[keep])
+
+
+def test_singular_system_is_left_to_the_iterative_solve():
+    """The factorisation meets a zero pivot; the conjugate gradients that follow do not: the solution of the rest
+    within 1e-8 of SuperLU's (a residual of 1e-13 and condition numbers up to ~1e5). The next system of the same solver is a factorised one again."""
+    t = mesh.small_disc(7, 700, 1200.0)
+    vals, g, rowptr, colidx = _system(t)
+    with NewtonRaphsonSolver.from_tissue(t, krylov_rtol=1e-13) as s:
+        good, rc, it, _ = s.solveForDeltaU(vals, g)
+        root = s.preconditioner()[1]
+        assert rc == capi.TF_OK and it <= 3 and root > 0
+        v, b, keep, ref = _cut_off(t, vals, g, rowptr, colidx)
+        du, rc, it, rr = s.solveForDeltaU(v, b)
+        assert rc == capi.TF_OK and rr <= 1e-13 and it > 3
+        assert s.preconditioner()[1] != root
+        assert np.all(np.isfinite(du)) and np.linalg.norm(du[keep] - ref) <= 1e-8 * np.linalg.norm(ref)
+        again, rc, _, _ = s.solveForDeltaU(vals, g)
+        assert rc == capi.TF_OK and s.preconditioner()[1] == root
+        assert np.array_equal(again, good)
+
+
+@pytest.mark.parametrize("bad", [[0], [1], [2, 3], [0, 1, 2, 3]])
+def test_tissues_of_a_batch_whose_factor_fails_leave_the_others_alone(bad):
+    """Some tissues of a batch with a zero pivot: the others' solutions equal, to the last bit, those of the batch
+    without it; the bad ones' come from the iterative solve (1e-8 of SuperLU's as above)."""
+    ts = [mesh.small_disc(50 + i, n, 900.0) for i, n in enumerate([700, 1500, 333, 1201])]
+    sys = [_system(t) for t in ts]
+    cut = [_cut_off(t, *s) for t, s in zip(ts, sys)]
+    cat = np.concatenate
+    with BatchSolver(ts, krylov_rtol=1e-13) as b:
+        good, rc, _, _ = b.solveForDeltaU(cat([s[0] for s in sys]), cat([s[1] for s in sys]))
+        assert rc == capi.TF_OK
+        du, rc, _, _ = b.solveForDeltaU(cat([(cut if i in bad else sys)[i][0] for i in range(4)]),
+                                        cat([(cut if i in bad else sys)[i][1] for i in range(4)]))
+        assert rc == capi.TF_OK
+        good, du = b.split(good), b.split(du)
+    for i in range(4):
+        if i in bad:
+            keep, ref = cut[i][2:]
+            assert np.linalg.norm(du[i].reshape(-1)[keep] - ref) <= 1e-8 * np.linalg.norm(ref)
+        else:
+            assert np.array_equal(du[i], good[i])
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_a_factor_that_fails_is_not_tried_again_in_the_step(batch):
+    """A node that nothing holds (no stiffness around it, no drag): every Newton iteration has a zero pivot. The
+    step factorises that tissue once; the other Newton iterations go to the iterative solve at once. Equal
+    Newton counts and positions (1e-9 of the size) to steps of that solve alone."""
+    t = mesh.small_disc(7, 700, 1200.0)
+    node = int(np.nonzero(t.fixed.sum(axis=1) == 0)[0][40])
+    around = (t.conn == node).any(axis=1)
+    t.lam[around] = t.mu[around] = 0.0
+    t.ext_visc.reshape(-1, 3)[node] = 0.0
+    other = mesh.small_disc(8, 900, 1000.0)
+    out = {}
+    for warm in (1, 0):  # 0: no factor
+        make = (lambda **kw: BatchSolver([other, t], **kw)) if batch else (lambda **kw: NewtonRaphsonSolver.from_tissue(t, **kw))
+        with make(krylov_rtol=1e-13, krylov_warm_start=warm) as s:
+            x0 = s.join([other.x, t.x]) if batch else t.x
+            x, rc, st = s.runOneStep(x0, t.dt)
+            assert rc == capi.TF_OK and st["newton_iters"] >= 4
+            out[warm] = (x, st["newton_iters"], st["solve_launches"], s.preconditioner()[2])
+    a, b = out[1], out[0]
+    assert a[1] == b[1] and a[2] == b[2]  # every Newton iteration has its iterative solve
+    # refreshes: coarse operators as without a factor, and factorisations: one, or for a batch one per
+    # Newton iteration (the other tissue's)
+    assert a[3] <= b[3] + (a[1] if batch else 1)
+    assert np.abs(a[0] - b[0]).max() <= 1e-9 * t.size

@@ -182,6 +182,7 @@ struct tf_ctx {
     bool fc_used = false;      // the last solve was a factorised one
     bool fc_same = false;      // the factor on the device is of the current J (further right-hand sides)
     bool fc_near = false;      // ... or of the J of an earlier iteration of this Newton loop, close to it
+    std::vector<char> fc_failed;  // [T] tissues the factor failed in this call: the iterative solve takes them
     std::vector<int32_t> fc_chunk0;
     // the launches of a factorisation and of a solve are the same every time (50 to 300 short kernels
     // whose launch alone, 3.4 us each, took longer than many of them): replayed as graphs (0.75 us each)
@@ -1840,12 +1841,24 @@ FcWork make_factor(tf_ctx* c) {
 
 // One factorised solve of every active tissue: conjugate gradients from zero whose preconditioner is
 // the factor of J, so that one or two iterations meet the tolerance (the residual's recurrence is
-// the refinement). *done = false when a tissue did not get there (a zero pivot, a non-finite
-// value, an ill-conditioned J): the caller solves them all again by the iterative path.
-int factor_solve(tf_ctx* ctx, bool* done) {
-    *done = false;
+// the refinement). left[t] = 1 for an active tissue that did not get there (a zero pivot, a non-finite
+// value, an ill-conditioned J), now or earlier in this call: the caller solves it by the iterative path.
+int factor_solve(tf_ctx* ctx, std::vector<int32_t>& left) {
+    const int T = ctx->T;
     const int cap = std::min(kFcMaxIters, ctx->params.krylov_max_iters);
-    if (cap < 1) return TF_OK;
+    ctx->fc_failed.resize(T, 0);
+    left.assign(T, 0);
+    std::vector<int32_t> mine(T, 0);
+    bool any = false, failed = false;
+    for (int t = 0; t < T; ++t) {
+        if (T > 1 && !ctx->h_active[t]) continue;
+        const bool out = ctx->fc_failed[t] != 0;
+        (out ? left : mine)[t] = 1;
+        (out ? failed : any) = true;
+    }
+    if (!any) return TF_OK;
+    if (failed)
+        TF_CK(cudaMemcpyAsync(ctx->active_d.p, mine.data(), sizeof(int32_t) * T, cudaMemcpyHostToDevice, ctx->stream));
     const KrylovWork w = make_work(ctx);
     FcWork f = make_factor(ctx);
     FcCg c;
@@ -1878,28 +1891,33 @@ int factor_solve(tf_ctx* ctx, bool* done) {
         if (rc != TF_OK) return rc;
         TF_CK(cudaStreamSynchronize(ctx->stream));
         running = false;
-        for (int t = 0; t < ctx->T; ++t)
-            if (ctx->T == 1 || ctx->h_active[t]) {
-                const int st = ctx->h_tsc[t].status;
-                if (st == KS_RUNNING)
-                    running = true;
-                else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters)) {
-                    if (!ctx->fc_near) return TF_OK;
-                    ctx->fc_near = false;  // the kept factor does not fit: with one of this J
-                    return factor_solve(ctx, done);
+        for (int t = 0; t < T; ++t) {
+            if (!mine[t] || left[t]) continue;
+            const int st = ctx->h_tsc[t].status;
+            if (st == KS_RUNNING) {
+                running = true;
+            } else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters)) {
+                if (ctx->fc_near) {  // the kept factor does not fit: with one of this J
+                    ctx->fc_near = false;
+                    return factor_solve(ctx, left);
                 }
+                ctx->fc_failed[t] = 1;
+                left[t] = 1;
+                failed = true;
             }
+        }
     }
+    ctx->fc_used = !failed;
+    if (failed) return TF_OK;  // the iterative solve of the others adds up for all of them
     *ctx->h_sc = ctx->h_tsc[0];
     ctx->last_solve_iters = 0;
-    for (int t = 0; t < ctx->T; ++t)
-        if (ctx->T == 1 || ctx->h_active[t]) {
+    for (int t = 0; t < T; ++t)
+        if (mine[t]) {
             ctx->last_method = std::max<int32_t>(ctx->last_method, ctx->h_tsc[t].method);
             if (!c.minres) ctx->cg_iters += ctx->h_tsc[t].iter;
             ctx->last_solve_iters = std::max(ctx->last_solve_iters, ctx->h_tsc[t].iter);
         }
     ctx->last_solve_method = c.minres ? KM_MINIMAL_RESIDUAL : KM_CG;
-    *done = true;
     return TF_OK;
 }
 
@@ -1908,14 +1926,17 @@ int factor_solve(tf_ctx* ctx, bool* done) {
 int krylov_solve(tf_ctx* ctx) {
     KrylovWork w = make_work(ctx);
     ctx->fc_used = false;
+    std::vector<int32_t> left;  // tissues the factor left to the iterative solve (empty: it did not run)
     if (use_persistent(ctx) && factor_wanted(ctx)) {
         if (ctx->fc_dirty) {
             const int frc = build_factor(ctx);
             if (frc != TF_OK) return frc;
         }
         if (ctx->fc_ready) {
-            const int frc = factor_solve(ctx, &ctx->fc_used);
+            const int frc = factor_solve(ctx, left);
             if (frc != TF_OK || ctx->fc_used) return frc;
+            if (ctx->T > 1)  // the others keep their results
+                TF_CK(cudaMemcpyAsync(ctx->active_d.p, left.data(), sizeof(int32_t) * ctx->T, cudaMemcpyHostToDevice, ctx->stream));
         }
     }
     if (use_persistent(ctx)) {
@@ -2047,6 +2068,8 @@ int krylov_solve(tf_ctx* ctx) {
                     }
             }
         }
+        if (ctx->T > 1 && !left.empty())
+            TF_CK(cudaMemcpyAsync(ctx->active_d.p, ctx->h_active, sizeof(int32_t) * ctx->T, cudaMemcpyHostToDevice, ctx->stream));
         *ctx->h_sc = ctx->h_tsc[0];
         if (warm_slot && ctx->h_tsc[0].status == KS_CONVERGED) {
             if ((int)ctx->warm_hist.size() <= wk) {
@@ -2172,6 +2195,7 @@ int newton_core(tf_ctx* ctx, double dt, tf_step_stats* st) {
     ctx->t_status.assign(T, TF_OK);
     ctx->t_krylov.assign(T, 0);
     for (int t = 0; t < T; ++t) ctx->h_active[t] = 1;
+    ctx->fc_failed.assign(T, 0);
     const bool persistent = use_persistent(ctx);
     int n_active = T;
     int round = 0;
@@ -2405,6 +2429,7 @@ int prologue(tf_ctx* ctx, double dt) {
 // Mark every tissue active on the device (the parity hooks and timers act on all tissues).
 int activate_all(tf_ctx* ctx) {
     for (int t = 0; t < ctx->T; ++t) ctx->h_active[t] = 1;
+    ctx->fc_failed.assign(ctx->T, 0);
     TF_CK(cudaMemcpyAsync(ctx->active_d.p, ctx->h_active, sizeof(int32_t) * ctx->T, cudaMemcpyHostToDevice, ctx->stream));
     return ctx->T > 1 ? build_plan_all(ctx) : TF_OK;
 }
