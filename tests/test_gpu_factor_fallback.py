@@ -153,3 +153,36 @@ def test_a_factor_that_fails_is_not_tried_again_in_the_step(batch):
     # Newton iteration (the other tissue's)
     assert a[3] <= b[3] + (a[1] if batch else 1)
     assert np.abs(a[0] - b[0]).max() <= 1e-9 * t.size
+
+
+def test_without_memory_for_the_factor_the_steps_are_iterative():
+    """Device memory held back until only so much is left, around every point at which one of the factor's buffers
+    no longer fits: the step succeeds all the same, equal Newton counts and positions (1e-9 of the size)."""
+    import torch
+
+    t = mesh.wing_disc(n_surface_points=6000)
+    mb = 1 << 20
+
+    def step(left=None):
+        with NewtonRaphsonSolver.from_tissue(t, krylov_rtol=1e-13) as s:
+            free = torch.cuda.mem_get_info()[0]
+            hold = torch.empty(free - left, dtype=torch.uint8, device="cuda") if left else None
+            free = torch.cuda.mem_get_info()[0]
+            x, rc, st = s.runOneStep(t.x, t.dt)
+            used = free - torch.cuda.mem_get_info()[0]
+        del hold
+        torch.cuda.empty_cache()
+        assert rc == capi.TF_OK
+        return x, st["newton_iters"], st["solve_launches"], used
+
+    with NewtonRaphsonSolver.from_tissue(t, krylov_warm_start=0) as s:  # the iterative kernels' local memory is the process's
+        s.runOneStep(t.x, t.dt)
+    step()
+    x, its, launches, used = step()
+    assert launches == 0 and used > 100 * mb
+    ways = []
+    for left in [3 * used, 2 * used + 8 * mb, 2 * used - 8 * mb] + [used + k * mb for k in range(4, -13, -2)]:
+        y, n, launches, _ = step(left)
+        assert n == its and np.abs(y - x).max() <= 1e-9 * t.size
+        ways.append(launches > 0)
+    assert not ways[0] and all(ways[3:])

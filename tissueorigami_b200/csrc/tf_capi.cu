@@ -1735,10 +1735,33 @@ int replay_factor(tf_ctx* ctx, int which, F launch) {
 
 FcWork make_factor(tf_ctx* c);
 
+// Gives back all that a factorisation holds on the device; its solves take the iterative path until the next plan.
+void release_factor(tf_ctx* c) {
+    if (c->stream) cudaStreamSynchronize(c->stream);
+    drop_factor_graphs(c);
+    DevBuf* b[] = {&c->fc_fronts, &c->fc_maps, &c->fc_verts, &c->fc_jblk, &c->fc_jblk_t, &c->fc_tasks, &c->fc_factor,
+                   &c->fc_scratch, &c->fc_contrib[0], &c->fc_contrib[1], &c->fc_kids, &c->fc_dofs, &c->fc_vec, &c->fc_z,
+                   &c->fc_sign, &c->fc_flags, &c->fc_neg, &c->fc_chunks, &c->fc_chunk0_d, &c->fc_running, &c->fc_part};
+    for (DevBuf* q : b) dfree(*q);
+    c->fc = FcPlan();
+    c->fc_ready = false;
+}
+
+int lay_out_factor(tf_ctx* ctx);
+
+// The plan of the current pattern and its buffers; without memory for them, none (fc_ready = false).
 int build_factor(tf_ctx* ctx) {
     ctx->fc_dirty = false;
     ctx->fc_ready = false;
     drop_factor_graphs(ctx);
+    const int rc = lay_out_factor(ctx);
+    if (!ctx->fc_ready) release_factor(ctx);
+    if (rc != TF_ERR_OUT_OF_MEMORY) return rc;
+    ctx->last_error[0] = 0;
+    return TF_OK;
+}
+
+int lay_out_factor(tf_ctx* ctx) {
     const int N = ctx->N, T = ctx->T;
     int G = std::max(ctx->col_G, 1);
     for (int t = 0; t < T; ++t)
@@ -1768,20 +1791,20 @@ int build_factor(tf_ctx* ctx) {
         if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(b.p, h, bytes, cudaMemcpyHostToDevice, ctx->stream);
         return e;
     };
-    cudaError_t e = room(ctx->fc_factor, P.n_factor + 64);  // the downward pass reads past the last row's columns
-    if (e == cudaSuccess) e = room(ctx->fc_scratch, P.n_scratch);
-    for (int q = 0; q < 2; ++q)
-        if (e == cudaSuccess) e = room(ctx->fc_contrib[q], P.n_contrib[q]);
-    if (e == cudaSuccess) e = room(ctx->fc_vec, P.n_vec);
-    if (e == cudaSuccess) e = room(ctx->fc_z, P.n_piv);
-    if (e == cudaSuccess) e = room(ctx->fc_sign, P.n_piv);
-    if (e == cudaSuccess) e = room(ctx->fc_part, 3 * (int64_t)chunks.size());
-    if (e == cudaErrorMemoryAllocation) {  // no room for the factor: the iterative solve needs far less
-        (void)cudaGetLastError();
-        for (DevBuf* b : {&ctx->fc_factor, &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1]}) dfree(*b);
-        return TF_OK;
-    }
-    TF_CK(e);
+    // Not more than half of what is free: the iterative solve needs an eighth of it (24,000 prisms: 32 MB and
+    // 258), and a program that got by without a factor still has room for what it allocates later.
+    size_t free_bytes = 0, all_bytes = 0;
+    TF_CK(cudaMemGetInfo(&free_bytes, &all_bytes));
+    for (const DevBuf* b : {&ctx->fc_factor, &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1]}) free_bytes += b->bytes;
+    const int64_t doubles = P.n_factor + P.n_scratch + P.n_contrib[0] + P.n_contrib[1];
+    if (sizeof(double) * (size_t)doubles > free_bytes / 2) return TF_OK;
+    TF_CK(room(ctx->fc_factor, P.n_factor + 64));  // the downward pass reads past the last row's columns
+    TF_CK(room(ctx->fc_scratch, P.n_scratch));
+    for (int q = 0; q < 2; ++q) TF_CK(room(ctx->fc_contrib[q], P.n_contrib[q]));
+    TF_CK(room(ctx->fc_vec, P.n_vec));
+    TF_CK(room(ctx->fc_z, P.n_piv));
+    TF_CK(room(ctx->fc_sign, P.n_piv));
+    TF_CK(room(ctx->fc_part, 3 * (int64_t)chunks.size()));
     // the padding of the rows, and x11 above its diagonal blocks, stay zero: no kernel writes there
     TF_CK(cudaMemsetAsync(ctx->fc_factor.p, 0, sizeof(double) * (size_t)(P.n_factor + 64), ctx->stream));
     FcStreams& st = ctx->fc_streams;
@@ -1934,7 +1957,13 @@ int krylov_solve(tf_ctx* ctx) {
         }
         if (ctx->fc_ready) {
             const int frc = factor_solve(ctx, left);
-            if (frc != TF_OK || ctx->fc_used) return frc;
+            if (frc == TF_ERR_OUT_OF_MEMORY) {  // for its graphs: without a factor
+                release_factor(ctx);
+                ctx->last_error[0] = 0;
+                left.assign(ctx->h_active, ctx->h_active + ctx->T);
+            } else if (frc != TF_OK || ctx->fc_used) {
+                return frc;
+            }
             if (ctx->T > 1)  // the others keep their results
                 TF_CK(cudaMemcpyAsync(ctx->active_d.p, left.data(), sizeof(int32_t) * ctx->T, cudaMemcpyHostToDevice, ctx->stream));
         }
@@ -2760,11 +2789,7 @@ void tf_destroy(tf_ctx* ctx) {
                      &ctx->ml_first_cta_d, &ctx->ml_slot_a_d, &ctx->ml_out_ptr_d, &ctx->ml_out_slots_d,
                      &ctx->ml_out_set_d, &ctx->ml_out_col_d, &ctx->ml_out_dst_d, &ctx->ml_pairs_d, &ctx->ml_pos_leaf_d};
     for (DevBuf* b : mlb) dfree(*b);
-    DevBuf* fcb[] = {&ctx->fc_fronts, &ctx->fc_maps, &ctx->fc_verts, &ctx->fc_jblk, &ctx->fc_jblk_t, &ctx->fc_tasks, &ctx->fc_factor,
-                     &ctx->fc_scratch, &ctx->fc_contrib[0], &ctx->fc_contrib[1], &ctx->fc_kids, &ctx->fc_dofs, &ctx->fc_vec, &ctx->fc_z,
-                     &ctx->fc_sign, &ctx->fc_flags, &ctx->fc_neg, &ctx->fc_chunks, &ctx->fc_chunk0_d, &ctx->fc_running, &ctx->fc_part};
-    for (DevBuf* b : fcb) dfree(*b);
-    drop_factor_graphs(ctx);
+    release_factor(ctx);
     if (ctx->fc_streams.fork) cudaEventDestroy(ctx->fc_streams.fork);
     for (int q = 0; q < 3; ++q) {
         if (ctx->fc_streams.join[q]) cudaEventDestroy(ctx->fc_streams.join[q]);
