@@ -33,3 +33,27 @@ def host(tmp_path_factory):
 def test_offsets_of_jacobian_values_do_not_wrap(host, k):
     """Nine doubles a block: from block 2^31 / 9 on their offsets need more than 32 bits."""
     assert host("span", k, k + 1) == [str(9 * k), str(9 * (k + 1))]
+
+
+@pytest.mark.parametrize("limit", [1e8, 3e9, 3e11])
+@pytest.mark.parametrize("nx,ny", [(500, 250), (2000, 50)])
+def test_dissection_ends_where_the_limit_is_passed(host, nx, ny, limit):
+    """A tissue whose factorisation is too large is not dissected to the end: the operations counted by then exceed
+    the limit by no more than the root front's 2/3 p^3 (the largest front of such a sheet without boundary) and
+    the fronts of a depth below it (as much again, with their boundaries ten times)."""
+    ok, flops, _, fronts, _ = host("plan", nx, ny, 4, limit, 0, 1)
+    whole = float(host("plan", nx, ny, 4, 1e15, 0, 1)[1])
+    assert whole > 3e9
+    if whole <= limit:
+        assert ok == "1"
+        return
+    root = 2.0 / 3.0 * (12 * min(nx, ny)) ** 3
+    assert (ok, fronts) == ("0", "0") and limit < float(flops) <= limit + 10 * root and float(flops) < whole
+
+
+@pytest.mark.parametrize("sheet", [(1, 1, 1, 0), (3, 2, 2, 0), (31, 23, 4, 0), (40, 35, 3, 0), (40, 35, 1, 2), (60, 50, 2, 7),
+                                   (9, 300, 1, 1)])
+def test_boundaries_of_the_fronts(host, sheet):
+    """Every column a pivot of one front; every front's boundary what its subtree touches, also around a column
+    with hundreds of neighbours (found from the other side there)."""
+    assert host("check", *sheet) == ["1", "0"]

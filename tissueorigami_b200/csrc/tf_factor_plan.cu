@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <mutex>
 #include <numeric>
 #include <thread>
 
@@ -16,6 +17,23 @@ struct Node {
     std::vector<int32_t> piv, bnd;  // columns
     int depth = 0;
     int child[2] = {-1, -1};
+    int32_t lo = 0, hi = 0;  // its subtree's columns in perm
+};
+
+// Operations of the fronts of all tissues, against the limit.
+struct Budget {
+    double max_flops;
+    std::mutex lock;
+    double flops = 0.0;
+    std::atomic<bool> over{false};
+
+    // A front of np pivot and nb boundary columns of gd unknowns each.
+    void add(size_t np, size_t nb, int gd) {
+        const double p = (double)np * gd, b = (double)nb * gd;
+        std::lock_guard<std::mutex> hold(lock);
+        flops += p * p * p * (2.0 / 3.0) + p * p * b + b * b * p;
+        if (p > kFcMaxPivots || p + b > kFcMaxFront || flops > max_flops) over = true;
+    }
 };
 
 // Columns of one tissue: their graph (ptr / adj over local ids), positions, and the dissection.
@@ -23,7 +41,7 @@ struct Dissection {
     const int32_t* ptr;
     const int32_t* adj;
     const double* X;  // [n][3]
-    int leaf;
+    int leaf, gd;
     std::vector<Node> nodes;
     std::vector<int32_t> perm, label, match, seen, pos;
     int32_t next_label = 0, stamp = 0;
@@ -53,16 +71,14 @@ struct Dissection {
         }
     }
 
-    // Splits perm[lo, hi) in two halves across the longest side of its bounding box; the separator is
-    // a smallest set of columns that covers every block between the halves (a minimum vertex cover
-    // of the cut edges, from a maximum matching).
-    int split(int32_t lo, int32_t hi, int depth) {
-        const int id = (int)nodes.size();
-        nodes.emplace_back();
-        nodes[id].depth = depth;
+    // Splits node id's columns perm[lo, hi) in two halves across the longest side of their bounding box; the
+    // separator is a smallest set of columns that covers every block between the halves (a minimum vertex
+    // cover of the cut edges, from a maximum matching). Its halves are appended to `nodes`.
+    void split(int id) {
+        const int32_t lo = nodes[id].lo, hi = nodes[id].hi;
         if (hi - lo <= leaf) {
             nodes[id].piv.assign(perm.begin() + lo, perm.begin() + hi);
-            return id;
+            return;
         }
         double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
         for (int32_t k = lo; k < hi; ++k)
@@ -135,16 +151,43 @@ struct Dissection {
             const double yu = X[(size_t)u * 3 + a2], yv = X[(size_t)v * 3 + a2];
             return yu != yv ? yu < yv : u < v;
         });
+        // A half's boundary: the columns of the enclosing separators, this one's among them, next to it. From the top
+        // down the fronts' sizes are known before the fronts below are.
+        std::vector<int32_t> out = nodes[id].bnd;
+        out.insert(out.end(), nodes[id].piv.begin(), nodes[id].piv.end());
         int n = 0;
-        if (ma > lo) {
-            const int c = split(lo, ma, depth + 1);
-            nodes[id].child[n++] = c;
-        }
-        if (mb > ma) {
-            const int c = split(ma, mb, depth + 1);
-            nodes[id].child[n++] = c;
-        }
-        return id;
+        auto half = [&](int32_t a, int32_t z, int32_t l) {
+            if (a == z) return;
+            nodes[id].child[n++] = (int)nodes.size();
+            Node h;
+            h.depth = nodes[id].depth + 1;
+            h.lo = a;
+            h.hi = z;
+            // from the separators' side or, where a column of theirs has very many neighbours, from the half's
+            int64_t far = 0, near = 0;
+            for (int32_t v : out) far += ptr[v + 1] - ptr[v];
+            for (int32_t k = a; k < z && near < far; ++k) near += ptr[perm[k] + 1] - ptr[perm[k]];
+            ++stamp;
+            if (far <= near) {
+                for (int32_t v : out)
+                    for (int32_t q = ptr[v]; q < ptr[v + 1]; ++q)
+                        if (label[adj[q]] == l) {
+                            h.bnd.push_back(v);
+                            break;
+                        }
+            } else {
+                for (int32_t k = a; k < z; ++k)
+                    for (int32_t q = ptr[perm[k]]; q < ptr[perm[k] + 1]; ++q) {
+                        const int32_t v = adj[q];
+                        if (label[v] == l || seen[v] == stamp) continue;
+                        seen[v] = stamp;
+                        h.bnd.push_back(v);
+                    }
+            }
+            nodes.push_back(std::move(h));
+        };
+        half(lo, ma, la);
+        half(ma, mb, lb);
     }
 
     // Elimination positions (children before their parent) and every front's boundary.
@@ -154,39 +197,40 @@ struct Dissection {
         for (int32_t v : nodes[id].piv) pos[v] = at++;
         return at;
     }
-    void boundary(int id) {
+    // The nodes in depth-first order from id on, into `to`.
+    int renumber(int id, std::vector<Node>& to) {
+        const int at = (int)to.size();
+        to.push_back(std::move(nodes[id]));
         for (int k = 0; k < 2; ++k)
-            if (nodes[id].child[k] >= 0) boundary(nodes[id].child[k]);
-        Node& f = nodes[id];
-        ++stamp;
-        for (int32_t v : f.piv) seen[v] = stamp;
-        auto add = [&](int32_t v, int32_t after) {
-            if (pos[v] > after && seen[v] != stamp) {
-                seen[v] = stamp;
-                f.bnd.push_back(v);
+            if (to[at].child[k] >= 0) {
+                const int c = renumber(to[at].child[k], to);
+                to[at].child[k] = c;
             }
-        };
-        int32_t last = -1;  // position of the subtree's last eliminated column
-        for (int32_t v : f.piv) last = std::max(last, pos[v]);
-        for (int32_t v : f.piv)
-            for (int32_t k = ptr[v]; k < ptr[v + 1]; ++k) add(adj[k], last);
-        for (int c : f.child)
-            if (c >= 0)
-                for (int32_t v : nodes[c].bnd) add(v, last);
-        std::sort(f.bnd.begin(), f.bnd.end(), [&](int32_t u, int32_t v) { return pos[u] < pos[v]; });
+        return at;
     }
 
-    void run(int32_t n) {
+    // Level by level, the largest fronts first: a tissue too large for a factorisation shows after the top two or
+    // three of its levels (2,000,000 nodes: after the first cut).
+    void run(int32_t n, Budget& budget) {
         perm.resize(n);
         std::iota(perm.begin(), perm.end(), 0);
         label.assign(n, -1);
         match.assign(n, -1);
         seen.assign(n, -1);
         pos.assign(n, 0);
-        split(0, n, 0);
+        nodes.emplace_back();
+        nodes[0].hi = n;
+        for (int id = 0; id < (int)nodes.size() && !budget.over; ++id) {
+            split(id);
+            budget.add(nodes[id].piv.size(), nodes[id].bnd.size(), gd);
+        }
+        if (budget.over) return;
+        std::vector<Node> sorted;
+        sorted.reserve(nodes.size());
+        renumber(0, sorted);
+        nodes.swap(sorted);
         order(0, 0);
-        stamp = next_label + 1 + stamp;
-        boundary(0);
+        for (Node& f : nodes) std::sort(f.bnd.begin(), f.bnd.end(), [&](int32_t u, int32_t v) { return pos[u] < pos[v]; });
     }
 };
 
@@ -213,31 +257,43 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
     plan = FcPlan();
     const int nc = N / G, gd = 3 * G;
     plan.gd = gd;
-    // column graph (no self edges), global ids; a tissue's columns are consecutive
+    // column graph (no self edges), global ids; a tissue's columns are consecutive. By runs of columns, so that a
+    // single large tissue has every thread on it.
     std::vector<int32_t> ptr(nc + 1, 0), adj;
     {
-        std::vector<std::vector<int32_t>> part(T);
-        parallel_items(T, [&](int t) {
-            const int c0 = node0[t] / G, c1 = node0[t + 1] / G;
+        struct Run {
+            int t, c0, c1;
+            std::vector<int32_t> adj;
+        };
+        std::vector<Run> runs;
+        for (int t = 0; t < T; ++t) {
+            const int c0 = node0[t] / G, c1 = node0[t + 1] / G, len = std::max(8192, (c1 - c0 + 15) / 16);
+            for (int c = c0; c < c1; c += len) runs.push_back({t, c, std::min(c + len, c1), {}});
+        }
+        parallel_items((int)runs.size(), [&](int i) {
+            Run& r = runs[i];
+            const int c0 = node0[r.t] / G, c1 = node0[r.t + 1] / G;
             std::vector<int32_t> mark(c1 - c0, -1);
-            for (int c = c0; c < c1; ++c) {
-                const size_t before = part[t].size();
+            for (int c = r.c0; c < r.c1; ++c) {
+                const size_t before = r.adj.size();
                 for (int i = c * G; i < (c + 1) * G; ++i)
                     for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
                         const int32_t d = colidx[k] / G;
                         if (d != c && mark[d - c0] != c) {
                             mark[d - c0] = c;
-                            part[t].push_back(d - c0);
+                            r.adj.push_back(d - c0);
                         }
                     }
-                ptr[c + 1] = (int32_t)(part[t].size() - before);
+                ptr[c + 1] = (int32_t)(r.adj.size() - before);
             }
         });
         for (int c = 0; c < nc; ++c) ptr[c + 1] += ptr[c];
-        adj.reserve(ptr[nc]);
-        for (int t = 0; t < T; ++t) adj.insert(adj.end(), part[t].begin(), part[t].end());
+        adj.resize(ptr[nc]);
+        parallel_items((int)runs.size(), [&](int i) { std::copy(runs[i].adj.begin(), runs[i].adj.end(), adj.begin() + ptr[runs[i].c0]); });
     }
     std::vector<Dissection> ds(T);
+    Budget budget;
+    budget.max_flops = max_flops;
     parallel_items(T, [&](int t) {
         const int c0 = node0[t] / G, c1 = node0[t + 1] / G;
         Dissection& d = ds[t];
@@ -247,23 +303,20 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
         d.adj = adj.data() + ptr[c0];
         d.X = X + (size_t)c0 * 3;
         d.leaf = std::max(1, kFcTile / gd);
-        d.run(c1 - c0);
+        d.gd = gd;
+        d.run(c1 - c0, budget);
     });
+    plan.flops = budget.flops;
+    if (budget.over) return;
     // fronts of all tissues by depth
     int depths = 0;
-    double flops = 0.0;
     std::vector<std::vector<std::pair<int, int>>> at;  // per depth: (tissue, node)
     for (int t = 0; t < T; ++t)
         for (int k = 0; k < (int)ds[t].nodes.size(); ++k) {
             const Node& f = ds[t].nodes[k];
             if (f.depth >= depths) at.resize(depths = f.depth + 1);
             at[f.depth].push_back({t, k});
-            const double p = (double)f.piv.size() * gd, b = (double)f.bnd.size() * gd;
-            flops += p * p * p * (2.0 / 3.0) + p * p * b + b * b * p;
-            if (p > kFcMaxPivots || p + b > kFcMaxFront) return;
         }
-    plan.flops = flops;
-    if (flops > max_flops) return;
     std::vector<std::vector<int32_t>> id(T);
     for (int t = 0; t < T; ++t) id[t].resize(ds[t].nodes.size());
     int nf = 0;
