@@ -6,7 +6,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <vector>
+
+#include <sys/resource.h>
 
 #include "tf_factor.cuh"
 
@@ -88,15 +91,13 @@ int check(const tfb::FcPlan& P, const Sheet& one, int G) {
     return 0;
 }
 
-}  // namespace
-
-int main(int argc, char** argv) {
+int run(int argc, char** argv) {
     if (argc == 4 && !std::strcmp(argv[1], "span")) {  // of blocks [a, b)
         const tfb::FcSpan s = tfb::fc_block_span(std::atoi(argv[2]), std::atoi(argv[3]));
         std::printf("%" PRId64 " %" PRId64 "\n", s.begin, s.end);
         return 0;
     }
-    if (argc == 8 && !std::strcmp(argv[1], "plan")) {  // nx ny G max_flops transposed tissues (all of that size)
+    if ((argc == 8 || argc == 9) && !std::strcmp(argv[1], "plan")) {  // nx ny G max_flops transposed tissues [kB]
         const int G = std::atoi(argv[4]), T = std::atoi(argv[7]);
         const Sheet one(std::atoi(argv[2]), std::atoi(argv[3]), G);
         const int n = (int)one.rowptr.size() - 1, blocks = one.rowptr.back();
@@ -107,6 +108,17 @@ int main(int argc, char** argv) {
             for (int32_t c : one.colidx) colidx.push_back(c + t * n);
             X.insert(X.end(), one.X.begin(), one.X.end());
             node0.push_back((t + 1) * n);
+        }
+        if (argc == 9) {  // as much address space besides what the process has by now
+            long pages = 0;
+            if (FILE* f = std::fopen("/proc/self/statm", "r")) {
+                if (std::fscanf(f, "%ld", &pages) != 1) return 3;
+                std::fclose(f);
+            }
+            rlimit lim;
+            getrlimit(RLIMIT_AS, &lim);
+            lim.rlim_cur = (rlim_t)pages * 4096 + (rlim_t)std::atoi(argv[8]) * 1024;
+            if (setrlimit(RLIMIT_AS, &lim)) return 3;
         }
         tfb::FcPlan P;
         const auto t0 = std::chrono::steady_clock::now();
@@ -128,4 +140,15 @@ int main(int argc, char** argv) {
         return 0;
     }
     return 2;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+    try {
+        return run(argc, argv);
+    } catch (const std::bad_alloc&) {
+        std::printf("bad_alloc\n");
+        return 0;
+    }
 }

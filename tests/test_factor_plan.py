@@ -1,5 +1,6 @@
 """The host side of the sparse factorisation on the CPU: tests/factor_plan_host.cpp, linked against the library."""
 import os
+import resource
 import subprocess
 
 import pytest
@@ -57,3 +58,21 @@ def test_boundaries_of_the_fronts(host, sheet):
     """Every column a pivot of one front; every front's boundary what its subtree touches, also around a column
     with hundreds of neighbours (found from the other side there)."""
     assert host("check", *sheet) == ["1", "0"]
+
+
+def _limited(what, value):
+    return lambda: resource.setrlimit(what, (value, resource.getrlimit(what)[1]))
+
+
+def test_plan_without_threads(host):
+    """Where no thread can be started (here: no address space for a stack of 64 TB), the caller's does it all."""
+    args = ("plan", 60, 50, 2, 3e11, 0, 3)
+    alone = host(*args, preexec_fn=_limited(resource.RLIMIT_STACK, 1 << 46))
+    with_threads = host(*args)
+    assert alone[0] == "1" and alone[:2] + alone[3:] == with_threads[:2] + with_threads[3:]
+
+
+def test_plan_without_host_memory(host):
+    """Too little memory, at whatever point of the plan: an exception for the caller, not the end of the process."""
+    ways = [host("plan", 150, 100, 3, 1e15, 1, 3, kb)[0] for kb in [100 * 2**k for k in range(14)]]
+    assert set(ways) == {"bad_alloc", "1"}

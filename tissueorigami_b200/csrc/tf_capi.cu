@@ -1749,12 +1749,17 @@ void release_factor(tf_ctx* c) {
 
 int lay_out_factor(tf_ctx* ctx);
 
-// The plan of the current pattern and its buffers; without memory for them, none (fc_ready = false).
+// The plan of the current pattern and its buffers; without host or device memory for them, none (fc_ready = false).
 int build_factor(tf_ctx* ctx) {
     ctx->fc_dirty = false;
     ctx->fc_ready = false;
     drop_factor_graphs(ctx);
-    const int rc = lay_out_factor(ctx);
+    int rc;
+    try {
+        rc = lay_out_factor(ctx);
+    } catch (const std::exception&) {  // host memory
+        rc = TF_ERR_OUT_OF_MEMORY;
+    }
     if (!ctx->fc_ready) release_factor(ctx);
     if (rc != TF_ERR_OUT_OF_MEMORY) return rc;
     ctx->last_error[0] = 0;

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <exception>
 #include <mutex>
 #include <numeric>
 #include <thread>
@@ -237,17 +238,32 @@ struct Dissection {
 // Fronts that one CTA factorises in shared memory.
 bool one_cta(const FcFront& F) { return F.p > 0 && F.p <= kFcTile && F.b <= kFcSmallB; }
 
+// f(0) .. f(n - 1) on up to 16 threads, fewer where no more can be started. What an f throws is thrown here, after
+// every thread has ended.
 template <class F>
 void parallel_items(int n, F f) {
     const int nt = std::min<int>(n, (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
     std::atomic<int> next{0};
+    std::exception_ptr thrown;
+    std::mutex lock;
     auto work = [&] {
-        for (int i; (i = next.fetch_add(1)) < n;) f(i);
+        try {
+            for (int i; (i = next.fetch_add(1)) < n;) f(i);
+        } catch (...) {
+            std::lock_guard<std::mutex> hold(lock);
+            if (!thrown) thrown = std::current_exception();
+            next = n;
+        }
     };
     std::vector<std::thread> th;
-    for (int t = 1; t < nt; ++t) th.emplace_back(work);
+    th.reserve(nt);
+    try {
+        for (int t = 1; t < nt; ++t) th.emplace_back(work);
+    } catch (const std::exception&) {
+    }
     work();
     for (auto& x : th) x.join();
+    if (thrown) std::rethrow_exception(thrown);
 }
 
 }  // namespace
