@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cinttypes>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -128,6 +129,15 @@ int run(int argc, char** argv) {
         uint64_t h = 14695981039346656037ull;
         h = mix(mix(mix(mix(mix(mix(h, P.fronts), P.maps), P.verts), P.jblk), P.jblk_t), P.tasks);
         std::printf("%d %.6e %.2f %zu %016" PRIx64 "\n", P.ok ? 1 : 0, P.flops, ms, P.fronts.size(), h);
+        return 0;
+    }
+    if (argc == 5 && !std::strcmp(argv[1], "nan")) {  // nx ny every: each such column's position not a number
+        Sheet one(std::atoi(argv[2]), std::atoi(argv[3]), 2);
+        for (size_t c = 0; c < one.X.size() / 3; c += std::atoi(argv[4])) one.X[3 * c + c % 3] = std::nan("");
+        const int32_t node0[2] = {0, (int32_t)one.rowptr.size() - 1};
+        tfb::FcPlan P;
+        tfb::build_factor_plan(node0[1], 2, one.rowptr.data(), one.colidx.data(), one.X.data(), 1, node0, 1e13, false, P);
+        std::printf("%d\n", P.ok ? 1 : 0);
         return 0;
     }
     if (argc == 6 && !std::strcmp(argv[1], "check")) {  // nx ny G star

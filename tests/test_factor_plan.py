@@ -76,3 +76,9 @@ def test_plan_without_host_memory(host):
     """Too little memory, at whatever point of the plan: an exception for the caller, not the end of the process."""
     ways = [host("plan", 150, 100, 3, 1e15, 1, 3, kb)[0] for kb in [100 * 2**k for k in range(14)]]
     assert set(ways) == {"bad_alloc", "1"}
+
+
+@pytest.mark.parametrize("every", [1, 7, 1000])
+def test_no_plan_for_positions_that_are_not_numbers(host, every):
+    """They cannot be ordered for the cuts; the iterative solve reports what becomes of such a tissue."""
+    assert host("nan", 100, 100, every) == ["0"]

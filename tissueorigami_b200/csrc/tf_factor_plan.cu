@@ -273,6 +273,8 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
     plan = FcPlan();
     const int nc = N / G, gd = 3 * G;
     plan.gd = gd;
+    // a comparison of positions that are not numbers is no order, and std::nth_element may leave its range then
+    if (!std::all_of(X, X + (size_t)nc * 3, [](double x) { return std::isfinite(x); })) return;
     // column graph (no self edges), global ids; a tissue's columns are consecutive. By runs of columns, so that a
     // single large tissue has every thread on it.
     std::vector<int32_t> ptr(nc + 1, 0), adj;
