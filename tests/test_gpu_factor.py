@@ -224,3 +224,24 @@ def test_set_growth_rejects_a_tensor_with_two_equal_rows(rows):
             else:
                 s.set_growth(fg=wrong)
         assert refused > 0
+
+
+@pytest.mark.parametrize("apart", [1e-2, 1e-13, 1e-15])
+def test_set_growth_inverts_nearly_singular_tensors_by_the_determinant_it_tests(apart):
+    """Tensors with two nearly equal rows: InvFg to the last bit what the adjugate over the determinant, every
+    product rounded, gives in numpy; a determinant rounded differently is off by its whole size there, or zero."""
+    t = mesh.small_disc(5, 301, 1000.0)
+    rng = np.random.default_rng(11)
+    fg = rng.uniform(0.5, 1.5, (t.n_elems, 3, 3))
+    fg[:, 2] = fg[:, 0] * (1.0 + apart * rng.uniform(-1.0, 1.0, (t.n_elems, 3)))
+    m = fg.reshape(-1, 9).T
+    det = (m[0] * (m[4] * m[8] - m[5] * m[7]) - m[1] * (m[3] * m[8] - m[5] * m[6])) + m[2] * (m[3] * m[7] - m[4] * m[6])
+    fg[det == 0.0] = np.eye(3)
+    m = fg.reshape(-1, 9).T.copy()
+    det = (m[0] * (m[4] * m[8] - m[5] * m[7]) - m[1] * (m[3] * m[8] - m[5] * m[6])) + m[2] * (m[3] * m[7] - m[4] * m[6])
+    adj = np.stack([m[4] * m[8] - m[5] * m[7], m[2] * m[7] - m[1] * m[8], m[1] * m[5] - m[2] * m[4],
+                    m[5] * m[6] - m[3] * m[8], m[0] * m[8] - m[2] * m[6], m[2] * m[3] - m[0] * m[5],
+                    m[3] * m[7] - m[4] * m[6], m[1] * m[6] - m[0] * m[7], m[0] * m[4] - m[1] * m[3]])
+    with NewtonRaphsonSolver.from_tissue(t) as s:
+        s.set_growth(fg=fg)
+        assert np.array_equal(s.get_growth()[1].reshape(-1, 9), (adj * (1.0 / det)).T)

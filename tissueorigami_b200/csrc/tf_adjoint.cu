@@ -257,17 +257,41 @@ __global__ void k_set_inv_fg(ElemRecord* elems, int32_t n_elems, const double* f
         for (int j = 0; j < 3; ++j) elems[e].inv_fg[i * 3 + j] = o[i][j];
 }
 
+// Determinant of a growth tensor with every product rounded: contracted, that of a tensor with two equal rows is not
+// zero. What is tested for and what the inverse divides by are the same number.
+__device__ __forceinline__ double fg_minor(double a, double b, double c, double d) {
+    return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d));
+}
+__device__ __forceinline__ double fg_det(const double* m) {
+    return __dadd_rn(__dsub_rn(__dmul_rn(m[0], fg_minor(m[4], m[8], m[5], m[7])),
+                               __dmul_rn(m[1], fg_minor(m[3], m[8], m[5], m[6]))),
+                     __dmul_rn(m[2], fg_minor(m[3], m[7], m[4], m[6])));
+}
+
 // *flag = 1 when some Fg is singular or not finite.
 __global__ void k_check_fg(int32_t n_elems, const double* fg, int32_t* flag) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_elems) return;
-    const double* m = fg + (size_t)e * 9;
-    // every product rounded: contracted, the determinant of a tensor with two equal rows is not zero
-    auto minor = [](double a, double b, double c, double d) { return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d)); };
-    const double det = __dadd_rn(__dsub_rn(__dmul_rn(m[0], minor(m[4], m[8], m[5], m[7])),
-                                           __dmul_rn(m[1], minor(m[3], m[8], m[5], m[6]))),
-                                 __dmul_rn(m[2], minor(m[3], m[7], m[4], m[6])));
+    const double det = fg_det(fg + (size_t)e * 9);
     if (det == 0.0 || !isfinite(det)) *flag = 1;
+}
+
+// InvFg of Fg given by a caller (checked before).
+__global__ void k_set_given_inv_fg(ElemRecord* elems, int32_t n_elems, const double* fg) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_elems) return;
+    const double* m = fg + (size_t)e * 9;
+    const double id = 1.0 / fg_det(m);
+    double* o = elems[e].inv_fg;
+    o[0] = fg_minor(m[4], m[8], m[5], m[7]) * id;
+    o[1] = fg_minor(m[2], m[7], m[1], m[8]) * id;
+    o[2] = fg_minor(m[1], m[5], m[2], m[4]) * id;
+    o[3] = fg_minor(m[5], m[6], m[3], m[8]) * id;
+    o[4] = fg_minor(m[0], m[8], m[2], m[6]) * id;
+    o[5] = fg_minor(m[2], m[3], m[0], m[5]) * id;
+    o[6] = fg_minor(m[3], m[7], m[4], m[6]) * id;
+    o[7] = fg_minor(m[1], m[6], m[0], m[7]) * id;
+    o[8] = fg_minor(m[0], m[4], m[1], m[3]) * id;
 }
 
 // field (a double offset in the records) of every record = src [E][ncomp]; one double per thread, so the
@@ -315,6 +339,11 @@ cudaError_t launch_check_fg(int32_t n_elems, const double* fg, int32_t* flag, cu
     cudaError_t err = cudaMemsetAsync(flag, 0, sizeof(int32_t), s);
     if (err != cudaSuccess) return err;
     k_check_fg<<<(n_elems + 255) / 256, 256, 0, s>>>(n_elems, fg, flag);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_set_given_inv_fg(ElemRecord* elems, int32_t n_elems, const double* fg, cudaStream_t s) {
+    k_set_given_inv_fg<<<(n_elems + 255) / 256, 256, 0, s>>>(elems, n_elems, fg);
     return cudaGetLastError();
 }
 

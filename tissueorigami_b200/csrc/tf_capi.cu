@@ -3250,7 +3250,7 @@ int tf_set_growth(tf_ctx* ctx, const double* fg, const double* rates, const doub
         rc = read_flags(ctx);
         if (rc != TF_OK) return rc;
         if (*ctx->h_flags) return TF_ERR_ARGUMENT;
-        TF_CK(launch_set_inv_fg(dptr<ElemRecord>(ctx->elems), ctx->E, dptr<double>(ctx->fg), ctx->stream));
+        TF_CK(launch_set_given_inv_fg(dptr<ElemRecord>(ctx->elems), ctx->E, dptr<double>(ctx->fg), ctx->stream));
         TF_CK(cudaStreamSynchronize(ctx->stream));
     }
     if (rates) TF_CK(cudaMemcpy(ctx->rates.p, rates, sizeof(double) * 3 * E, cudaMemcpyHostToDevice));

@@ -273,6 +273,8 @@ cudaError_t launch_position_vjp(const ElemRecord* elems, int32_t n_elems, int32_
 cudaError_t launch_set_inv_fg(ElemRecord* elems, int32_t n_elems, const double* fg, cudaStream_t s);
 // *flag = 1 when the growth tensor of some element is singular or not finite, else 0
 cudaError_t launch_check_fg(int32_t n_elems, const double* fg, int32_t* flag, cudaStream_t s);
+// InvFg of growth tensors that passed it, by the same determinant
+cudaError_t launch_set_given_inv_fg(ElemRecord* elems, int32_t n_elems, const double* fg, cudaStream_t s);
 // ncomp doubles from double `field` on of every record = src [n_elems][ncomp] (device)
 cudaError_t launch_set_field(ElemRecord* elems, int32_t n_elems, int field, int ncomp, const double* src, cudaStream_t s);
 cudaError_t launch_mask_fixed(int32_t n_nodes, const uint8_t* fixmask, double* v, cudaStream_t s);
