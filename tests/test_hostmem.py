@@ -1,6 +1,7 @@
 """The pool of page-locked result arrays: blocks that are in use are not handed out again, what is dropped is
 reused, what does not fit its bound is an ordinary array. On the CPU with a library that only counts."""
 import gc
+import sys
 
 import numpy as np
 import pytest
@@ -56,6 +57,53 @@ def test_pool_is_bounded():
     assert sum(lib.live.values()) <= hostmem.KEEP
     other = pool.take(lib, "ctx", (250 * MB // 8,))  # gives the kept blocks back
     assert other is not None and sum(lib.live.values()) <= hostmem.LIMIT
+
+
+def test_arrays_dropped_while_another_is_taken():
+    """The garbage collector may drop arrays between any two lines of take() on the same thread: no block is
+    handed out twice, none is lost, and the bound holds."""
+    pool, lib = hostmem._Pool(), _Lib()
+
+    def garbage(mb):
+        a = pool.take(lib, "ctx", (mb * MB // 8,))
+        cycle = [a]
+        cycle.append(cycle)
+
+    lines = [0]
+
+    def trace(frame, event, arg):
+        if frame.f_code.co_filename != hostmem.__file__ or frame.f_code.co_name in ("_give", "_reset"):
+            return None
+        if event == "line":
+            lines[0] += 1
+            if lines[0] == at:
+                gc.collect()
+        return trace
+
+    gc.disable()
+    gc.freeze()  # collections look at what follows only
+    try:
+        for at in range(1, 60):
+            for sizes in ([1, 2, 3], [3, 2, 1], [70, 1, 1]):
+                held = [pool.take(lib, "ctx", (MB // 8,)) for _ in range(2)]
+                del held  # two kept blocks
+                for mb in sizes:
+                    garbage(mb)
+                lines[0] = 0
+                sys.settrace(trace)
+                try:
+                    held = [pool.take(lib, "ctx", (mb * MB // 8,)) for mb in (1, 2, 1)]
+                finally:
+                    sys.settrace(None)
+                spans = sorted((h.ctypes.data, h.nbytes) for h in held)
+                assert all(p + n <= q for (p, n), (q, _) in zip(spans, spans[1:]))
+                assert all(p in lib.live for p, _ in spans)
+                del held
+                gc.collect()
+                assert sum(lib.live.values()) == pool._bytes <= hostmem.KEEP
+    finally:
+        gc.unfreeze()
+        gc.enable()
 
 
 @pytest.mark.gpu

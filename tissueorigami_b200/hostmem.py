@@ -6,6 +6,7 @@ page-locked blocks that go back to a bounded pool when the last view of the arra
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import mmap
 import os
@@ -25,8 +26,9 @@ class _Pool:
 
     def _reset(self):
         """Also in a forked child, where the parent's registrations do not count."""
-        self._lock = threading.RLock()  # a finalizer may run inside take()
-        self._free = []  # (size, block), oldest first
+        self._lock = threading.Lock()
+        self._free = []  # (size, block), oldest first; only the lock's holder touches it
+        self._back = collections.deque()  # (lib, size, block) dropped and not yet in _free
         self._bytes = 0
         self._pid = os.getpid()
 
@@ -50,33 +52,57 @@ class _Pool:
         size = -(-n // MIN_BYTES) * MIN_BYTES
         if n < MIN_BYTES or size > LIMIT:
             return None
-        with self._lock:
-            for i, (have, block) in enumerate(self._free):
-                if size <= have <= size + size // 4:
-                    size = have
-                    del self._free[i]
-                    break
-            else:
-                self._drop(lib, size)
-                if self._bytes + size > LIMIT:
-                    return None
-                block = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
-                if hasattr(mmap, "MADV_HUGEPAGE"):
-                    block.madvise(mmap.MADV_HUGEPAGE)
-                view = ctypes.c_char.from_buffer(block)
-                ok = lib.tf_host_register(handle, ctypes.addressof(view), size) == 0
-                del view
-                if not ok:
-                    return None
-                self._bytes += size
+        try:
+            with self._lock:
+                self._settle()
+                size, block = self._block(lib, handle, size)
+        finally:
+            self._settle_unless_held()
+        if block is None:
+            return None
         owner = (ctypes.c_char * n).from_buffer(block)
         weakref.finalize(owner, self._give, lib, size, block, self._pid).atexit = False
         return np.frombuffer(owner, dtype=np.float64).reshape(shape)
 
+    def _block(self, lib, handle, size):
+        """A kept block of about `size` bytes or a new one, or None; and its size."""
+        for i, (have, block) in enumerate(self._free):
+            if size <= have <= size + size // 4:
+                del self._free[i]
+                return have, block
+        self._drop(lib, size)
+        if self._bytes + size > LIMIT:
+            return size, None
+        block = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        if hasattr(mmap, "MADV_HUGEPAGE"):
+            block.madvise(mmap.MADV_HUGEPAGE)
+        view = ctypes.c_char.from_buffer(block)
+        ok = lib.tf_host_register(handle, ctypes.addressof(view), size) == 0
+        del view
+        if not ok:
+            return size, None
+        self._bytes += size
+        return size, block
+
     def _give(self, lib, size, block, pid):
-        with self._lock:
-            if pid != self._pid:
-                return
+        """The last view of a block is gone. A finalizer: the garbage collector may run it between any two
+        instructions, those of the lock's holder on the same thread among them, so it only queues the block."""
+        if pid != self._pid:
+            return
+        self._back.append((lib, size, block))
+        self._settle_unless_held()
+
+    def _settle_unless_held(self):
+        while self._back and self._lock.acquire(blocking=False):
+            try:
+                self._settle()
+            finally:
+                self._lock.release()
+
+    def _settle(self):
+        """Queued blocks into _free, the oldest given back beyond KEEP."""
+        while self._back:
+            lib, size, block = self._back.popleft()
             self._free.append((size, block))
             while self._kept() > KEEP:
                 self._unregister(lib, *self._free.pop(0))
