@@ -59,6 +59,25 @@ def test_pool_is_bounded():
     assert other is not None and sum(lib.live.values()) <= hostmem.LIMIT
 
 
+@pytest.mark.parametrize("what", ["mmap", "madvise"])
+def test_a_refused_mapping_is_no_error(monkeypatch, what):
+    """Without a mapping the result is an ordinary array, without huge pages the block has small ones."""
+    real = hostmem.mmap.mmap
+
+    class Mapping(real):
+        def madvise(self, *args):
+            raise OSError(22, "Invalid argument")
+
+    def refuse(*args, **kw):
+        raise OSError(12, "Cannot allocate memory")
+
+    monkeypatch.setattr(hostmem.mmap, "mmap", refuse if what == "mmap" else Mapping)
+    pool, lib = hostmem._Pool(), _Lib()
+    a = pool.take(lib, "ctx", (MB // 8,))
+    assert (a is None) == (what == "mmap") and len(lib.live) == (what == "madvise")
+    assert pool._bytes == sum(lib.live.values())
+
+
 def test_arrays_dropped_while_another_is_taken():
     """The garbage collector may drop arrays between any two lines of take() on the same thread: no block is
     handed out twice, none is lost, and the bound holds."""

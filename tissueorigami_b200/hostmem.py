@@ -73,9 +73,14 @@ class _Pool:
         self._drop(lib, size)
         if self._bytes + size > LIMIT:
             return size, None
-        block = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
-        if hasattr(mmap, "MADV_HUGEPAGE"):
+        try:
+            block = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        except OSError:  # no address space or mapping left
+            return size, None
+        try:
             block.madvise(mmap.MADV_HUGEPAGE)
+        except (AttributeError, OSError):  # a kernel without huge pages
+            pass
         view = ctypes.c_char.from_buffer(block)
         ok = lib.tf_host_register(handle, ctypes.addressof(view), size) == 0
         del view
