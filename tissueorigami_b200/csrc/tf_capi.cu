@@ -190,7 +190,7 @@ struct tf_ctx {
     cudaGraphExec_t fc_graph[3] = {};  // the factorisation, the first iteration, a further one
     int64_t fc_graph_launches[3] = {};
     DevBuf fc_fronts, fc_maps, fc_verts, fc_jblk, fc_jblk_t, fc_tasks, fc_factor, fc_scratch, fc_contrib[2], fc_kids, fc_dofs, fc_vec, fc_z,
-        fc_sign, fc_flags, fc_neg, fc_chunks, fc_chunk0_d, fc_running, fc_part;
+        fc_sign, fc_neg, fc_chunks, fc_chunk0_d, fc_running, fc_part;
 
     // adjoint: forward checkpoints every adj_k steps, segment recompute buffers, adjoint state
     int32_t adj_steps = 0, adj_k = 0;
@@ -1741,7 +1741,7 @@ void release_factor(tf_ctx* c) {
     drop_factor_graphs(c);
     DevBuf* b[] = {&c->fc_fronts, &c->fc_maps, &c->fc_verts, &c->fc_jblk, &c->fc_jblk_t, &c->fc_tasks, &c->fc_factor,
                    &c->fc_scratch, &c->fc_contrib[0], &c->fc_contrib[1], &c->fc_kids, &c->fc_dofs, &c->fc_vec, &c->fc_z,
-                   &c->fc_sign, &c->fc_flags, &c->fc_neg, &c->fc_chunks, &c->fc_chunk0_d, &c->fc_running, &c->fc_part};
+                   &c->fc_sign, &c->fc_neg, &c->fc_chunks, &c->fc_chunk0_d, &c->fc_running, &c->fc_part};
     for (DevBuf* q : b) dfree(*q);
     c->fc = FcPlan();
     c->fc_ready = false;
@@ -1819,7 +1819,6 @@ int lay_out_factor(tf_ctx* ctx) {
         if (!st.side[q]) TF_CK(cudaStreamCreateWithFlags(&st.side[q], cudaStreamNonBlocking));
         if (!st.join[q]) TF_CK(cudaEventCreateWithFlags(&st.join[q], cudaEventDisableTiming));
     }
-    TF_CK(dalloc(ctx->fc_flags, sizeof(int32_t) * T));
     TF_CK(dalloc(ctx->fc_neg, sizeof(int32_t) * P.fronts.size()));
     TF_CK(dalloc(ctx->fc_running, sizeof(int32_t) * T));
     TF_CK(up(ctx->fc_fronts, P.fronts.data(), sizeof(FcFront) * P.fronts.size()));
@@ -1862,7 +1861,6 @@ FcWork make_factor(tf_ctx* c) {
     f.vec = dptr<double>(c->fc_vec);
     f.z = dptr<double>(c->fc_z);
     f.sign = dptr<double>(c->fc_sign);
-    f.flags = dptr<int32_t>(c->fc_flags);
     f.neg = dptr<int32_t>(c->fc_neg);
     return f;
 }
@@ -1891,7 +1889,6 @@ int factor_solve(tf_ctx* ctx, std::vector<int32_t>& left) {
     FcWork f = make_factor(ctx);
     FcCg c;
     c.n_chunks = ctx->fc_chunk0.back();
-    c.T = ctx->T;
     c.chunks = dptr<FcChunk>(ctx->fc_chunks);
     c.chunk0 = dptr<int32_t>(ctx->fc_chunk0_d);
     c.sc = dptr<KrylovScalars>(ctx->tscalars);
@@ -1903,8 +1900,7 @@ int factor_solve(tf_ctx* ctx, std::vector<int32_t>& left) {
     const bool kept = ctx->fc_same || ctx->fc_near;
     if (!kept) {
         const int rc = replay_factor(ctx, 0, [&](int64_t* n) -> cudaError_t {
-            cudaError_t e = cudaMemsetAsync(ctx->fc_flags.p, 0, sizeof(int32_t) * ctx->T, ctx->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(ctx->fc_neg.p, 0, sizeof(int32_t) * ctx->fc.fronts.size(), ctx->stream);
+            const cudaError_t e = cudaMemsetAsync(ctx->fc_neg.p, 0, sizeof(int32_t) * ctx->fc.fronts.size(), ctx->stream);
             return e == cudaSuccess ? launch_factor(ctx->fc, f, w.vals, n, ctx->fc_streams) : e;
         });
         if (rc != TF_OK) return rc;

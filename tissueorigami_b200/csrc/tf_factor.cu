@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(256) k_fc_scatter(FcWork w, const double* __re
 // fragments of eight 8 x 8 tiles. Per block of 8 pivots every warp below it eliminates the pivot tile
 // and its own tile of those columns by shuffles (the pivot tile redundantly, so that the 8 steps need no
 // barrier), and its other tiles by two tensor instructions each. Returns the rows of
-// G^-1 = |D|^-1/2 L^-1 (zero right of the diagonal and outside the block) and writes sign(D).
+// G^-1 = |D|^-1/2 L^-1 (zero right of the diagonal and outside the block) and writes sign(D). A zero pivot leaves
+// non-finite values, which the solve's first residual shows.
 // Bound by the chain of 8 steps (a shuffle, a reciprocal and two FP64 operations, ~125 cycles each). A row
 // per four threads with the pivot row read from shared memory took 571 cycles a step (64 pivots:
 // 36.6 k): 256 threads x 16 entries a step is 256 cycles of shared-memory reads alone.
@@ -157,7 +158,7 @@ struct __align__(16) FactorShared {
     double d[kT];
 };
 __device__ __forceinline__ void factor_block(const double* s, int ld, int n, FactorShared& sh, double (&v)[8][2], double* sign,
-                                             int32_t* flag, int32_t* neg) {
+                                             int32_t* neg) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, lr = lane >> 2, lk = lane & 3, r = 8 * w + lr;
 #pragma unroll
     for (int t = 0; t < 8; ++t)
@@ -240,7 +241,6 @@ __device__ __forceinline__ void factor_block(const double* s, int ld, int n, Fac
     if (r < n && lk == 0) {
         sign[r] = d < 0.0 ? -1.0 : 1.0;
         if (d < 0.0) *neg = 1;
-        if (!(fabs(d) > 0.0) || !isfinite(d)) *flag = 1;
     }
 }
 
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(256) k_fc_diag(FcWork w, int begin) {
     load_tile(s, A, F.ldp, n, n);  // above the diagonal: not initialised, and not read
     tile_wait();
     double v[8][2];
-    factor_block(&s[0][0], kLd, n, sh, v, w.sign + F.piv, w.flags + F.tissue, w.neg + tk.front);
+    factor_block(&s[0][0], kLd, n, sh, v, w.sign + F.piv, w.neg + tk.front);
     store_rows(v, n, A, F.ldp);
 }
 
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
             tile_each(old, [&](int r, int c, double v) { sA[r][c] = v; });
             __syncthreads();
             double v[8][2];
-            factor_block(&sA[0][0], kLd, ni, sh, v, w.sign + F.piv + i * kT, w.flags + F.tissue, w.neg + tk.front);
+            factor_block(&sA[0][0], kLd, ni, sh, v, w.sign + F.piv + i * kT, w.neg + tk.front);
             store_rows(v, ni, out, F.ldp);
         } else {
             tile_sub(old, acc);
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
     __syncthreads();
     {
         double v[8][2];
-        factor_block(sX, ld, p, sh, v, s_sign, w.flags + F.tissue, w.neg + tk.front);
+        factor_block(sX, ld, p, sh, v, s_sign, w.neg + tk.front);
         store_rows(v, p, w.factor + F.x11, F.ldp);
         const int r = 8 * warp + (lane >> 2);  // every row of s was read before factor_block's last barrier
         if (r < p8r)

@@ -91,7 +91,6 @@ struct FcPlan {
     int64_t n_vec = 0, n_piv = 0, n_ent = 0;
     int64_t n_root = 0;   // pivots of the root fronts
     double flops = 0.0;   // multiplications and additions of one factorisation
-    int chain = 0;        // dependent 64-pivot panels over the depths
     bool ok = false;
 };
 
@@ -118,7 +117,6 @@ struct FcWork {
     double* vec;
     double* z;
     double* sign;    // [n_piv] +1 / -1
-    int32_t* flags;  // [T] 1: a zero or non-finite pivot
     int32_t* neg;    // [fronts] 1: the front has negative pivots
 };
 
@@ -154,7 +152,7 @@ struct FcSpan {
 __host__ __device__ inline FcSpan fc_block_span(int32_t k0, int32_t k1) { return {(int64_t)k0 * 9, (int64_t)k1 * 9}; }
 
 struct FcCg {
-    int n_chunks, T;
+    int n_chunks;
     const FcChunk* chunks;
     const int32_t* chunk0;  // [T+1]
     KrylovScalars* sc;      // [T]

@@ -501,7 +501,6 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
         });
         int np = 0;
         for (int32_t fi : fs) np = std::max(np, cdiv(plan.fronts[fi].p, kFcTile));
-        plan.chain += np;
         L.panel0 = (int32_t)plan.panels.size();
         L.n_panel = std::max(0, np);
         for (int k = 0; k < np; ++k) {
