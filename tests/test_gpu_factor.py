@@ -109,6 +109,19 @@ def test_singular_system_falls_back():
     assert rc in (capi.TF_OK, capi.TF_KRYLOV_MAX_ITERS, capi.TF_KRYLOV_BREAKDOWN, capi.TF_NONFINITE)
 
 
+@pytest.mark.parametrize("name", ["one_front", "root_66", "three_nodes"])
+def test_launches_outside_graphs(name):
+    """use_graphs = 0 launches the same kernels one by one: equal to the last bit."""
+    t = TISSUES[name]()
+    vals, g, _ = _system(t)
+    out = []
+    for graphs in (0, 1):
+        with NewtonRaphsonSolver.from_tissue(t, use_graphs=graphs) as s:
+            out.append([s.solveForDeltaU(vals, g)[0] for _ in range(2)])
+            assert s.krylov_method() == 2 and s.preconditioner()[2] == 2
+    assert all(np.array_equal(a, out[0][0]) for r in out for a in r)
+
+
 def test_slaves_and_boundary_changes_rebuild_the_plan():
     """Slave-master pairs couple distant columns (a new pattern, a new dissection); setting the boundary
     again returns to the first one. Positions against the iterative path (krylov_warm_start = 0)."""

@@ -39,6 +39,25 @@ def test_second_right_hand_side_of_a_lumen_replaces_a_kept_factor(rate):
     assert np.abs(out[1][0] - out[0][0]).max() <= 1e-9 * t.size
 
 
+def test_kept_factor_is_replaced_where_newton_moves_far():
+    """Steps of 600 s of fast growth: the factor kept from the second Newton iteration does not serve all of the
+    later ones and is made anew (a third time and more), without the iterative solve. Positions within 1e-9 of
+    the size of that solve's."""
+    out = {}
+    for warm in (1, 0):  # 0: no factor
+        t = mesh.small_rectangle(nx=60, ny=40)
+        t.rates *= 5.0
+        with NewtonRaphsonSolver.from_tissue(t, krylov_warm_start=warm, krylov_rtol=1e-13) as s:
+            x, launches = t.x, 0
+            for _ in range(2):
+                x, rc, st = s.runOneStep(x, 600.0)
+                assert rc == capi.TF_OK
+                launches += st["solve_launches"]
+            out[warm] = (x, launches, s.preconditioner()[2])
+    assert out[1][1] == 0 and out[1][2] >= 6
+    assert np.abs(out[1][0] - out[0][0]).max() <= 1e-9 * t.size
+
+
 def test_packing_pairs_that_come_and_go_on_one_solver():
     """Two sheets apart, in contact and apart again, each step from given positions: the factor serves the first
     and the last, MINRES the one with pairs, and what the solver says of its preconditioner is what a solver
