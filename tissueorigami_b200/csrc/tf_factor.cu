@@ -435,12 +435,13 @@ __global__ void __launch_bounds__(256) k_fc_upd(FcWork w, int begin, int k) {
     load_tile(sA, lp + (size_t)i * kT * kT, kT, ni, nk);
     if (j > k) {
         const double* sg = w.sign + F.piv + k * kT;
+        const double sign = (int)threadIdx.x < nk ? sg[threadIdx.x] : 1.0;  // on its way with the tiles
         load_tile(sB, lp + (size_t)j * kT * kT, kT, nj, nk);
         cp_commit();
         cp_wait<0>();
         // Panel k's signs are of an earlier launch. The front's flag is not: the CTA of the next diagonal block sets
         // it in this one, and threads that read it for themselves could part ways around the barrier below.
-        if (__syncthreads_or((int)threadIdx.x < nk && sg[threadIdx.x] < 0.0)) {
+        if (__syncthreads_or(sign < 0.0)) {
             for (int e = threadIdx.x; e < kT * kT; e += 256) sB[e >> 6][e & 63] *= (e & 63) < nk ? sg[e & 63] : 0.0;
             __syncthreads();
         }
