@@ -64,6 +64,9 @@ __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void prefetch(const double* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// A parameter's array indexed by a variable is copied to local memory (128 bytes a thread); two of it are not.
+__device__ __forceinline__ double* contrib(const FcWork& w, int parity) { return parity ? w.contrib[1] : w.contrib[0]; }
+
 // ---- assembly of a front -------------------------------------------------------------------
 
 // Rows [i j, (i + 1) j) of the front's pivot columns (task j: 8 or 32): what its children left there. Rows below p
@@ -78,8 +81,8 @@ __global__ void __launch_bounds__(256) k_fc_gather(FcWork w, int begin, int pari
     __syncthreads();
     chain_wait();
     if (!w.active[F.tissue]) return;
-    const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
-    const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
+    const double* __restrict__ C0 = F.child[0] >= 0 ? contrib(w, parity ^ 1) + F.child_c[0] : w.factor;
+    const double* __restrict__ C1 = F.child[1] >= 0 ? contrib(w, parity ^ 1) + F.child_c[1] : w.factor;
     const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r1 = min((tk.i + 1) * tk.j, F.p + F.b);
@@ -523,8 +526,8 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
         cp_wait<0>();
         return;
     }
-    const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
-    const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
+    const double* __restrict__ C0 = F.child[0] >= 0 ? contrib(w, parity ^ 1) + F.child_c[0] : w.factor;
+    const double* __restrict__ C1 = F.child[1] >= 0 ? contrib(w, parity ^ 1) + F.child_c[1] : w.factor;
     const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
     if (F.child[0] >= 0) {  // eight rows a warp pass, the loads of all of them in flight
         bool first = true;
@@ -625,7 +628,7 @@ __global__ void __launch_bounds__(256, 3) k_fc_small(FcWork w, const double* __r
     __syncthreads();
     // contribution, 16 x 16 tiles of the lower triangle
     const bool neg = w.neg[tk.front] != 0;
-    double* Cf = w.contrib[parity] + F.c;
+    double* Cf = contrib(w, parity) + F.c;
     const int nt = b16 >> 4;
     for (int task = warp; task < nt * (nt + 1) / 2; task += 8) {
         int i = (int)((sqrtf(8.0f * task + 1.0f) - 1.0f) * 0.5f);
@@ -817,8 +820,8 @@ __global__ void __launch_bounds__(128, 4) k_fc_schur(FcWork w, int begin, int pa
         const int2 k = idx < F.b ? w.kids[F.ent + F.p + idx] : make_int2(-1, -1);
         s_map[q][side][c] = q ? k.y : k.x;
     }
-    const double* __restrict__ C0 = F.child[0] >= 0 ? w.contrib[parity ^ 1] + F.child_c[0] : w.factor;
-    const double* __restrict__ C1 = F.child[1] >= 0 ? w.contrib[parity ^ 1] + F.child_c[1] : w.factor;
+    const double* __restrict__ C0 = F.child[0] >= 0 ? contrib(w, parity ^ 1) + F.child_c[0] : w.factor;
+    const double* __restrict__ C1 = F.child[1] >= 0 ? contrib(w, parity ^ 1) + F.child_c[1] : w.factor;
     const int ld0 = F.child_ldb[0], ld1 = F.child_ldb[1];
     // the product accumulates onto minus the children's entries, so that nothing but stores follows it
     gemm_tile<true>(L + (size_t)i * kT * F.ldp, F.ldp, ni, L + (size_t)j * kT * F.ldp, F.ldp, nj, F.p,
@@ -838,7 +841,7 @@ __global__ void __launch_bounds__(128, 4) k_fc_schur(FcWork w, int begin, int pa
                           }
                   }
               });
-    double* out = w.contrib[parity] + F.c + (size_t)i * kT * F.ldb + j * kT;
+    double* out = contrib(w, parity) + F.c + (size_t)i * kT * F.ldb + j * kT;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
