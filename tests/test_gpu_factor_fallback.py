@@ -58,6 +58,23 @@ def test_kept_factor_is_replaced_where_newton_moves_far():
     assert np.abs(out[1][0] - out[0][0]).max() <= 1e-9 * t.size
 
 
+@pytest.mark.parametrize("cap", [2, 3])
+def test_kept_factor_is_replaced_at_a_low_iteration_cap(cap):
+    """krylov_max_iters below what a kept factor needs (three to five iterations, where a factor of J itself needs
+    one): the steps converge all the same, to the positions without a cap (1e-9 of the size)."""
+    t = mesh.wing_disc(n_surface_points=1500)
+    out = {}
+    for most in (cap, 20000):
+        with NewtonRaphsonSolver.from_tissue(t, krylov_max_iters=most) as s:
+            x = t.x
+            for _ in range(2):
+                x, rc, st = s.runOneStep(x, t.dt)
+                assert rc == capi.TF_OK and st["solve_launches"] == 0
+            out[most] = (x, s.preconditioner()[2])
+    assert out[20000][1] == 4 and out[cap][1] > 4  # two factorisations a step without a cap
+    assert np.abs(out[cap][0] - out[20000][0]).max() <= 1e-9 * t.size
+
+
 def test_packing_pairs_that_come_and_go_on_one_solver():
     """Two sheets apart, in contact and apart again, each step from given positions: the factor serves the first
     and the last, MINRES the one with pairs, and what the solver says of its preconditioner is what a solver

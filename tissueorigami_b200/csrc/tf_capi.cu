@@ -1920,8 +1920,8 @@ int factor_solve(tf_ctx* ctx, std::vector<int32_t>& left) {
             const int st = ctx->h_tsc[t].status;
             if (st == KS_RUNNING) {
                 running = true;
-            } else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters)) {
-                if (ctx->fc_near) {  // the kept factor does not fit: with one of this J
+            } else if (st != KS_CONVERGED && !(st == KS_MAXIT && cap == ctx->params.krylov_max_iters && !ctx->fc_near)) {
+                if (ctx->fc_near) {  // the kept factor does not fit, or needs more iterations than allowed: with one of this J
                     ctx->fc_near = false;
                     return factor_solve(ctx, left);
                 }
