@@ -68,7 +68,10 @@ extern "C" {
                               /* TF_PRECOND_TWO_LEVEL and warm starts on, tissues whose   */
                               /* factorisation is below 3e11 operations are preconditioned */
                               /* by the sparse factor of J's symmetric part instead: one  */
-                              /* or two iterations (not on steps with packing pairs)      */
+                              /* or two iterations with a factor of J itself, three to    */
+                              /* five with one kept from an earlier Newton iteration (not */
+                              /* on steps with packing pairs, nor where it would take     */
+                              /* more than half of the free device memory)                */
 #define TF_KRYLOV_BICGSTAB 1  /* BiCGStab                                                 */
 #define TF_KRYLOV_CG 2        /* preconditioned conjugate gradients; a tissue whose J turns */
                               /* out indefinite is solved again with BiCGStab              */
