@@ -96,8 +96,9 @@ struct FcPlan {
 
 // Symbolic factorisation of the block pattern (G consecutive nodes form one column with in-plane
 // position X[3 column]); tissue t owns nodes [node0[t], node0[t+1]). plan.ok = false when a front
-// is too large for the kernels, the operation count exceeds max_flops or a position is not a finite number. transposed: with jblk_t, so that
-// the symmetric part (J + J^T) / 2 of an unsymmetric J is factorised. Throws std::bad_alloc.
+// is too large for the kernels, the operation count exceeds max_flops or a position is not a finite number.
+// transposed: with jblk_t, so that the symmetric part (J + J^T) / 2 of an unsymmetric J is factorised. Throws
+// std::bad_alloc.
 void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colidx, const double* X, int T,
                        const int32_t* node0, double max_flops, bool transposed, FcPlan& plan);
 

@@ -21,6 +21,9 @@ struct Node {
     int32_t lo = 0, hi = 0;  // its subtree's columns in perm
 };
 
+// Operations of a front of p pivots and b boundary unknowns.
+double front_flops(double p, double b) { return p * p * p * (2.0 / 3.0) + p * p * b + b * b * p; }
+
 // Operations of the fronts of all tissues, against the limit.
 struct Budget {
     double max_flops;
@@ -32,7 +35,7 @@ struct Budget {
     void add(size_t np, size_t nb, int gd) {
         const double p = (double)np * gd, b = (double)nb * gd;
         std::lock_guard<std::mutex> hold(lock);
-        flops += p * p * p * (2.0 / 3.0) + p * p * b + b * b * p;
+        flops += front_flops(p, b);
         if (p > kFcMaxPivots || p + b > kFcMaxFront || flops > max_flops) over = true;
     }
 };
@@ -326,14 +329,16 @@ void build_factor_plan(int N, int G, const int32_t* rowptr, const int32_t* colid
     });
     plan.flops = budget.flops;
     if (budget.over) return;
-    // fronts of all tissues by depth
+    // fronts of all tissues by depth; their operations again, in an order that no thread decides
     int depths = 0;
+    plan.flops = 0.0;
     std::vector<std::vector<std::pair<int, int>>> at;  // per depth: (tissue, node)
     for (int t = 0; t < T; ++t)
         for (int k = 0; k < (int)ds[t].nodes.size(); ++k) {
             const Node& f = ds[t].nodes[k];
             if (f.depth >= depths) at.resize(depths = f.depth + 1);
             at[f.depth].push_back({t, k});
+            plan.flops += front_flops((double)f.piv.size() * gd, (double)f.bnd.size() * gd);
         }
     std::vector<std::vector<int32_t>> id(T);
     for (int t = 0; t < T; ++t) id[t].resize(ds[t].nodes.size());
