@@ -31,12 +31,10 @@ struct Budget {
     double flops = 0.0;
     std::atomic<bool> over{false};
 
-    // A front of np pivot and nb boundary columns of gd unknowns each.
-    void add(size_t np, size_t nb, int gd) {
-        const double p = (double)np * gd, b = (double)nb * gd;
+    void add(double more) {
         std::lock_guard<std::mutex> hold(lock);
-        flops += front_flops(p, b);
-        if (p > kFcMaxPivots || p + b > kFcMaxFront || flops > max_flops) over = true;
+        flops += more;
+        if (flops > max_flops) over = true;
     }
 };
 
@@ -224,10 +222,18 @@ struct Dissection {
         pos.assign(n, 0);
         nodes.emplace_back();
         nodes[0].hi = n;
+        double mine = 0.0;  // not in the budget yet: its lock is for shares that matter, not for every front
         for (int id = 0; id < (int)nodes.size() && !budget.over; ++id) {
             split(id);
-            budget.add(nodes[id].piv.size(), nodes[id].bnd.size(), gd);
+            const double p = (double)nodes[id].piv.size() * gd, b = (double)nodes[id].bnd.size() * gd;
+            if (p > kFcMaxPivots || p + b > kFcMaxFront) budget.over = true;
+            mine += front_flops(p, b);
+            if (mine * 1024 > budget.max_flops) {
+                budget.add(mine);
+                mine = 0.0;
+            }
         }
+        budget.add(mine);
         if (budget.over) return;
         std::vector<Node> sorted;
         sorted.reserve(nodes.size());
